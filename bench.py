@@ -46,10 +46,10 @@ import numpy as np  # noqa: E402
 METRIC = "particle-steps/s FP32c vs FP64 at ≤1e-3 rel L2; ensemble p50/p99 time-to-result"
 UNIT = "particle-steps/s"
 # launches of one FP32c step graph (3D, sph_api.cu step_sequence): momentum
-# pair sums and finish, 8 sort, 3 boundary, lists, continuity pair sums and
+# pair sums and finish, 4 sort, 2 boundary, lists, continuity pair sums and
 # finish, finalize; the FP64 graph has one momentum and one continuity kernel
-KERNELS_PER_STEP = 17
-KERNELS_PER_STEP_FP64 = 15
+KERNELS_PER_STEP = 12
+KERNELS_PER_STEP_FP64 = 10
 # algorithmic bytes of the fused FP32c momentum pass (k_momentum_f32 pair
 # sums + k_momentum_f32_finish): per particle, each record read once -- X 32,
 # V 32, RP 16, XF 16, VF 16, RM 8 (the neighbours' XF/VF/RM are these same

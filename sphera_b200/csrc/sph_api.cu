@@ -748,13 +748,11 @@ int sync_dyn(SphHandle* h) {
   return SPH_OK;
 }
 
-void sort_sequence(SphHandle* h, cudaStream_t st) {
-  launch_sort_reset(h->db, st);
+void sort_sequence(SphHandle* h, bool boundary_follows, cudaStream_t st) {
   launch_bin(h->db, KeyKind::Sort, st);
-  launch_removal(h->db, st);
-  launch_scan(h->db, h->P.cell_start, st);
+  launch_scan(h->db, h->P.cell_start, true, st);
   launch_place(h->db, st);
-  launch_rank_permute(h->db, st);
+  launch_rank_permute(h->db, boundary_follows, st);
 }
 
 // CalcVarLength: the neighbour lists and, with C1_BE, the fluid part of
@@ -817,10 +815,10 @@ void step_sequence(SphHandle* h, cudaStream_t st, EarlyCopy* early = nullptr) {
   momentum_pass(h, true, st);
   if (h->any_teta_v) launch_velocity_smoothing(h->db, true, h->precision == SPH_PREC_FP32C, st);
   if (early) enqueue_early_copy(h, st, *early);
-  sort_sequence(h, st);
+  sort_sequence(h, true, st);
   cudaEventRecord(h->ev_fork, st);
   cudaStreamWaitEvent(h->stream2, h->ev_fork, 0);
-  launch_boundary(h->db, h->stream2);
+  launch_boundary(h->db, true, h->stream2);
   cudaEventRecord(h->ev_join, h->stream2);
   lists_pass(h, st);
   if (h->precision == SPH_PREC_FP32C) {
@@ -1024,6 +1022,7 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_near, nr.data(), C, cudaMemcpyHostToDevice, q);
   if (e == cudaSuccess && !cfl.empty()) e = cudaMemcpyAsync(h->d_cf_list, cfl.data(), sizeof(int) * cfl.size(), cudaMemcpyHostToDevice, q);
   if (e == cudaSuccess) e = cudaMemsetAsync(P.cell_count, 0, sizeof(int) * (C + 1), q);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->d_scan, 0, sizeof(int) * nb, q);
   if (e == cudaSuccess) e = cudaMemsetAsync(P.out_flag, 0, N, q);
   if (e == cudaSuccess) e = cudaMemsetAsync(P.bdt_count, 0, sizeof(int) * N, q);
   if (e == cudaSuccess) e = cudaMemsetAsync(P.ACC, 0, sizeof(double4) * N, q);
@@ -1135,10 +1134,8 @@ int upload_and_initialise(SphHandle* h, const SphState* states) {
   SPH_CUDA(cudaStreamWaitEvent(q3, h->ev_pos, 0));
   for (int s = 0; s < h->nsims; ++s) SPH_TRY(upload_rest(h, s, &states[s], q3));
   launch_init_rest(h->db, h->d_cv, h->d_crho, h->d_cp, q3);
-  launch_sort_reset(h->db, q);
   launch_bin(h->db, KeyKind::Sort, q);
-  launch_removal(h->db, q);
-  launch_scan(h->db, h->P.cell_start, q);
+  launch_scan(h->db, h->P.cell_start, true, q);
   launch_place(h->db, q);
   launch_rank_permute_positions(h->db, q);
   SPH_CUDA(cudaEventRecord(h->ev_sorted, q));
@@ -1147,7 +1144,7 @@ int upload_and_initialise(SphHandle* h, const SphState* states) {
   SPH_CUDA(cudaEventRecord(h->ev_rest, q3));
   SPH_CUDA(cudaEventRecord(h->ev_fork, q));
   SPH_CUDA(cudaStreamWaitEvent(h->stream2, h->ev_fork, 0));
-  launch_boundary(h->db, h->stream2);
+  launch_boundary(h->db, true, h->stream2);
   SPH_CUDA(cudaEventRecord(h->ev_join, h->stream2));
   launch_neighbour_lists(h->db, q);
   SPH_CUDA(cudaStreamWaitEvent(q, h->ev_join, 0));
@@ -1427,9 +1424,9 @@ int sph_replace_particles(SphHandle* h, const SphState* state, const int32_t* la
   if (laminar && state->n > 0)
     SPH_CUDA(cudaMemcpyAsync(h->d_ci1, laminar, sizeof(int32_t) * state->n, cudaMemcpyDefault, q));
   launch_init_from_caller(h->db, h->d_cx, h->d_cv, h->d_crho, h->d_cp, h->d_cm, q);
-  sort_sequence(h, q);
+  sort_sequence(h, true, q);
   if (laminar && state->n > 0) launch_load_laminar(h->db, h->d_ci1, q);
-  launch_boundary(h->db, q);
+  launch_boundary(h->db, true, q);
   lists_pass(h, q);
   SPH_CUDA(cudaGetLastError());
   return sync_dyn(h);
@@ -1548,7 +1545,7 @@ int sph_ord_grid(SphHandle* h) {
   NvtxRange range_("OrdGrid1 + CalcVarLength");
   if (!h || !h->uploaded) return SPH_ERR_INVALID_ARGUMENT;
   launch_stage(h->db, h->stream);
-  sort_sequence(h, h->stream);
+  sort_sequence(h, false, h->stream);
   lists_pass(h, h->stream);
   SPH_CUDA(cudaGetLastError());
   return sync_dyn(h);
@@ -1558,7 +1555,7 @@ int sph_boundary_data_tab(SphHandle* h) {
   DeviceGuard dev_guard_(h);
   NvtxRange range_("ComputeBoundaryDataTab");
   if (!h || !h->uploaded) return SPH_ERR_INVALID_ARGUMENT;
-  launch_boundary(h->db, h->stream);
+  launch_boundary(h->db, false, h->stream);
   SPH_CUDA(cudaGetLastError());
   return sync_dyn(h);
 }
@@ -1624,9 +1621,8 @@ int sph_dump_grid(SphHandle* h, int32_t* cella, int32_t* icont, int32_t* npartor
     SPH_CUDA(cudaMemcpyAsync(cella, h->d_ci1, sizeof(int) * n, cudaMemcpyDeviceToHost, q));
   }
   if (icont || npartord) {
-    launch_sort_reset(h->db, q);
     launch_bin(h->db, KeyKind::Reference, q);
-    launch_scan(h->db, h->d_ci2, q);
+    launch_scan(h->db, h->d_ci2, false, q);
     launch_rank_reference(h->db, h->d_ci2, h->d_ci3, q);
     SPH_CUDA(cudaGetLastError());
     if (icont) {
@@ -1791,7 +1787,7 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
           case kGridLists: launch_neighbour_lists(b, q); break;
           case kGridMomentum: momentum_pass(h, false, q); break;
           case kGridContinuity: continuity_pass(h, false, q); break;
-          default: launch_boundary(b, q); break;
+          default: launch_boundary(b, false, q); break;
         }
       };
       run();   // warm-up
@@ -1858,9 +1854,9 @@ int sph_profile_phases(SphHandle* h, int32_t nsteps, double* ms) {
     momentum_pass(h, true, q);
     if (h->any_teta_v) launch_velocity_smoothing(h->db, true, h->precision == SPH_PREC_FP32C, q);
     cudaEventRecord(ev[1], q);
-    sort_sequence(h, q);
+    sort_sequence(h, true, q);
     cudaEventRecord(ev[2], q);
-    launch_boundary(h->db, q);
+    launch_boundary(h->db, true, q);
     cudaEventRecord(ev[3], q);
     lists_pass(h, q);
     cudaEventRecord(ev[4], q);

@@ -257,12 +257,19 @@ __global__ void k_stage(DevBatch b) {
   }
 }
 
-// Cell key of every slot + atomic histogram.  KeyKind::Sort bins the
+constexpr int kScanThreads = 1024;
+constexpr int kScanPer = 4;
+constexpr int kScanChunk = kScanThreads * kScanPer;
+constexpr int kBinChunks = 8;            // chunks around a block's first that k_bin gathers
+
+// Cell key of every slot + atomic histogram, and the histogram's sums over
+// chunks of kScanChunk cells that the scan starts from.  KeyKind::Sort bins the
 // scratch record by the z-fastest layout key; KeyKind::Reference bins the
 // sorted state by CellNumber.f90's numbering for the grid dump.
 template <KeyKind KIND>
 __global__ void k_bin(DevBatch b) {
   __shared__ SimDev s;
+  __shared__ int first_chunk, chunk_sum[kBinChunks];
   int cur = -1;
   const Particles& P = b.P;
   const int lane = threadIdx.x & 31;
@@ -299,15 +306,30 @@ __global__ void k_bin(DevBatch b) {
     if (valid && lane == leader) base = atomicAdd(P.cell_count + key, __popc(peers));
     base = __shfl_sync(0xffffffffu, base, leader);
     if (valid) P.slot[p] = base + __popc(peers & ((1u << lane) - 1u));
+    // the chunk sums of the scan, gathered over the block (its particles
+    // lie in one chunk or a few): a global addition per warp met the others
+    // on the same few addresses and cost 14 us at 864,000 particles
+    const int chunk = valid ? key / kScanChunk : -1;
+    if (threadIdx.x == 0) first_chunk = chunk;
+    if (threadIdx.x < kBinChunks) chunk_sum[threadIdx.x] = 0;
+    __syncthreads();
+    const unsigned same = __match_any_sync(0xffffffffu, chunk);
+    if (valid && lane == __ffs(same) - 1) {
+      const unsigned c = (unsigned)(chunk - first_chunk + kBinChunks / 2);
+      if (c < (unsigned)kBinChunks) atomicAdd(chunk_sum + c, __popc(same));
+      else atomicAdd(b.scan_block_sums + chunk, __popc(same));
+    }
+    __syncthreads();
+    if (threadIdx.x < kBinChunks && chunk_sum[threadIdx.x] != 0)
+      atomicAdd(b.scan_block_sums + first_chunk - kBinChunks / 2 + threadIdx.x, chunk_sum[threadIdx.x]);
+    __syncthreads();
   }
 }
 
 // OrdGrid1.f90:58-82: particles out of the grid are removed by moving the
 // last particle into their place, in increasing particle index.  Replayed
 // exactly (one thread per simulation, only when a removal happened).
-__global__ void k_removal(DevBatch b) {
-  int sim = blockIdx.x;
-  if (threadIdx.x != 0 || sim >= b.nsims) return;
+__device__ void replay_removals(const DevBatch& b, int sim) {
   SimDyn* d = b.dyn + sim;
   if (d->n_out == 0) return;
   const SimDev& s = b.sims[sim];
@@ -360,59 +382,56 @@ __device__ __forceinline__ int block_excl_scan(int v, int* warp_sums, int& total
   return base + x - v;
 }
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanPer = 4;
-constexpr int kScanChunk = kScanThreads * kScanPer;
-
-__global__ void __launch_bounds__(kScanThreads) k_scan1(const int* __restrict__ cnt, int n, int* block_sums) {
-  __shared__ int ws[32];
-  int base = blockIdx.x * kScanChunk + threadIdx.x * kScanPer;
-  int v = 0;
-  for (int q = 0; q < kScanPer; ++q) v += (base + q < n) ? cnt[base + q] : 0;
-  int total;
-  block_excl_scan(v, ws, total);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan2(int* block_sums, int nb, int* cell_start, int n) {
-  __shared__ int ws[32];
-  int carry = 0;
-  for (int c0 = 0; c0 < nb; c0 += kScanThreads) {
-    int i = c0 + threadIdx.x;
-    int v = i < nb ? block_sums[i] : 0;
-    int total;
-    int ex = block_excl_scan(v, ws, total);
-    if (i < nb) block_sums[i] = ex + carry;
-    carry += total;
+// Exclusive scan of the cell histogram, clearing it: block c < nb handles
+// one chunk of kScanChunk cells, starting from the sum of the chunk sums
+// before it (k_bin added those up).  The blocks past the chunks replay the
+// removals, one simulation each: both need the finished binning and
+// neither needs the other, so one launch holds what were four (chunk sums,
+// their scan, the scan, the removals).  These launches are latency alone:
+// at 5,000 particles the sort took 35 us in eight launches.
+__global__ void __launch_bounds__(kScanThreads) k_scan(DevBatch b, int n, int nb, int* cell_start, int removals) {
+  if (blockIdx.x >= nb) {
+    const int sim = blockIdx.x - nb;
+    if (removals && threadIdx.x == 0 && sim < b.nsims) replay_removals(b, sim);
+    return;
   }
-  if (threadIdx.x == 0) cell_start[n] = carry;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan3(int* cnt, int n, const int* block_sums, int* cell_start) {
   __shared__ int ws[32];
-  int base = blockIdx.x * kScanChunk + threadIdx.x * kScanPer;
+  __shared__ int before;
+  int* cnt = b.P.cell_count;
+  const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanPer;
   int vals[kScanPer];
   int v = 0;
   for (int q = 0; q < kScanPer; ++q) {
     vals[q] = (base + q < n) ? cnt[base + q] : 0;
     v += vals[q];
   }
+  int prev = 0;
+  for (int c = threadIdx.x; c < (int)blockIdx.x; c += kScanThreads) prev += b.scan_block_sums[c];
+  if (threadIdx.x == 0) before = 0;
+  __syncthreads();
+  prev = __reduce_add_sync(0xffffffffu, prev);
+  if ((threadIdx.x & 31) == 0 && prev) atomicAdd(&before, prev);
   int total;
-  int ex = block_excl_scan(v, ws, total) + block_sums[blockIdx.x];
+  int ex = block_excl_scan(v, ws, total);
+  ex += before;
   for (int q = 0; q < kScanPer; ++q) {
     if (base + q < n) {
       cell_start[base + q] = ex;
       cnt[base + q] = 0;
     }
     ex += vals[q];
+    if (base + q == n - 1) cell_start[n] = ex;
   }
 }
 
 // Unstable placement by cell (the atomic slot), remembering the source.
+// Also clears the scan's chunk sums for the next binning.
 __global__ void k_place(DevBatch b, const int* __restrict__ cstart, int use_scratch_ids) {
   __shared__ SimDev s;
   int cur = -1;
   const Particles& P = b.P;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < b.scan_nblocks; c += gridDim.x * blockDim.x)
+    b.scan_block_sums[c] = 0;
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
@@ -439,11 +458,26 @@ __global__ void k_place(DevBatch b, const int* __restrict__ cstart, int use_scra
 // kPermuteRest gathers the rest through it.
 constexpr int kPermuteAll = 0, kPermutePositions = 1, kPermuteRest = 2;
 
+// The last launch of a sort also clears counters: the out-of-grid count for
+// the next binning and, where the boundary pass follows at once, that
+// pass's own.
+__device__ __forceinline__ void reset_boundary_counters(const DevBatch& b, int sim) {
+  b.dyn[sim].ncbf_max = 0;
+  b.dyn[sim].bdt_sim_used = 0;
+  if (sim == 0) b.dyn[b.nsims].bdt_used = 0;
+}
+
 template <int PART>
-__global__ void k_rank_permute(DevBatch b) {
+__global__ void k_rank_permute(DevBatch b, int boundary_follows) {
   __shared__ SimDev s;
   int cur = -1;
   const Particles& P = b.P;
+  if (PART != kPermuteRest) {
+    for (int sim = blockIdx.x * blockDim.x + threadIdx.x; sim < b.nsims; sim += gridDim.x * blockDim.x) {
+      b.dyn[sim].n_out = 0;
+      if (boundary_follows) reset_boundary_counters(b, sim);
+    }
+  }
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
@@ -3613,18 +3647,10 @@ __global__ void k_cancel(DevBatch b, int sim) {
   }
 }
 
-__global__ void k_sort_reset(DevBatch b) {
-  int sim = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sim < b.nsims) b.dyn[sim].n_out = 0;
-}
-
+// A boundary pass that no sort has just preceded (the per-call ABI).
 __global__ void k_bdt_reset(DevBatch b) {
   int sim = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sim < b.nsims) {
-    b.dyn[sim].ncbf_max = 0;
-    b.dyn[sim].bdt_sim_used = 0;
-  }
-  if (sim == 0) b.dyn[b.nsims].bdt_used = 0;
+  if (sim < b.nsims) reset_boundary_counters(b, sim);
 }
 
 // ==========================================================================
@@ -4085,14 +4111,9 @@ void launch_bin(const DevBatch& b, KeyKind kind, cudaStream_t st) {
   else k_bin<KeyKind::Reference><<<blocks_for(b), kBlock, 0, st>>>(b);
 }
 
-void launch_removal(const DevBatch& b, cudaStream_t st) { k_removal<<<b.nsims, 32, 0, st>>>(b); }
-
-void launch_scan(const DevBatch& b, int* cell_start, cudaStream_t st) {
-  int n = b.P.total_cells;
-  int nb = (n + kScanChunk - 1) / kScanChunk;
-  k_scan1<<<nb, kScanThreads, 0, st>>>(b.P.cell_count, n, b.scan_block_sums);
-  k_scan2<<<1, kScanThreads, 0, st>>>(b.scan_block_sums, nb, cell_start, n);
-  k_scan3<<<nb, kScanThreads, 0, st>>>(b.P.cell_count, n, b.scan_block_sums, cell_start);
+void launch_scan(const DevBatch& b, int* cell_start, bool removals, cudaStream_t st) {
+  const int n = b.P.total_cells, nb = (n + kScanChunk - 1) / kScanChunk;
+  k_scan<<<nb + (removals ? b.nsims : 0), kScanThreads, 0, st>>>(b, n, nb, cell_start, removals ? 1 : 0);
 }
 
 void launch_cancel(const DevBatch& b, int sim, cudaStream_t st) { k_cancel<<<1, 32, 0, st>>>(b, sim); }
@@ -4109,10 +4130,6 @@ void launch_set_dt(const DevBatch& b, double dt, cudaStream_t st) {
   k_set_dt<<<(b.nsims + 127) / 128, 128, 0, st>>>(b, dt);
 }
 
-void launch_sort_reset(const DevBatch& b, cudaStream_t st) {
-  k_sort_reset<<<(b.nsims + 127) / 128, 128, 0, st>>>(b);
-}
-
 void upload_bit2d(const double* tab, cudaStream_t st) {
   cudaMemcpyToSymbolAsync(c_bit2d, tab, sizeof(double) * 22 * 6, 0, cudaMemcpyHostToDevice, st);
 }
@@ -4121,16 +4138,16 @@ void launch_place(const DevBatch& b, cudaStream_t st) {
   k_place<<<blocks_for(b), kBlock, 0, st>>>(b, b.P.cell_start, 1);
 }
 
-void launch_rank_permute(const DevBatch& b, cudaStream_t st) {
-  k_rank_permute<kPermuteAll><<<blocks_for(b), kBlock, 0, st>>>(b);
+void launch_rank_permute(const DevBatch& b, bool boundary_follows, cudaStream_t st) {
+  k_rank_permute<kPermuteAll><<<blocks_for(b), kBlock, 0, st>>>(b, boundary_follows ? 1 : 0);
 }
 
 void launch_rank_permute_positions(const DevBatch& b, cudaStream_t st) {
-  k_rank_permute<kPermutePositions><<<blocks_for(b), kBlock, 0, st>>>(b);
+  k_rank_permute<kPermutePositions><<<blocks_for(b), kBlock, 0, st>>>(b, 1);
 }
 
 void launch_rank_permute_rest(const DevBatch& b, cudaStream_t st) {
-  k_rank_permute<kPermuteRest><<<blocks_for(b), kBlock, 0, st>>>(b);
+  k_rank_permute<kPermuteRest><<<blocks_for(b), kBlock, 0, st>>>(b, 0);
 }
 
 void launch_rank_reference(const DevBatch& b, const int* cell_start_ref, int* npartord, cudaStream_t st) {
@@ -4138,8 +4155,8 @@ void launch_rank_reference(const DevBatch& b, const int* cell_start_ref, int* np
   k_rank_reference<<<blocks_for(b), kBlock, 0, st>>>(b, cell_start_ref, npartord);
 }
 
-void launch_boundary(const DevBatch& b, cudaStream_t st) {
-  k_bdt_reset<<<(b.nsims + 127) / 128, 128, 0, st>>>(b);
+void launch_boundary(const DevBatch& b, bool cleared, cudaStream_t st) {
+  if (!cleared) k_bdt_reset<<<(b.nsims + 127) / 128, 128, 0, st>>>(b);
   if (b.dim == 3) {
     k_boundary3d<<<blocks_for(b, kGridBoundary), kBlock, 0, st>>>(b);
     k_boundary3d_integrals<<<b.grid[kGridIntegrals] > 0 ? b.grid[kGridIntegrals] : b.grid_blocks * 2, 128, 0, st>>>(b);

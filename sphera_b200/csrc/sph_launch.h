@@ -30,7 +30,7 @@ struct DevBatch {
   int list_cap4;           // 4-entry chunks reserved per particle (max NMAXPARTJ / 4)
   unsigned long long* counters;  // [0] momentum candidates, [1] momentum pairs,
                                  // [2] continuity candidates, [3] continuity pairs
-  int* scan_block_sums;    // scan scratch
+  int* scan_block_sums;    // sums of the cell histogram over the scan's chunks (zero between sorts)
   int scan_nblocks;
   int grid_blocks;         // blocks of the persistent particle kernels (default)
   int sms;                 // streaming multiprocessors of the device
@@ -47,12 +47,11 @@ enum class KeyKind { Sort = 0, Reference = 1 };
 // sorting
 void launch_stage(const DevBatch& b, cudaStream_t st);
 void launch_bin(const DevBatch& b, KeyKind kind, cudaStream_t st);
-void launch_removal(const DevBatch& b, cudaStream_t st);
-void launch_scan(const DevBatch& b, int* cell_start, cudaStream_t st);
-void launch_sort_reset(const DevBatch& b, cudaStream_t st);
+void launch_scan(const DevBatch& b, int* cell_start, bool removals, cudaStream_t st);
 void upload_bit2d(const double* tab, cudaStream_t st);
 void launch_place(const DevBatch& b, cudaStream_t st);
-void launch_rank_permute(const DevBatch& b, cudaStream_t st);
+// boundary_follows: clears the boundary pass's counters too
+void launch_rank_permute(const DevBatch& b, bool boundary_follows, cudaStream_t st);
 // the IC of an upload: positions first (destinations kept in P.slot), then the rest
 void launch_rank_permute_positions(const DevBatch& b, cudaStream_t st);
 void launch_rank_permute_rest(const DevBatch& b, cudaStream_t st);
@@ -61,7 +60,8 @@ void launch_rank_reference(const DevBatch& b, const int* cell_start_ref, int* np
 void launch_neighbour_lists(const DevBatch& b, cudaStream_t st);
 void launch_renormalisation(const DevBatch& b, cudaStream_t st);   // C1: fluid part of the matrices
 // physics (FP64)
-void launch_boundary(const DevBatch& b, cudaStream_t st);
+// cleared: the sort before it has cleared its counters
+void launch_boundary(const DevBatch& b, bool cleared, cudaStream_t st);
 void launch_momentum(const DevBatch& b, bool fused, cudaStream_t st);
 void launch_continuity(const DevBatch& b, bool fused, cudaStream_t st);
 // physics (FP32-compensated form)
