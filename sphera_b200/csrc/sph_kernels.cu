@@ -777,213 +777,282 @@ __global__ void __launch_bounds__(128) k_boundary3d_integrals(DevBatch b) {
   }
 }
 
+// The integrals of a particle close to two sides (a corner), both entries
+// at a time by one warp: lanes 0-15 the first, 16-31 the second.  Each of
+// the three quadratures has at most 10 abscissae (an arc of at most pi in
+// steps of about pi / 10; a chord of at most 4 h in steps of about h / 2), so
+// a lane forms one term of each -- its abscissa by the reference's repeated
+// addition -- and the terms are summed in the reference's order.  One lane
+// doing all of a corner's sines, cosines, tangents and arc tangents in
+// sequence took 37 us at 5,000 particles, the longest launch of a 2D step.
+__device__ __forceinline__ void corner_integrals2d(const SimDev& s, const SideDev* __restrict__ sd, SimDyn* dyn,
+                                                   const int* ib, const double* ix, const double* iy,
+                                                   BdtEntry* out) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, i = lane & 15, c = lane >> 4;
+  const double px = c ? ix[1] : ix[0], py = c ? iy[1] : iy[0];
+  const int isi = c ? ib[1] : ib[0];
+  // the half's terms 0..n-1 added to acc in order
+  auto add_terms = [&](double acc, double term, int n) {
+    for (int k = 0; k < 16; ++k) {
+      const double v = __shfl_sync(FULL, term, k, 16);
+      if (k < n) acc = acc + v;
+    }
+    return acc;
+  };
+  auto sub_terms = [&](double acc, double term, int n) {
+    for (int k = 0; k < 16; ++k) {
+      const double v = __shfl_sync(FULL, term, k, 16);
+      if (k < n) acc = acc - v;
+    }
+    return acc;
+  };
+  // FindBoundaryIntersection2D.f90:61-92
+  const double minlen = 0.01 * s.h;
+  const double ypi = py < 0.0 ? 0.0 : py;
+  const double halfchord = sqrt(s.square_doubleh - ypi * ypi);
+  const double XA = px - halfchord, XB = px + halfchord;
+  double xpmin = 0.0;
+  if (XA > xpmin) xpmin = XA;
+  double xpmax = sd[isi - 1].length;
+  if (XB < xpmax) xpmax = XB;
+  double interlen = xpmax - xpmin;
+  if (interlen <= minlen) interlen = 0.0;
+  const bool cut = interlen > 0.0;
+  // ComputeSurfaceIntegral_WdS2D.f90:57-83
+  int ndiv = 0;
+  double term = 0.0;
+  if (cut) {
+    const double dsrif = s.h / 2;
+    const double ypiq = ypi * ypi;
+    ndiv = (int)(interlen / dsrif + 0.5);
+    if (ndiv < 2) ndiv = 2;
+    const double deltas = interlen / ndiv;
+    double xpip = xpmin - 0.5 * deltas;
+    for (int k = 0; k <= i; ++k) xpip = xpip + deltas;
+    const double dxpip = xpip - px;
+    const double ris = sqrt(dxpip * dxpip + ypiq);
+    term = w_kernel(ris, s.h, s.coefke) * deltas;
+  }
+  const double IntWdS = add_terms(0.0, term, ndiv);
+  // BoundaryVolumeIntegrals2D.f90
+  const double dalfarif = kPigreco / 10;
+  const double yplimite = 0.05 * s.h;
+  const double ypb = py < yplimite ? yplimite : py;
+  double alfaA = 0.0, Intalfa = 0.0, t0 = 0.0, t1 = 0.0, t2 = 0.0;
+  ndiv = 0;
+  if (cut) {
+    alfaA = atan2(xpmin - px, ypb);
+    Intalfa = atan2(xpmax - px, ypb) - alfaA;
+    ndiv = (int)(Intalfa / dalfarif + 0.5);
+    if (ndiv < 1) ndiv = 1;
+    const double dalfa = Intalfa / ndiv;
+    double alfa_k = alfaA - 0.5 * dalfa;
+    for (int k = 0; k <= i; ++k) alfa_k = alfa_k + dalfa;
+    if (i < ndiv) {
+      const double sa = sin(alfa_k), ca = cos(alfa_k);
+      const double rb = ypb / ca;
+      const double rob = div_rn(rb, s.h, s.rcp_h);
+      const double mult = s.h * j2_wro2(rob) * dalfa;
+      t0 = sa * mult;
+      t1 = ca * mult;
+      t2 = w_integr(rb, s.h) * dalfa;
+    }
+  }
+  const double D0 = add_terms(0.0, t0, ndiv);
+  const double D1 = sub_terms(0.0, t1, ndiv);
+  double IntWdV = add_terms(0.0, t2, ndiv);
+  if (cut && ypb == yplimite) IntWdV = 0.5;
+  // ComputeVolumeIntegral_WdV2D.f90; at py >= yplimite (so ypb = py) its arc
+  // is the one above
+  term = 0.0;
+  const bool arc = cut && py >= yplimite;
+  ndiv = 0;
+  if (arc) {
+    ndiv = (int)(Intalfa / dalfarif + 0.5);
+    if (ndiv < 2) ndiv = 2;
+    const double dalfa = Intalfa / ndiv;
+    double alfa = alfaA - 0.5 * dalfa;
+    for (int k = 0; k <= i; ++k) alfa = alfa + dalfa;
+    if (i < ndiv) {
+      const double ta = tan(alfa);
+      const double ris = py * sqrt(1.0 + ta * ta);
+      term = w_integr(ris, s.h) * dalfa;
+    }
+  }
+  double IntWdV1 = add_terms(0.0, term, ndiv);
+  if (cut && !arc) {
+    const double ypj = c ? iy[0] : iy[1];   // the other side
+    if (ypj <= yplimite) {
+      double angle = 0.0;
+      if (sd[ib[0] - 1].previous_side == ib[1]) angle = sd[ib[0] - 1].angle;
+      else if (sd[ib[1] - 1].previous_side == ib[0]) angle = sd[ib[1] - 1].angle;
+      else set_status(dyn, 804);
+      IntWdV1 = 0.5 * (angle + kPigreco) / (2.0 * kPigreco);
+    } else {
+      IntWdV1 = (xpmin >= px && px <= xpmax) ? 0.5 : 0.0;
+    }
+  }
+  if (i != 0) return;
+  double func[3];
+  const int col[3] = {3, 4, 5};
+  interp_bit2d(3, col, py / s.h, func);
+  BdtEntry e;
+  for (int q = 0; q < 9; ++q) e.ig[q] = 0.0;
+  e.clobonum = isi;
+  e.pad = 0;
+  e.loc[0] = px;
+  e.loc[1] = py;
+  e.loc[2] = 0.0;
+  e.bi[0] = IntWdS;
+  e.bi[1] = IntWdV;
+  e.bi[2] = IntWdV1;
+  e.bi[3] = D0;
+  e.bi[4] = D1;
+  e.bi[5] = func[0] / s.squareh;
+  e.bi[6] = func[1] / s.squareh;
+  e.bi[7] = func[2] / s.squareh;
+  out[c] = e;
+}
+
 // ComputeBoundaryDataTab_2D.f90:70-157 with FindCloseBoundarySides2D,
 // SelectCloseBoundarySides2D, FindBoundaryIntersection2D,
 // ComputeSurfaceIntegral_WdS2D, BoundaryVolumeIntegrals2D,
-// ComputeVolumeIntegral_WdV2D and InterpolateBoundaryIntegrals2D.
+// ComputeVolumeIntegral_WdV2D and InterpolateBoundaryIntegrals2D.  A
+// particle close to one side finishes its entry itself; the corner particles
+// of the block (neighbours in the cell order) are then shared out over its
+// warps (corner_integrals2d).
 __global__ void __launch_bounds__(kBlock) k_boundary2d(DevBatch b) {
   __shared__ SimDev s;
+  __shared__ int ncorner, corner_ib[kBlock][2], corner_base[kBlock];
+  __shared__ double corner_xy[kBlock][4];   // x of both entries, y of both
   int cur = -1;
   const Particles& P = b.P;
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
-    if (threadIdx.x >= tl.count) continue;
-    int p = tl.start + threadIdx.x;
+    const int p = tl.start + threadIdx.x;
+    const bool slot = threadIdx.x < tl.count;
     SimDyn* dyn = b.dyn + tl.sim;
-    P.bdt_count[p] = 0;
-    if (p >= s.p_off + dyn->nag || s.nsides == 0) continue;
-    double4 x = P.X[p];
+    if (slot) P.bdt_count[p] = 0;
+    const bool on = slot && p < s.p_off + dyn->nag && s.nsides > 0;
     const SideDev* sd = b.sides + s.side_off;
-    int clob[kMaxCloseSides];
-    double lx[kMaxCloseSides], ly[kMaxCloseSides];
-    int ncbs = 0;
-    bool overflow = false;
-    for (int isi = 1; isi <= s.nsides; ++isi) {
-      const SideDev& S = sd[isi - 1];
-      double P1P0 = x.x - S.v1[0], P1P1 = x.z - S.v1[1];
-      double sidel = S.length;
-      double xp = P1P0 * S.sss[0] + P1P1 * S.sss[1];
-      double yp = P1P0 * S.nnn[0] + P1P1 * S.nnn[1];
-      double xpmin = -s.doubleh, xpmax = sidel + s.doubleh;
-      double ypmin = -s.doubleh, ypmax = s.doubleh;
-      if ((xpmin < xp && xp < xpmax) && (ypmin < yp && yp < ypmax)) {
-        double ypmx = 0.0, ypmn = 0.0;
-        if (xp < 0.0) {
-          ypmx = sqrt(s.square_doubleh - xp * xp);
-          ypmn = -ypmx;
-        } else if (xp <= sidel) {
-          ypmx = ypmax;
-          ypmn = ypmin;
-        } else if (xp < xpmax) {
-          double L = (sidel - xp) * (sidel - xp);
-          ypmx = sqrt(s.square_doubleh - L);
-          ypmn = -ypmx;
-        }
-        if (ypmn < yp && yp < ypmx) {
-          if (ncbs >= kMaxCloseSides) {
-            overflow = true;
-          } else {
-            clob[ncbs] = isi;
-            lx[ncbs] = xp;
-            ly[ncbs] = yp;
-          }
-          ncbs++;
-        }
-      }
-    }
-    if (overflow) {
-      set_status(dyn, SPH_ERR_CLOSE_SIDES);
-      continue;
-    }
-    if (ncbs == 0) continue;
-    if (ncbs == 2) {
-      if (sd[clob[0] - 1].previous_side == clob[1]) lx[1] = sd[clob[1] - 1].length - lx[1];
-      else if (sd[clob[1] - 1].previous_side == clob[0]) lx[0] = sd[clob[0] - 1].length - lx[0];
-    }
     // SelectCloseBoundarySides2D: fixe / tapi sides in front of the particle
-    int ib[kMaxCloseSides];
-    double ix[kMaxCloseSides], iy[kMaxCloseSides];
-    int nint = 0;
-    for (int c = 0; c < ncbs; ++c)
-      if (ly[c] > 0.0) {
-        ib[nint] = clob[c];
-        ix[nint] = lx[c];
-        iy[nint] = ly[c];
-        nint++;
-      }
-    if (nint == 0) continue;
-    if (atomicAdd(&dyn->bdt_sim_used, nint) + nint > s.bdt_quota) {
-      set_status(dyn, SPH_ERR_BDT_OVERFLOW);
-      continue;
-    }
-    int gbase = atomicAdd(&b.dyn[b.nsims].bdt_used, nint);
-    if (gbase + nint > P.bdt_cap) {
-      set_status(dyn, SPH_ERR_BDT_OVERFLOW);
-      continue;
-    }
-    P.bdt_count[p] = nint;
-    P.bdt_start[p] = gbase;
-    for (int c = 0; c < nint; ++c) {
-      BdtEntry e;
-      for (int q = 0; q < 9; ++q) e.ig[q] = 0.0;
-      for (int q = 0; q < 8; ++q) e.bi[q] = 0.0;
-      e.clobonum = ib[c];
-      e.pad = 0;
-      e.loc[0] = ix[c];
-      e.loc[1] = iy[c];
-      e.loc[2] = 0.0;
-      double func[5] = {0, 0, 0, 0, 0};
-      if (nint == 2) {
-        // FindBoundaryIntersection2D.f90:61-92
-        double minlen = 0.01 * s.h;
-        double xpi = ix[c], ypi = iy[c];
-        if (ypi < 0.0) ypi = 0.0;
-        double halfchord = sqrt(s.square_doubleh - ypi * ypi);
-        double XA = xpi - halfchord, XB = xpi + halfchord;
-        double xpmin = 0.0;
-        if (XA > xpmin) xpmin = XA;
-        double xpmax = sd[ib[c] - 1].length;
-        if (XB < xpmax) xpmax = XB;
-        double interlen = xpmax - xpmin;
-        if (interlen <= minlen) interlen = 0.0;
-        // ComputeSurfaceIntegral_WdS2D.f90:57-83
-        double IntWdS = 0.0;
-        if (interlen > 0.0) {
-          double dsrif = s.h / 2;
-          double ypc = iy[c] < 0.0 ? 0.0 : iy[c];
-          double ypiq = ypc * ypc;
-          int ndiv = (int)(interlen / dsrif + 0.5);
-          if (ndiv < 2) ndiv = 2;
-          double deltas = interlen / ndiv;
-          double xpip = xpmin - 0.5 * deltas;
-          for (int ipt = 1; ipt <= ndiv; ++ipt) {
-            xpip = xpip + deltas;
-            double dxpip = xpip - ix[c];
-            double ris = sqrt(dxpip * dxpip + ypiq);
-            IntWdS = IntWdS + w_kernel(ris, s.h, s.coefke) * deltas;
+    int ib[kMaxCloseSides] = {0, 0, 0, 0};
+    double ix[kMaxCloseSides] = {0.0, 0.0, 0.0, 0.0}, iy[kMaxCloseSides] = {0.0, 0.0, 0.0, 0.0};
+    int nint = 0, gbase = 0;
+    if (on) {
+      double4 x = P.X[p];
+      int clob[kMaxCloseSides];
+      double lx[kMaxCloseSides], ly[kMaxCloseSides];
+      int ncbs = 0;
+      bool overflow = false;
+      for (int isi = 1; isi <= s.nsides; ++isi) {
+        const SideDev& S = sd[isi - 1];
+        double P1P0 = x.x - S.v1[0], P1P1 = x.z - S.v1[1];
+        double sidel = S.length;
+        double xp = P1P0 * S.sss[0] + P1P1 * S.sss[1];
+        double yp = P1P0 * S.nnn[0] + P1P1 * S.nnn[1];
+        double xpmin = -s.doubleh, xpmax = sidel + s.doubleh;
+        double ypmin = -s.doubleh, ypmax = s.doubleh;
+        if ((xpmin < xp && xp < xpmax) && (ypmin < yp && yp < ypmax)) {
+          double ypmx = 0.0, ypmn = 0.0;
+          if (xp < 0.0) {
+            ypmx = sqrt(s.square_doubleh - xp * xp);
+            ypmn = -ypmx;
+          } else if (xp <= sidel) {
+            ypmx = ypmax;
+            ypmn = ypmin;
+          } else if (xp < xpmax) {
+            double L = (sidel - xp) * (sidel - xp);
+            ypmx = sqrt(s.square_doubleh - L);
+            ypmn = -ypmx;
           }
-        }
-        // BoundaryVolumeIntegrals2D.f90
-        double IntWdV = 0.0, D0 = 0.0, D1 = 0.0;
-        double dalfarif = kPigreco / 10;
-        double yplimite = 0.05 * s.h;
-        if (interlen > 0.0) {
-          double ypb = iy[c];
-          if (ypb < yplimite) ypb = yplimite;
-          double alfaA = atan2(xpmin - ix[c], ypb), alfaB = atan2(xpmax - ix[c], ypb);
-          double Intalfa = alfaB - alfaA;
-          int ndiv = (int)(Intalfa / dalfarif + 0.5);
-          if (ndiv < 1) ndiv = 1;
-          double dalfa = Intalfa / ndiv;
-          double alfa_k = alfaA - 0.5 * dalfa;
-          for (int k = 1; k <= ndiv; ++k) {
-            alfa_k = alfa_k + dalfa;
-            double sa = sin(alfa_k), ca = cos(alfa_k);
-            double rb = ypb / ca;
-            double rob = div_rn(rb, s.h, s.rcp_h);
-            double mult = s.h * j2_wro2(rob) * dalfa;
-            D0 = D0 + sa * mult;
-            D1 = D1 - ca * mult;
-            IntWdV = IntWdV + w_integr(rb, s.h) * dalfa;
-          }
-          if (ypb == yplimite) IntWdV = 0.5;
-        }
-        // ComputeVolumeIntegral_WdV2D.f90
-        double IntWdV1 = 0.0;
-        if (interlen > 0.0) {
-          double ypv = iy[c];
-          if (ypv >= yplimite) {
-            double alfaA = atan2(xpmin - ix[c], ypv), alfaB = atan2(xpmax - ix[c], ypv);
-            double Intalfa = alfaB - alfaA;
-            int ndiv = (int)(Intalfa / dalfarif + 0.5);
-            if (ndiv < 2) ndiv = 2;
-            double dalfa = Intalfa / ndiv;
-            double alfa = alfaA - 0.5 * dalfa;
-            for (int ipt = 1; ipt <= ndiv; ++ipt) {
-              alfa = alfa + dalfa;
-              double ta = tan(alfa);
-              double ris = ypv * sqrt(1.0 + ta * ta);
-              IntWdV1 = IntWdV1 + w_integr(ris, s.h) * dalfa;
-            }
-          } else {
-            int jc = 1 - c;  // the other side (nint == 2)
-            double ypj = iy[jc];
-            if (ypj <= yplimite) {
-              double angle = 0.0;
-              if (sd[ib[0] - 1].previous_side == ib[1]) angle = sd[ib[0] - 1].angle;
-              else if (sd[ib[1] - 1].previous_side == ib[0]) angle = sd[ib[1] - 1].angle;
-              else set_status(dyn, 804);
-              IntWdV1 = 0.5 * (angle + kPigreco) / (2.0 * kPigreco);
+          if (ypmn < yp && yp < ypmx) {
+            if (ncbs >= kMaxCloseSides) {
+              overflow = true;
             } else {
-              IntWdV1 = (xpmin >= ix[c] && ix[c] <= xpmax) ? 0.5 : 0.0;
+              clob[ncbs] = isi;
+              lx[ncbs] = xp;
+              ly[ncbs] = yp;
             }
+            ncbs++;
           }
         }
-        const int col[3] = {3, 4, 5};
-        interp_bit2d(3, col, iy[c] / s.h, func);
-        e.bi[0] = IntWdS;
-        e.bi[1] = IntWdV;
-        e.bi[2] = IntWdV1;
-        e.bi[3] = D0;
-        e.bi[4] = D1;
-        e.bi[5] = func[0] / s.squareh;
-        e.bi[6] = func[1] / s.squareh;
-        e.bi[7] = func[2] / s.squareh;
-      } else if (nint == 1) {
-        const int col[5] = {1, 2, 3, 4, 5};
-        interp_bit2d(5, col, iy[c] / s.h, func);
-        e.bi[0] = func[0] / s.h;
-        e.bi[1] = func[1];
-        e.bi[2] = func[1];
-        e.bi[3] = 0.0;
-        e.bi[4] = 0.0;
-        e.bi[5] = func[2] / s.squareh;
-        e.bi[6] = func[3] / s.squareh;
-        e.bi[7] = func[4] / s.squareh;
       }
-      P.bdt[gbase + c] = e;
+      if (overflow) {
+        set_status(dyn, SPH_ERR_CLOSE_SIDES);
+        ncbs = 0;
+      }
+      if (ncbs == 2) {
+        if (sd[clob[0] - 1].previous_side == clob[1]) lx[1] = sd[clob[1] - 1].length - lx[1];
+        else if (sd[clob[1] - 1].previous_side == clob[0]) lx[0] = sd[clob[0] - 1].length - lx[0];
+      }
+      for (int c = 0; c < ncbs; ++c)
+        if (ly[c] > 0.0) {
+          ib[nint] = clob[c];
+          ix[nint] = lx[c];
+          iy[nint] = ly[c];
+          nint++;
+        }
     }
+    if (nint > 0) {
+      if (atomicAdd(&dyn->bdt_sim_used, nint) + nint > s.bdt_quota) {
+        set_status(dyn, SPH_ERR_BDT_OVERFLOW);
+        nint = 0;
+      }
+    }
+    if (nint > 0) {
+      gbase = atomicAdd(&b.dyn[b.nsims].bdt_used, nint);
+      if (gbase + nint > P.bdt_cap) {
+        set_status(dyn, SPH_ERR_BDT_OVERFLOW);
+        nint = 0;
+      }
+    }
+    if (nint > 0) {
+      P.bdt_count[p] = nint;
+      P.bdt_start[p] = gbase;
+    }
+    if (nint == 1 || nint > 2) {
+      for (int c = 0; c < nint; ++c) {
+        BdtEntry e;
+        for (int q = 0; q < 9; ++q) e.ig[q] = 0.0;
+        for (int q = 0; q < 8; ++q) e.bi[q] = 0.0;
+        e.clobonum = ib[c];
+        e.pad = 0;
+        e.loc[0] = ix[c];
+        e.loc[1] = iy[c];
+        e.loc[2] = 0.0;
+        if (nint == 1) {
+          double func[5];
+          const int col[5] = {1, 2, 3, 4, 5};
+          interp_bit2d(5, col, iy[c] / s.h, func);
+          e.bi[0] = func[0] / s.h;
+          e.bi[1] = func[1];
+          e.bi[2] = func[1];
+          e.bi[5] = func[2] / s.squareh;
+          e.bi[6] = func[3] / s.squareh;
+          e.bi[7] = func[4] / s.squareh;
+        }
+        P.bdt[gbase + c] = e;
+      }
+    }
+    if (threadIdx.x == 0) ncorner = 0;
+    __syncthreads();
+    if (nint == 2) {
+      const int c = atomicAdd(&ncorner, 1);
+      corner_ib[c][0] = ib[0];
+      corner_ib[c][1] = ib[1];
+      corner_xy[c][0] = ix[0];
+      corner_xy[c][1] = ix[1];
+      corner_xy[c][2] = iy[0];
+      corner_xy[c][3] = iy[1];
+      corner_base[c] = gbase;
+    }
+    __syncthreads();
+    for (int c = threadIdx.x >> 5; c < ncorner; c += kBlock / 32)
+      corner_integrals2d(s, sd, dyn, corner_ib[c], corner_xy[c], corner_xy[c] + 2, P.bdt + corner_base[c]);
+    __syncthreads();
   }
 }
 
