@@ -73,7 +73,6 @@ struct HostSim {
   std::vector<EdgeDev> edges;          // convex edges (3D)
   std::vector<double> bit;             // 256 x 7
   std::vector<int> cf_count, cf_start, cf_list;
-  std::vector<uint8_t> near;
   int cap = 0;
 };
 
@@ -528,26 +527,28 @@ int prepare_sim(const SphParams& prm, const SphGeometry& g, int cap, HostSim& hs
         }
       }
     }
+    // FindCloseBoundaryFaces3D visits the 27 cells around a particle's (x,
+    // then y, then z) and takes a face at its first visit: one list per
+    // cell, in that order
+    std::vector<uint8_t> near(s.ncells, 0);
+    auto around = [&](int key, auto&& visit) {
+      const int k = key % s.ncd[2] + 1, i = key / s.ncd[2] % s.ncd[0] + 1, j = key / s.ncd[2] / s.ncd[0] + 1;
+      for (int a = std::max(i - 1, 1); a <= std::min(i + 1, s.ncd[0]); ++a)
+        for (int bq = std::max(j - 1, 1); bq <= std::min(j + 1, s.ncd[1]); ++bq)
+          for (int c = std::max(k - 1, 1); c <= std::min(k + 1, s.ncd[2]); ++c) visit(cell_key_local(s, a, bq, c));
+    };
+    for (int key = 0; key < s.ncells; ++key)
+      if (!per[key].empty()) around(key, [&](int q) { near[q] = 1; });
     for (int key = 0; key < s.ncells; ++key) {
       hs.cf_start[key] = (int)hs.cf_list.size();
-      hs.cf_count[key] = (int)per[key].size();
-      hs.cf_list.insert(hs.cf_list.end(), per[key].begin(), per[key].end());
+      if (!near[key]) continue;
+      around(key, [&](int q) {
+        for (int nf : per[q])
+          if (std::find(hs.cf_list.begin() + hs.cf_start[key], hs.cf_list.end(), nf) == hs.cf_list.end())
+            hs.cf_list.push_back(nf);
+      });
+      hs.cf_count[key] = (int)hs.cf_list.size() - hs.cf_start[key];
     }
-    // a cell needs the face search when any of its 27 neighbours is cut
-    hs.near.assign(s.ncells + 1, 0);
-    for (int k = 1; k <= s.ncd[2]; ++k)
-      for (int j = 1; j <= s.ncd[1]; ++j)
-        for (int i = 1; i <= s.ncd[0]; ++i) {
-          uint8_t any = 0;
-          for (int di = -1; di <= 1 && !any; ++di)
-            for (int dj = -1; dj <= 1 && !any; ++dj)
-              for (int dk = -1; dk <= 1 && !any; ++dk) {
-                int a = i + di, bq = j + dj, c = k + dk;
-                if (a < 1 || a > s.ncd[0] || bq < 1 || bq > s.ncd[1] || c < 1 || c > s.ncd[2]) continue;
-                if (hs.cf_count[cell_key_local(s, a, bq, c)] > 0) any = 1;
-              }
-          hs.near[cell_key_local(s, i, j, k)] = any;
-        }
     s.nfaces = g.n_faces;
   } else {
     // DefineBoundarySideGeometry2D.f90 + BoundaryMassForceMatrix2D.f90 +
@@ -601,7 +602,6 @@ int prepare_sim(const SphParams& prm, const SphGeometry& g, int cap, HostSim& hs
     s.nsides = ns;
     hs.cf_count.assign(s.ncells + 1, 0);
     hs.cf_start.assign(s.ncells + 1, 0);
-    hs.near.assign(s.ncells + 1, 0);
   }
   return SPH_OK;
 }
@@ -650,7 +650,6 @@ struct SphHandle {
   EdgeDev* d_edges = nullptr;
   double* d_bit = nullptr;
   int *d_cf_start = nullptr, *d_cf_count = nullptr, *d_cf_list = nullptr;
-  uint8_t* d_near = nullptr;
   int* d_scan = nullptr;
   int* d_nlist = nullptr;
   int* d_ncount = nullptr;
@@ -751,8 +750,8 @@ int sync_dyn(SphHandle* h) {
 void sort_sequence(SphHandle* h, bool boundary_follows, cudaStream_t st) {
   launch_bin(h->db, KeyKind::Sort, st);
   launch_scan(h->db, h->P.cell_start, true, st);
-  launch_place(h->db, st);
-  launch_rank_permute(h->db, boundary_follows, st);
+  launch_place(h->db, boundary_follows, st);
+  launch_rank_permute(h->db, st);
 }
 
 // CalcVarLength: the neighbour lists and, with C1_BE, the fluid part of
@@ -943,7 +942,6 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   A(h->d_bit, (size_t)nsims * kBitRows * 7);
   A(h->d_cf_start, C);
   A(h->d_cf_count, C);
-  A(h->d_near, C);
   A(P.X, N); A(P.XF, N); A(P.VF, N); A(P.RF, N); A(P.RM, N); A(P.V, N); A(P.RP, N); A(P.I, N); A(P.L, N);
   A(P.X2, N); A(P.V2, N); A(P.P2, N); A(P.I2, N); A(P.L2, N);
   A(P.bdt_count, N); A(P.bdt_start, N); A(P.bdt, bdt_cap);
@@ -979,7 +977,6 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   std::vector<EdgeDev> hed;
   std::vector<double> hbit;
   std::vector<int> cfs(C, 0), cfc(C, 0), cfl;
-  std::vector<uint8_t> nr(C, 0);
   for (int s = 0; s < nsims; ++s) {
     HostSim& hs = h->sims[s];
     hsd[s] = hs.dev;
@@ -991,7 +988,6 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
     for (int k = 0; k < hs.dev.ncells; ++k) {
       cfs[hs.dev.cell_off + k] = base + hs.cf_start[k];
       cfc[hs.dev.cell_off + k] = hs.cf_count[k];
-      nr[hs.dev.cell_off + k] = hs.near[k];
     }
     cfl.insert(cfl.end(), hs.cf_list.begin(), hs.cf_list.end());
   }
@@ -1019,7 +1015,6 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_bit, hbit.data(), sizeof(double) * hbit.size(), cudaMemcpyHostToDevice, q);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_cf_start, cfs.data(), sizeof(int) * C, cudaMemcpyHostToDevice, q);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_cf_count, cfc.data(), sizeof(int) * C, cudaMemcpyHostToDevice, q);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h->d_near, nr.data(), C, cudaMemcpyHostToDevice, q);
   if (e == cudaSuccess && !cfl.empty()) e = cudaMemcpyAsync(h->d_cf_list, cfl.data(), sizeof(int) * cfl.size(), cudaMemcpyHostToDevice, q);
   if (e == cudaSuccess) e = cudaMemsetAsync(P.cell_count, 0, sizeof(int) * (C + 1), q);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->d_scan, 0, sizeof(int) * nb, q);
@@ -1047,7 +1042,6 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   b.cf_start = h->d_cf_start;
   b.cf_count = h->d_cf_count;
   b.cf_list = h->d_cf_list;
-  b.cell_near = h->d_near;
   b.scan_block_sums = h->d_scan;
   b.counters = h->d_counters;
   b.nlist = h->d_nlist;
@@ -1136,7 +1130,7 @@ int upload_and_initialise(SphHandle* h, const SphState* states) {
   launch_init_rest(h->db, h->d_cv, h->d_crho, h->d_cp, q3);
   launch_bin(h->db, KeyKind::Sort, q);
   launch_scan(h->db, h->P.cell_start, true, q);
-  launch_place(h->db, q);
+  launch_place(h->db, true, q);
   launch_rank_permute_positions(h->db, q);
   SPH_CUDA(cudaEventRecord(h->ev_sorted, q));
   SPH_CUDA(cudaStreamWaitEvent(q3, h->ev_sorted, 0));

@@ -80,9 +80,8 @@ __device__ __forceinline__ bool particle_cell(const SimDev& s, double x, double 
 // FP32 offset of a particle from the origin of its cell; w holds the cell's
 // k index as a float (exact: k < 2^24), so cell differences are FP32
 // subtractions, exact, with no integer-to-float conversion in the pair loops.
-__device__ __forceinline__ float4 screening_copy(const SimDev& s, const double4& x) {
-  int i, j, k;
-  if (!particle_cell(s, x.x, x.y, x.z, i, j, k)) return make_float4(0.f, 0.f, 0.f, -8.0f);
+__device__ __forceinline__ float4 screening_copy(const SimDev& s, const double4& x, bool inside, int i, int j, int k) {
+  if (!inside) return make_float4(0.f, 0.f, 0.f, -8.0f);
   double ox = s.extr_lo[0] + s.dcd[0] * (i + s.ioff - 1);
   double oy = (s.dim == 3) ? s.extr_lo[1] + s.dcd[1] * (j - 1) : 0.0;
   double oz = s.extr_lo[2] + s.dcd[2] * (k - 1);
@@ -424,14 +423,24 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(DevBatch b, int n, int nb
   }
 }
 
+__device__ __forceinline__ void reset_boundary_counters(const DevBatch& b, int sim) {
+  b.dyn[sim].ncbf_max = 0;
+  b.dyn[sim].bdt_sim_used = 0;
+  if (sim == 0) b.dyn[b.nsims].bdt_used = 0;
+}
+
 // Unstable placement by cell (the atomic slot), remembering the source.
-// Also clears the scan's chunk sums for the next binning.
-__global__ void k_place(DevBatch b, const int* __restrict__ cstart, int use_scratch_ids) {
+// Also clears the scan's chunk sums for the next binning and, where the
+// boundary pass follows, that pass's counters.
+__global__ void k_place(DevBatch b, const int* __restrict__ cstart, int use_scratch_ids, int boundary_follows) {
   __shared__ SimDev s;
   int cur = -1;
   const Particles& P = b.P;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < b.scan_nblocks; c += gridDim.x * blockDim.x)
     b.scan_block_sums[c] = 0;
+  if (boundary_follows)
+    for (int sim = blockIdx.x * blockDim.x + threadIdx.x; sim < b.nsims; sim += gridDim.x * blockDim.x)
+      reset_boundary_counters(b, sim);
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
@@ -458,26 +467,14 @@ __global__ void k_place(DevBatch b, const int* __restrict__ cstart, int use_scra
 // kPermuteRest gathers the rest through it.
 constexpr int kPermuteAll = 0, kPermutePositions = 1, kPermuteRest = 2;
 
-// The last launch of a sort also clears counters: the out-of-grid count for
-// the next binning and, where the boundary pass follows at once, that
-// pass's own.
-__device__ __forceinline__ void reset_boundary_counters(const DevBatch& b, int sim) {
-  b.dyn[sim].ncbf_max = 0;
-  b.dyn[sim].bdt_sim_used = 0;
-  if (sim == 0) b.dyn[b.nsims].bdt_used = 0;
-}
-
 template <int PART>
-__global__ void k_rank_permute(DevBatch b, int boundary_follows) {
+__global__ void __launch_bounds__(kBlock) k_rank_permute(DevBatch b) {
   __shared__ SimDev s;
   int cur = -1;
   const Particles& P = b.P;
-  if (PART != kPermuteRest) {
-    for (int sim = blockIdx.x * blockDim.x + threadIdx.x; sim < b.nsims; sim += gridDim.x * blockDim.x) {
+  if (PART != kPermuteRest)   // the out-of-grid count, for the next binning
+    for (int sim = blockIdx.x * blockDim.x + threadIdx.x; sim < b.nsims; sim += gridDim.x * blockDim.x)
       b.dyn[sim].n_out = 0;
-      if (boundary_follows) reset_boundary_counters(b, sim);
-    }
-  }
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
@@ -502,7 +499,9 @@ __global__ void k_rank_permute(DevBatch b, int boundary_follows) {
     double4 x = P.X2[src];
     if (PART != kPermuteRest) {
       P.X[fin] = x;
-      P.XF[fin] = screening_copy(s, x);
+      int ic, jc, kc;
+      const bool inside = particle_cell(s, x.x, x.y, x.z, ic, jc, kc);
+      P.XF[fin] = screening_copy(s, x, inside, ic, jc, kc);
       P.L[fin] = P.L2[src];
     }
     if (PART != kPermutePositions) {
@@ -570,89 +569,198 @@ struct FaceTest {
   }
 };
 
-__device__ void face_integrals(const SimDev& s, const double* __restrict__ bit, const FaceDev& f,
-                               const double* locx, BdtEntry& e) {
+// The hemisphere table as the quadrature reads it.  coef(q, l, .) are the
+// factors of point q in the three sums of lane l: (1, 1, r2 r2), (r0, r1,
+// r2), (r0 r0, r0 r1, r0 r2) and (r1 r1, r1 r2, r2 r2).
+struct SharedBit {
+  const double (*xy)[2];      // [256] x, y of the points
+  const double (*ring)[2];    // [8] z and weight of a ring's points (the same for all of them)
+  const double (*cf)[12];     // [256] the factors, lane by lane
+  __device__ __forceinline__ double x(int q) const { return xy[q][0]; }
+  __device__ __forceinline__ double y(int q) const { return xy[q][1]; }
+  __device__ __forceinline__ double z(int r) const { return ring[r][0]; }
+  __device__ __forceinline__ double da(int r) const { return ring[r][1]; }
+  __device__ __forceinline__ void coef(int q, int l, double* c) const {
+    for (int k = 0; k < 3; ++k) c[k] = cf[q][3 * l + k];
+  }
+};
+
+struct GlobalBit {
+  const double* bit;          // [256][7] of the simulation
+  __device__ __forceinline__ double x(int q) const { return bit[7 * q]; }
+  __device__ __forceinline__ double y(int q) const { return bit[7 * q + 1]; }
+  __device__ __forceinline__ double z(int r) const { return bit[7 * 32 * r + 2]; }
+  __device__ __forceinline__ double da(int r) const { return bit[7 * 32 * r + 3]; }
+  __device__ __forceinline__ void coef(int q, int l, double* c) const { factors(bit + 7 * q, l, c); }
+  __device__ static __forceinline__ void factors(const double* row, int l, double* c) {
+    const double r0 = row[4], r1 = row[5], r2 = row[6];
+    c[0] = l == 0 ? 1.0 : (l == 1 ? r0 : (l == 2 ? r0 * r0 : r1 * r1));
+    c[1] = l == 0 ? 1.0 : (l == 1 ? r1 : (l == 2 ? r0 * r1 : r1 * r2));
+    c[2] = l == 0 ? r2 * r2 : (l == 1 ? r2 : (l == 2 ? r0 * r2 : r2 * r2));
+  }
+};
+
+// ComputeBoundaryVolumeIntegrals_P0.f90:81-155 for one (particle, face) by
+// four neighbouring lanes.  Its 256 points add to twelve sums one after the
+// other; each lane keeps three of them (l = 0: IntWdV, IntdWrm1dV,
+// IntGWZrm1dV; 1: G; 2: R00, R01, R02; 3: R11, R12, R22), every sum in the
+// reference's order.  The points' tests are shared out over the lanes, and
+// left out for a face that the whole projected hemisphere lies inside
+// (`whole`, with a margin far above the test's rounding): most entries of a
+// wall that is large against 2h.  The chain of one entry is what bounds
+// this pass: by one lane (12 sums, 256 tests and the products of the
+// factors, which come from the table here) it took 65 us at 13,500
+// particles and 143 us at 864,000.
+template <class BIT>
+__device__ __forceinline__ void face_integrals(const SimDev& s, const BIT& bit, const FaceDev& f, const double* locx,
+                                               int l, double* sum) {
   FaceTest ft;
   ft.load(f);
-  double IntWdV = 0.0, IntdWrm1dV = 0.0, IntGWZrm1dV = 0.0;
-  double G0 = 0.0, G1 = 0.0, G2 = 0.0;
-  double R00 = 0.0, R01 = 0.0, R02 = 0.0, R11 = 0.0, R12 = 0.0, R22 = 0.0;
-  double J0 = 0.0, J1 = 0.0, J2 = 0.0, J3 = 0.0;
-  double L0 = locx[0], L1 = locx[1], L2 = locx[2];
-  if (!(L2 < 0.0)) {
-    if (L2 < s.zpmin) L2 = s.zpmin;
-    double robpre = 2.1;
-    for (int ring = 0; ring < 8; ++ring) {
-      const double* row0 = bit + ring * 32 * 7;
-      double zp = row0[2];
-      double lpj2 = L2 + zp;
-      if (!(lpj2 <= 0.0)) continue;       // the whole ring lies above the face plane
-      double tsegnato = L2 / (L2 - lpj2);
-      // The points of a ring share their polar angle, so their distances to
-      // the particle differ by rounding only (s.ring_skip bounds that far
-      // below 1e-6 in rob).  After the ring's first inside point the
-      // refresh test |rob - robpre| > 1e-3 is therefore false for every
-      // later point -- unless the first point missed the threshold by less
-      // than 1e-6, when the ring is tested point by point.  Skipping the
-      // test skips its distance, square root and division.
-      bool test_all = !s.ring_skip, first = true;
-      for (int q = 0; q < 32; ++q) {
-        const double* row = row0 + q * 7;
-        double lpj0 = L0 + row[0];
-        double lpj1 = L1 + row[1];
-        double px0 = L0 + (lpj0 - L0) * tsegnato;
-        double px1 = L1 + (lpj1 - L1) * tsegnato;
-        if (!ft.inside(px0, px1)) continue;
-        if (first || test_all) {
-          double d0 = px0 - L0, d1 = px1 - L1, d2 = 0.0 - L2;
-          double dist = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-          double rob = div_rn(dist, s.h, s.rcp_h);
-          const double gap = fabs(rob - robpre);
-          if (first && !(gap > 1.0e-3) && gap > 1.0e-3 - 1.0e-6) test_all = true;
-          first = false;
-          if (gap > 1.0e-3) {
-            double iv[4];
-            interpolate_table(s, rob, iv);
-            double da = row[3];
-            J0 = iv[0] * da;
-            J1 = iv[1] * da;
-            J2 = iv[2] * da;
-            J3 = iv[3] * da;
-            robpre = rob;
-          }
-        }
-        double r0 = row[4], r1 = row[5], r2 = row[6];
-        double RZ2 = r2 * r2;
-        IntWdV = IntWdV + J0;
-        IntdWrm1dV = IntdWrm1dV + J1;
-        IntGWZrm1dV = IntGWZrm1dV + RZ2 * J1;
-        G0 = G0 + r0 * J2;
-        R00 = R00 + r0 * r0 * J3;
-        R01 = R01 + r0 * r1 * J3;
-        R02 = R02 + r0 * r2 * J3;
-        G1 = G1 + r1 * J2;
-        R11 = R11 + r1 * r1 * J3;
-        R12 = R12 + r1 * r2 * J3;
-        G2 = G2 + r2 * J2;
-        R22 = R22 + r2 * r2 * J3;
-      }
+  sum[0] = sum[1] = sum[2] = 0.0;
+  const double L0 = locx[0], L1 = locx[1];
+  double L2 = locx[2];
+  if (L2 < 0.0) return;
+  if (L2 < s.zpmin) L2 = s.zpmin;
+  const unsigned group = 0xfu << (threadIdx.x & 28);
+  bool whole;
+  {
+    // a projected point lies within 2h of (L0, L1); the test's coordinates
+    // are linear in it
+    const double R = s.doubleh * 1.000001, u = fabs(ft.u);
+    const double k0 = (ft.a0 + ft.b0 * L0 + ft.c0 * L1) * ft.u, k1 = (ft.a1 + ft.b1 * L0 + ft.c1 * L1) * ft.u;
+    const double d0 = (fabs(ft.b0) + fabs(ft.c0)) * R * u, d1 = (fabs(ft.b1) + fabs(ft.c1)) * R * u;
+    const double m = 1.0e-12 + 1.0e-12 * u * (fabs(ft.a0) + fabs(ft.a1) + (fabs(ft.b0) + fabs(ft.b1)) * (fabs(L0) + R) +
+                                              (fabs(ft.c0) + fabs(ft.c1)) * (fabs(L1) + R));
+    whole = k0 - d0 > m && k0 + d0 < 1.0 - m && k1 - d1 > m && k1 + d1 < 1.0 - m;
+    if (ft.fkod == 1) {
+      const double k2 = 1.0 - (k0 + k1), d2 = d0 + d1, m2 = 2.0 * m;
+      whole = whole && k2 - d2 > m2 && k2 + d2 < 1.0 - m2;
     }
-    if (L2 == s.zpmin) IntWdV = point_internal(f, L0, L1) ? 0.5 : 0.0;
   }
-  e.bi[0] = 0.0;
-  e.bi[1] = IntWdV;
-  e.bi[2] = IntdWrm1dV;
-  e.bi[3] = G0;
-  e.bi[4] = G1;
-  e.bi[5] = G2;
-  e.bi[6] = IntGWZrm1dV;
-  e.bi[7] = 0.0;
-  e.ig[0] = R00; e.ig[1] = R01; e.ig[2] = R02;
-  e.ig[3] = R01; e.ig[4] = R11; e.ig[5] = R12;
-  e.ig[6] = R02; e.ig[7] = R12; e.ig[8] = R22;
+  double J0 = 0.0, J1 = 0.0, J2 = 0.0, J3 = 0.0;   // the kernel-table values of the last refresh
+  double Ja = 0.0, Jb = 0.0;                       // this lane's: of its first sum, of the other two
+  double robpre = 2.1;
+  for (int ring = 0; ring < 8; ++ring) {
+    const double zp = bit.z(ring);
+    const double lpj2 = L2 + zp;
+    if (!(lpj2 <= 0.0)) continue;       // the whole ring lies above the face plane
+    const double tsegnato = L2 / (L2 - lpj2);
+    const int q0 = ring * 32;
+    auto project = [&](int q, double& px0, double& px1) {
+      const double lpj0 = L0 + bit.x(q), lpj1 = L1 + bit.y(q);
+      px0 = L0 + (lpj0 - L0) * tsegnato;
+      px1 = L1 + (lpj1 - L1) * tsegnato;
+    };
+    unsigned in = 0xffffffffu;
+    if (!whole) {
+      in = 0u;
+      for (int k = 0; k < 8; ++k) {
+        const int q = 4 * k + l;
+        double px0, px1;
+        project(q0 + q, px0, px1);
+        if (ft.inside(px0, px1)) in |= 1u << q;
+      }
+      in |= __shfl_xor_sync(group, in, 1);
+      in |= __shfl_xor_sync(group, in, 2);
+    }
+    if (in == 0u) continue;
+    // |rob - robpre| > 1e-3 at point q: new table values
+    auto refresh = [&](int q) {
+      double px0, px1;
+      project(q, px0, px1);
+      const double d0 = px0 - L0, d1 = px1 - L1, d2 = 0.0 - L2;
+      const double dist = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
+      const double rob = div_rn(dist, s.h, s.rcp_h);
+      const double gap = fabs(rob - robpre);
+      if (gap > 1.0e-3) {
+        double iv[4];
+        interpolate_table(s, rob, iv);
+        const double da = bit.da(ring);
+        J0 = iv[0] * da;
+        J1 = iv[1] * da;
+        J2 = iv[2] * da;
+        J3 = iv[3] * da;
+        Ja = l == 0 ? J0 : (l == 1 ? J2 : J3);
+        Jb = l == 0 ? J1 : (l == 1 ? J2 : J3);
+        robpre = rob;
+      }
+      return gap;
+    };
+    auto add = [&](int q) {
+      double c[3];
+      bit.coef(q, l, c);
+      sum[0] = sum[0] + c[0] * Ja;
+      sum[1] = sum[1] + c[1] * Jb;
+      sum[2] = sum[2] + c[2] * Jb;
+    };
+    // The points of a ring share their polar angle, so their distances to
+    // the particle differ by rounding only (s.ring_skip bounds that far
+    // below 1e-6 in rob).  After the ring's first inside point the
+    // refresh test |rob - robpre| > 1e-3 is therefore false for every
+    // later point -- unless the first point missed the threshold by less
+    // than 1e-6, when the ring is tested point by point.  Skipping the
+    // test skips its distance, square root and division.
+    const double gap = refresh(q0 + __ffs(in) - 1);
+    const bool test_all = !s.ring_skip || (!(gap > 1.0e-3) && gap > 1.0e-3 - 1.0e-6);
+    if (test_all) {
+      bool first = true;
+      for (int q = 0; q < 32; ++q) {
+        if (!((in >> q) & 1u)) continue;
+        if (!first) refresh(q0 + q);
+        first = false;
+        add(q0 + q);
+      }
+    } else if (in == 0xffffffffu) {
+#pragma unroll 8
+      for (int q = 0; q < 32; ++q) add(q0 + q);
+    } else {
+      for (int q = 0; q < 32; ++q)
+        if ((in >> q) & 1u) add(q0 + q);
+    }
+  }
+  if (l == 0 && L2 == s.zpmin) sum[0] = point_internal(f, L0, L1) ? 0.5 : 0.0;
 }
 
-// ComputeBoundaryDataTab_3D.f90:67-105 with FindCloseBoundaryFaces3D.f90:79-188.
+// Room for n boundary entries of each lane's particle (one simulation to a
+// warp): the first entry, or -1 where n is 0 or there is none.  Each
+// simulation draws on its own quota of the shared pool first, so one that
+// overflows fails alone and the others' entries are unaffected.  One
+// addition per warp and counter: a lane's own met all the others at one
+// address (72 us for the 864,000-particle dam break's face search).
+__device__ __forceinline__ int claim_entries(const SimDev& s, const DevBatch& b, SimDyn* dyn, int n) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (!__any_sync(FULL, n > 0)) return -1;
+  auto scan = [&](int v) {
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(FULL, v, o);
+      if (lane >= o) v += u;
+    }
+    return v;
+  };
+  int inc = scan(n), base = 0;
+  if (lane == 31) base = atomicAdd(&dyn->bdt_sim_used, inc);
+  base = __shfl_sync(FULL, base, 31);
+  if (n > 0 && base + inc > s.bdt_quota) {
+    set_status(dyn, SPH_ERR_BDT_OVERFLOW);
+    n = 0;
+  }
+  inc = scan(n);
+  if (lane == 31) base = atomicAdd(&b.dyn[b.nsims].bdt_used, inc);  // global allocation counter
+  base = __shfl_sync(FULL, base, 31);
+  if (n > 0 && base + inc > b.P.bdt_cap) {
+    set_status(dyn, SPH_ERR_BDT_OVERFLOW);
+    n = 0;
+  }
+  return n > 0 ? base + inc - n : -1;
+}
+
+// ComputeBoundaryDataTab_3D.f90:67-105 with FindCloseBoundaryFaces3D.f90:79-188:
+// a particle's close faces, in the order the 27 cells around its cell name
+// them, become entries of the boundary table (their integrals are a pass of
+// their own).  The host has merged the 27 cells' face lists into one list
+// per cell, each face at its first place: a particle reads that list instead
+// of 27.
 __global__ void __launch_bounds__(kBlock) k_boundary3d(DevBatch b) {
   __shared__ SimDev s;
   int cur = -1;
@@ -660,65 +768,48 @@ __global__ void __launch_bounds__(kBlock) k_boundary3d(DevBatch b) {
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
-    if (threadIdx.x >= tl.count) continue;
-    int p = tl.start + threadIdx.x;
+    const int p = tl.start + threadIdx.x;
+    const bool slot = threadIdx.x < tl.count;
     SimDyn* dyn = b.dyn + tl.sim;
-    P.bdt_count[p] = 0;
-    if (p >= s.p_off + dyn->nag || s.nfaces == 0) continue;
-    double4 x = P.X[p];
-    int ic, jc, kc;
-    if (!particle_cell(s, x.x, x.y, x.z, ic, jc, kc)) continue;
-    if (!b.cell_near[s.cell_off + cell_key_local(s, ic, jc, kc)]) continue;
     int clob[kMaxLocalFaces];
     double pin[kMaxLocalFaces];
     int ncbf = 0;
-    bool overflow = false;
-    for (int i = ic - 1; i <= ic + 1; ++i)
-      for (int j = jc - 1; j <= jc + 1; ++j)
-        for (int k = kc - 1; k <= kc + 1; ++k) {
-          if (i < 1 || i > s.ncd[0] || j < 1 || j > s.ncd[1] || k < 1 || k > s.ncd[2]) continue;
-          int gk = s.cell_off + cell_key_local(s, i, j, k);
-          int nf = b.cf_count[gk];
-          int fs = b.cf_start[gk];
-          for (int q = 0; q < nf; ++q) {
-            int fid = b.cf_list[fs + q];
-            bool there = false;
-            for (int u = 0; u < ncbf && u < kMaxLocalFaces; ++u) there |= (clob[u] == fid);
-            if (there) continue;
-            const FaceDev& f = b.faces[s.face_off + fid - 1];
-            double pn = 0.0;
-            pn = pn + f.T[0][2] * (x.x - f.GXref[0]);
-            pn = pn + f.T[1][2] * (x.y - f.GXref[1]);
-            pn = pn + f.T[2][2] * (x.z - f.GXref[2]);
-            if (pn >= 0.0 && pn < s.doubleh) {
-              if (ncbf >= s.maxcb || ncbf >= kMaxLocalFaces) {
-                overflow = true;
-              } else {
-                clob[ncbf] = fid;
-                pin[ncbf] = pn;
-              }
-              ncbf++;
-            }
+    double4 x = make_double4(0.0, 0.0, 0.0, 0.0);
+    int ic, jc, kc;
+    if (slot && p < s.p_off + dyn->nag && s.nfaces > 0) x = P.X[p];
+    if (slot && p < s.p_off + dyn->nag && s.nfaces > 0 && particle_cell(s, x.x, x.y, x.z, ic, jc, kc)) {
+      const int gk = s.cell_off + cell_key_local(s, ic, jc, kc);
+      const int nf = b.cf_count[gk];
+      const int fs = nf > 0 ? b.cf_start[gk] : 0;
+      bool overflow = false;
+      for (int q = 0; q < nf; ++q) {
+        const int fid = b.cf_list[fs + q];
+        const FaceDev& f = b.faces[s.face_off + fid - 1];
+        double pn = 0.0;
+        pn = pn + f.T[0][2] * (x.x - f.GXref[0]);
+        pn = pn + f.T[1][2] * (x.y - f.GXref[1]);
+        pn = pn + f.T[2][2] * (x.z - f.GXref[2]);
+        if (pn >= 0.0 && pn < s.doubleh) {
+          if (ncbf >= s.maxcb || ncbf >= kMaxLocalFaces) {
+            overflow = true;
+          } else {
+            clob[ncbf] = fid;
+            pin[ncbf] = pn;
           }
+          ncbf++;
         }
-    if (overflow) {
-      set_status(dyn, SPH_ERR_CLOSE_FACES);
-      continue;
+      }
+      if (overflow) {
+        set_status(dyn, SPH_ERR_CLOSE_FACES);
+        ncbf = 0;
+      }
     }
+    const int gbase = claim_entries(s, b, dyn, ncbf);
+    if (gbase < 0) ncbf = 0;
+    if (slot) P.bdt_count[p] = ncbf;
+    const int most = warp_max(ncbf);
+    if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(&dyn->ncbf_max, most);
     if (ncbf == 0) continue;
-    // each simulation draws on its own quota of the shared pool first, so
-    // one that overflows fails alone and the others' entries are unaffected
-    if (atomicAdd(&dyn->bdt_sim_used, ncbf) + ncbf > s.bdt_quota) {
-      set_status(dyn, SPH_ERR_BDT_OVERFLOW);
-      continue;
-    }
-    int gbase = atomicAdd(&b.dyn[b.nsims].bdt_used, ncbf);  // global allocation counter
-    if (gbase + ncbf > P.bdt_cap) {
-      set_status(dyn, SPH_ERR_BDT_OVERFLOW);
-      continue;
-    }
-    atomicMax(&dyn->ncbf_max, ncbf);
-    P.bdt_count[p] = ncbf;
     P.bdt_start[p] = gbase;
     for (int u = 0; u < ncbf; ++u) {
       const FaceDev& f = b.faces[s.face_off + clob[u] - 1];
@@ -742,38 +833,68 @@ __global__ void __launch_bounds__(kBlock) k_boundary3d(DevBatch b) {
 }
 
 // ComputeBoundaryVolumeIntegrals_P0.f90:81-155 for every entry the find
-// pass allocated, one (particle, face) per thread: the quadrature costs are
+// pass allocated, four lanes to a (particle, face): the quadrature costs are
 // balanced across the GPU whatever the particles' distribution over tiles.
 __global__ void __launch_bounds__(128) k_boundary3d_integrals(DevBatch b) {
   // the simulation constants and hemisphere table of the chunk's first
   // entry, staged in shared memory (a batch chunk can mix simulations:
   // entries of another one read theirs from global memory)
   __shared__ SimDev ssim;
-  __shared__ double sbit[kBitRows * 7];
+  __shared__ double sxy[kBitRows][2];
+  __shared__ double sring[8][2];
+  __shared__ double scf[kBitRows][12];
   int loaded = -1;
   int used = b.dyn[b.nsims].bdt_used;
   if (used > b.P.bdt_cap) used = b.P.bdt_cap;
-  for (int base = blockIdx.x * blockDim.x; base < used; base += gridDim.x * blockDim.x) {
+  const int l = threadIdx.x & 3;
+  const int per = blockDim.x / 4;
+  for (int base = blockIdx.x * per; base < used; base += gridDim.x * per) {
     const int first = b.P.bdt[base].pad;
     if (first != loaded) {
       load_sim(ssim, b.sims, first, loaded);
       const double* src = b.bit + (size_t)first * kBitRows * 7;
-      for (int i = threadIdx.x; i < kBitRows * 7; i += blockDim.x) sbit[i] = src[i];
+      for (int q = threadIdx.x; q < kBitRows; q += blockDim.x) {
+        const double* row = src + 7 * q;
+        sxy[q][0] = row[0];
+        sxy[q][1] = row[1];
+        if ((q & 31) == 0) {
+          sring[q >> 5][0] = row[2];
+          sring[q >> 5][1] = row[3];
+        }
+        for (int k = 0; k < 4; ++k) GlobalBit::factors(row, k, &scf[q][3 * k]);
+      }
       __syncthreads();
     }
-    const int idx = base + threadIdx.x;
+    const int idx = base + (threadIdx.x >> 2);
     if (idx >= used) continue;
     BdtEntry& e = b.P.bdt[idx];
     const int sim = e.pad;
-    const bool mine = sim == loaded;
-    const SimDev& s = mine ? ssim : b.sims[sim];
-    const double* bit = mine ? sbit : b.bit + (size_t)sim * kBitRows * 7;
-    const FaceDev& f = b.faces[s.face_off + e.clobonum - 1];
-    double locx[3] = {e.loc[0], e.loc[1], e.loc[2]};
-    BdtEntry r;
-    face_integrals(s, bit, f, locx, r);
-    for (int q = 0; q < 8; ++q) e.bi[q] = r.bi[q];
-    for (int q = 0; q < 9; ++q) e.ig[q] = r.ig[q];
+    const double locx[3] = {e.loc[0], e.loc[1], e.loc[2]};
+    double sum[3];
+    if (sim == loaded) {
+      face_integrals(ssim, SharedBit{sxy, sring, scf}, b.faces[ssim.face_off + e.clobonum - 1], locx, l, sum);
+    } else {
+      const SimDev& s = b.sims[sim];
+      face_integrals(s, GlobalBit{b.bit + (size_t)sim * kBitRows * 7}, b.faces[s.face_off + e.clobonum - 1], locx, l,
+                     sum);
+    }
+    if (l == 0) {
+      e.bi[0] = 0.0;
+      e.bi[1] = sum[0];
+      e.bi[2] = sum[1];
+      e.bi[6] = sum[2];
+      e.bi[7] = 0.0;
+    } else if (l == 1) {
+      for (int k = 0; k < 3; ++k) e.bi[3 + k] = sum[k];
+    } else if (l == 2) {
+      e.ig[0] = sum[0];
+      e.ig[1] = e.ig[3] = sum[1];
+      e.ig[2] = e.ig[6] = sum[2];
+    } else {
+      e.ig[4] = sum[0];
+      e.ig[5] = e.ig[7] = sum[1];
+      e.ig[8] = sum[2];
+    }
   }
 }
 
@@ -996,19 +1117,8 @@ __global__ void __launch_bounds__(kBlock) k_boundary2d(DevBatch b) {
           nint++;
         }
     }
-    if (nint > 0) {
-      if (atomicAdd(&dyn->bdt_sim_used, nint) + nint > s.bdt_quota) {
-        set_status(dyn, SPH_ERR_BDT_OVERFLOW);
-        nint = 0;
-      }
-    }
-    if (nint > 0) {
-      gbase = atomicAdd(&b.dyn[b.nsims].bdt_used, nint);
-      if (gbase + nint > P.bdt_cap) {
-        set_status(dyn, SPH_ERR_BDT_OVERFLOW);
-        nint = 0;
-      }
-    }
+    gbase = claim_entries(s, b, dyn, nint);
+    if (gbase < 0) nint = 0;
     if (nint > 0) {
       P.bdt_count[p] = nint;
       P.bdt_start[p] = gbase;
@@ -4203,24 +4313,24 @@ void upload_bit2d(const double* tab, cudaStream_t st) {
   cudaMemcpyToSymbolAsync(c_bit2d, tab, sizeof(double) * 22 * 6, 0, cudaMemcpyHostToDevice, st);
 }
 
-void launch_place(const DevBatch& b, cudaStream_t st) {
-  k_place<<<blocks_for(b), kBlock, 0, st>>>(b, b.P.cell_start, 1);
+void launch_place(const DevBatch& b, bool boundary_follows, cudaStream_t st) {
+  k_place<<<blocks_for(b), kBlock, 0, st>>>(b, b.P.cell_start, 1, boundary_follows ? 1 : 0);
 }
 
-void launch_rank_permute(const DevBatch& b, bool boundary_follows, cudaStream_t st) {
-  k_rank_permute<kPermuteAll><<<blocks_for(b), kBlock, 0, st>>>(b, boundary_follows ? 1 : 0);
+void launch_rank_permute(const DevBatch& b, cudaStream_t st) {
+  k_rank_permute<kPermuteAll><<<blocks_for(b), kBlock, 0, st>>>(b);
 }
 
 void launch_rank_permute_positions(const DevBatch& b, cudaStream_t st) {
-  k_rank_permute<kPermutePositions><<<blocks_for(b), kBlock, 0, st>>>(b, 1);
+  k_rank_permute<kPermutePositions><<<blocks_for(b), kBlock, 0, st>>>(b);
 }
 
 void launch_rank_permute_rest(const DevBatch& b, cudaStream_t st) {
-  k_rank_permute<kPermuteRest><<<blocks_for(b), kBlock, 0, st>>>(b, 0);
+  k_rank_permute<kPermuteRest><<<blocks_for(b), kBlock, 0, st>>>(b);
 }
 
 void launch_rank_reference(const DevBatch& b, const int* cell_start_ref, int* npartord, cudaStream_t st) {
-  k_place<<<blocks_for(b), kBlock, 0, st>>>(b, cell_start_ref, 0);
+  k_place<<<blocks_for(b), kBlock, 0, st>>>(b, cell_start_ref, 0, 0);
   k_rank_reference<<<blocks_for(b), kBlock, 0, st>>>(b, cell_start_ref, npartord);
 }
 
@@ -4228,7 +4338,7 @@ void launch_boundary(const DevBatch& b, bool cleared, cudaStream_t st) {
   if (!cleared) k_bdt_reset<<<(b.nsims + 127) / 128, 128, 0, st>>>(b);
   if (b.dim == 3) {
     k_boundary3d<<<blocks_for(b, kGridBoundary), kBlock, 0, st>>>(b);
-    k_boundary3d_integrals<<<b.grid[kGridIntegrals] > 0 ? b.grid[kGridIntegrals] : b.grid_blocks * 2, 128, 0, st>>>(b);
+    k_boundary3d_integrals<<<b.grid[kGridIntegrals] > 0 ? b.grid[kGridIntegrals] : b.grid_blocks, 128, 0, st>>>(b);
   } else {
     k_boundary2d<<<blocks_for(b, kGridBoundary), kBlock, 0, st>>>(b);
   }

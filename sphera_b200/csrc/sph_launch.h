@@ -22,9 +22,8 @@ struct DevBatch {
   const EdgeDev* edges;    // convex edges of all simulations (3D)
   const double* bit;       // per-sim BoundIntegralTab, 256 x 7 each
   const int* cf_start;     // per global cell: first entry in cf_list
-  const int* cf_count;     // per global cell: faces cutting the cell
-  const int* cf_list;      // face ids (1-based within the simulation)
-  const uint8_t* cell_near;  // per global cell: faces cut the 27-cell block
+  const int* cf_count;     // per global cell: faces cutting the 27 cells around it
+  const int* cf_list;      // face ids (1-based within the simulation), in visiting order
   int* nlist;              // neighbour lists (see k_neighbour_lists)
   int* ncount;             // entries per particle
   int list_cap4;           // 4-entry chunks reserved per particle (max NMAXPARTJ / 4)
@@ -49,9 +48,9 @@ void launch_stage(const DevBatch& b, cudaStream_t st);
 void launch_bin(const DevBatch& b, KeyKind kind, cudaStream_t st);
 void launch_scan(const DevBatch& b, int* cell_start, bool removals, cudaStream_t st);
 void upload_bit2d(const double* tab, cudaStream_t st);
-void launch_place(const DevBatch& b, cudaStream_t st);
 // boundary_follows: clears the boundary pass's counters too
-void launch_rank_permute(const DevBatch& b, bool boundary_follows, cudaStream_t st);
+void launch_place(const DevBatch& b, bool boundary_follows, cudaStream_t st);
+void launch_rank_permute(const DevBatch& b, cudaStream_t st);
 // the IC of an upload: positions first (destinations kept in P.slot), then the rest
 void launch_rank_permute_positions(const DevBatch& b, cudaStream_t st);
 void launch_rank_permute_rest(const DevBatch& b, cudaStream_t st);
