@@ -63,11 +63,29 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
   return r1 == 0.0 ? q1 : __fma_rn(r1, y, q1);
 }
 
+// div_rn without the two selections: the same quotient wherever it is not
+// zero (a zero remainder adds a zero, which changes no nonzero number), and
+// for a zero dividend a zero whose sign is the IEEE one except that -0 over
+// a positive divisor gives +0.  For operands that cannot be -0 and for
+// quotients whose zeros only ever meet a sum that started at +0.  The two
+// compares are FP64 instructions: without them a pair of the FP64 momentum
+// pass is 10 of its 202 FP64 instructions shorter, one of the matrix pass 30
+// of about 230.
+__device__ __forceinline__ double div_rn_unsigned0(double a, double b, double y) {
+  const double q0 = __dmul_rn(a, y);
+  const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+  return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+}
+
+// q >= 1 and q >= 2 for q >= 0, from its upper word (integer instructions).
+__device__ __forceinline__ bool at_least_one(double q) { return __double2hiint(q) >= 0x3ff00000; }
+__device__ __forceinline__ bool at_least_two(double q) { return __double2hiint(q) >= 0x40000000; }
+
 __device__ __forceinline__ bool particle_cell(const SimDev& s, double x, double y, double z, int& i, int& j,
                                               int& k) {
-  double ci = ceil(div_rn(x - s.extr_lo[0], s.dcd[0], s.rcp_dcd[0])) - (double)s.ioff;   // exact: whole numbers
-  double ck = ceil(div_rn(z - s.extr_lo[2], s.dcd[2], s.rcp_dcd[2]));
-  double cj = (s.dim == 3) ? ceil(div_rn(y - s.extr_lo[1], s.dcd[1], s.rcp_dcd[1])) : 1.0;
+  double ci = ceil(div_rn_unsigned0(x - s.extr_lo[0], s.dcd[0], s.rcp_dcd[0])) - (double)s.ioff;   // exact: whole numbers
+  double ck = ceil(div_rn_unsigned0(z - s.extr_lo[2], s.dcd[2], s.rcp_dcd[2]));
+  double cj = (s.dim == 3) ? ceil(div_rn_unsigned0(y - s.extr_lo[1], s.dcd[1], s.rcp_dcd[1])) : 1.0;
   if (!(ci >= 1.0 && ci <= (double)s.ncd[0] && cj >= 1.0 && cj <= (double)s.ncd[1] && ck >= 1.0 &&
         ck <= (double)s.ncd[2]))
     return false;
@@ -108,17 +126,16 @@ __device__ __forceinline__ void neighbour_run(const SimDev& s, const int* __rest
 __device__ __forceinline__ void kernel_values(const SimDev& s, double rijtemp2, double& PK1, double& PK2,
                                               double& PK3) {
   double rijtemp = sqrt(rijtemp2);
-  double rij_su_h = div_rn(rijtemp, s.h, s.rcp_h);
-  double rij_su_h_quad = div_rn(rijtemp2, s.squareh, s.rcp_squareh);
-  int index_rij_su_h = (int)rij_su_h;
+  double rij_su_h = div_rn_unsigned0(rijtemp, s.h, s.rcp_h);
+  double rij_su_h_quad = div_rn_unsigned0(rijtemp2, s.squareh, s.rcp_squareh);
   double denom = 1.0 / (rijtemp + s.eta);
   PK1 = 0.0;
   PK2 = 0.0;
   PK3 = 0.0;
-  if (index_rij_su_h >= 2) return;
+  if (at_least_two(rij_su_h)) return;
   double gradmod = -(2.0 * rij_su_h) + 1.5 * rij_su_h_quad;
   double gradmodwacl = -12.0 - 3.0 * rij_su_h_quad + 12.0 * rij_su_h;
-  if (index_rij_su_h > 0) gradmod = -gradmod + rij_su_h_quad - 2.0;
+  if (at_least_one(rij_su_h)) gradmod = -gradmod + rij_su_h_quad - 2.0;
   gradmod = gradmod * s.ke_coef;
   gradmodwacl = gradmodwacl * s.kacl_coef;
   PK1 = gradmod * denom;
@@ -670,7 +687,7 @@ __device__ __forceinline__ void face_integrals(const SimDev& s, const BIT& bit, 
       project(q, px0, px1);
       const double d0 = px0 - L0, d1 = px1 - L1, d2 = 0.0 - L2;
       const double dist = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-      const double rob = div_rn(dist, s.h, s.rcp_h);
+      const double rob = div_rn_unsigned0(dist, s.h, s.rcp_h);
       const double gap = fabs(rob - robpre);
       if (gap > 1.0e-3) {
         double iv[4];
@@ -1848,7 +1865,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_neighbour_lists(DevBatch b) {
 // division r / h are shared by the range test and both gradients; the
 // constant factors come from the host (SimDev::c1_w*).  The pair's twelve
 // divisions by |r| and rho_j go through one correctly rounded reciprocal
-// of each (div_rn: the IEEE quotients, bit for bit).
+// of each (the IEEE quotients; the sums start at +0, so the sign of a zero
+// term is of no account).
 // The 2D SA-SPH frontier terms of the renormalisation matrices, -RN IntWdV
 // per close side (AddBoundaryContribution_to_CE2D.f90:81-94 for both
 // matrices in every continuity pass; AddBoundaryContributions_to_ME2D.f90:
@@ -1933,28 +1951,28 @@ __global__ void __launch_bounds__(kBlock, 2) k_renormalisation(DevBatch b) {
       const double4 xj = load_record(P.X + q);
       double r[3] = {xj.x - xi.x, xj.y - xi.y, xj.z - xi.z};
       double abs_r = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-      double qh = div_rn(abs_r, s.h, s.rcp_h);
-      if ((int)qh >= 2 || abs_r < s.h * 1.0e-6) continue;
+      double qh = div_rn_unsigned0(abs_r, s.h, s.rcp_h);
+      if (at_least_two(qh) || abs_r < s.h * 1.0e-6) continue;
       const double mj = xj.w, rhoj = P.RP[q].x;
       const double w = 2.0 - qh;
       double go[3];
       // anti-cluster kernel (q <= 2 here)
       const double rcp_r = __drcp_rn(abs_r), rcp_rhoj = __drcp_rn(rhoj);
-      double t = div_rn(-(3.0 * (w * w) * s.c1_w2), s.h, s.rcp_h);
+      double t = div_rn_unsigned0(-(3.0 * (w * w) * s.c1_w2), s.h, s.rcp_h);
       for (int c = 0; c < 3; ++c) {
-        double gw = div_rn(t * r[c], abs_r, rcp_r);
+        double gw = div_rn_unsigned0(t * r[c], abs_r, rcp_r);
         if (DIM == 2) gw = gw * s.h * 4.0 / 3.0;
-        go[c] = div_rn(gw * mj, rhoj, rcp_rhoj);
+        go[c] = div_rn_unsigned0(gw * mj, rhoj, rcp_rhoj);
       }
       for (int c = 0; c < 3; ++c)
         for (int kk = 0; kk < 3; ++kk) Bg[3 * kk + c] = Bg[3 * kk + c] + r[c] * go[kk];
       if (divu) {
         // beta-spline (q < 2 here)
-        t = div_rn(qh <= 1.0 ? s.c1_w1a * (9.0 / 4.0 * (qh * qh) - 3.0 * qh) : -(s.c1_w1b * (w * w)), s.h, s.rcp_h);
+        t = div_rn_unsigned0(qh <= 1.0 ? s.c1_w1a * (9.0 / 4.0 * (qh * qh) - 3.0 * qh) : -(s.c1_w1b * (w * w)), s.h, s.rcp_h);
         for (int c = 0; c < 3; ++c) {
-          double gw = div_rn(t * r[c], abs_r, rcp_r);
+          double gw = div_rn_unsigned0(t * r[c], abs_r, rcp_r);
           if (DIM == 2) gw = gw * s.h * 10.0 / 7.0;
-          go[c] = div_rn(gw * mj, rhoj, rcp_rhoj);
+          go[c] = div_rn_unsigned0(gw * mj, rhoj, rcp_rhoj);
         }
         for (int c = 0; c < 3; ++c)
           for (int kk = 0; kk < 3; ++kk) Bd[3 * kk + c] = Bd[3 * kk + c] + r[c] * go[kk];
@@ -1965,6 +1983,18 @@ __global__ void __launch_bounds__(kBlock, 2) k_renormalisation(DevBatch b) {
       if (divu) store_b(P.BD, total, p, Bd);
     }
   }
+}
+
+// A particle of a finished simulation of a batch: its record as it is, for
+// the step's sort.
+__device__ __forceinline__ void carry_record(const Particles& P, int p) {
+  const double4 v4 = P.V[p];
+  const double2 rp = P.RP[p];
+  P.X2[p] = P.X[p];
+  P.V2[p] = make_double4(v4.x, v4.y, v4.z, rp.x);
+  P.P2[p] = rp.y;
+  P.I2[p] = P.I[p];
+  P.L2[p] = P.L[p];
 }
 
 // C1: with input_any_t%C1_BE the pressure terms are renormalised with
@@ -1988,14 +2018,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_momentum(DevBatch b) {
     int p = tl.start + threadIdx.x;
     bool active = threadIdx.x < tl.count && p < s.p_off + dyn->nag;
     if (FUSED && active && dyn->frozen) {
-      // a finished simulation of a batch: carry the record through the sort
-      double4 v4 = P.V[p];
-      double2 rp = P.RP[p];
-      P.X2[p] = P.X[p];
-      P.V2[p] = make_double4(v4.x, v4.y, v4.z, rp.x);
-      P.P2[p] = rp.y;
-      P.I2[p] = P.I[p];
-      P.L2[p] = P.L[p];
+      carry_record(P, p);
       active = false;
     }
     double4 xi = make_double4(0.0, 0.0, 0.0, 0.0);
@@ -2058,11 +2081,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_momentum(DevBatch b) {
       // the two divisions by rho_i rho_j and the one by rho_i share correctly
       // rounded reciprocals (div_rn: the IEEE quotients, bit for bit)
       const double rr_ij = rhoi * rhoj, rcp_rr = __drcp_rn(rr_ij);
-      double alpha = div_rn(pj - pi, rr_ij, rcp_rr);
+      double alpha = div_rn_unsigned0(pj - pi, rr_ij, rcp_rr);
       tp0 = tp0 + -(amassj * alpha * r0 * PK3);
       if (DIM == 3) tp1 = tp1 + -(amassj * alpha * r1 * PK3);
       tp2 = tp2 + -(amassj * alpha * r2 * PK3);
-      double alpha2 = div_rn(pi * (div_rn(rhoj, rhoi, rcp_rhoi) + 1.0) + pj * (rhoi / rhoj - 1.0), rr_ij, rcp_rr);
+      double alpha2 = div_rn_unsigned0(pi * (div_rn_unsigned0(rhoj, rhoi, rcp_rhoi) + 1.0) + pj * (rhoi / rhoj - 1.0), rr_ij, rcp_rr);
       al0 = al0 - amassj * alpha2 * r0 * PK3;
       if (DIM == 3) al1 = al1 - amassj * alpha2 * r1 * PK3;
       al2 = al2 - amassj * alpha2 * r2 * PK3;
@@ -2867,14 +2890,7 @@ __global__ void __launch_bounds__(kBlock) k_momentum_f32_finish(DevBatch b) {
     int p = tl.start + threadIdx.x;
     bool active = threadIdx.x < tl.count && p < s.p_off + dyn->nag;
     if (FUSED && active && dyn->frozen) {
-      // a finished simulation of a batch: carry the record through the sort
-      double4 v4 = P.V[p];
-      double2 rp = P.RP[p];
-      P.X2[p] = P.X[p];
-      P.V2[p] = make_double4(v4.x, v4.y, v4.z, rp.x);
-      P.P2[p] = rp.y;
-      P.I2[p] = P.I[p];
-      P.L2[p] = P.L[p];
+      carry_record(P, p);
       active = false;
     }
     double dtc = 1.0e300;
@@ -3185,12 +3201,11 @@ __global__ void k_refresh_f32(DevBatch b) {
 // PartKernel(4) of CalcVarLength.f90:241-268: the kernel value W = wu coefke.
 __device__ __forceinline__ double kernel_w(const SimDev& s, double rr) {
   double r = sqrt(rr);
-  double q = div_rn(r, s.h, s.rcp_h);
-  double q2 = div_rn(rr, s.squareh, s.rcp_squareh);
-  int idx = (int)q;
-  if (idx >= 2) return 0.0;
+  double q = div_rn_unsigned0(r, s.h, s.rcp_h);
+  double q2 = div_rn_unsigned0(rr, s.squareh, s.rcp_squareh);
+  if (at_least_two(q)) return 0.0;
   double wu = 0.666666667 + q2 * (q * 0.5 - 1.0);
-  if (idx > 0) wu = (2.0 - q) * (2.0 - q) * (2.0 - q) * 0.166666666667;
+  if (at_least_one(q)) wu = (2.0 - q) * (2.0 - q) * (2.0 - q) * 0.166666666667;
   return wu * s.coefke;
 }
 
