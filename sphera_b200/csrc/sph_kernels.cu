@@ -1480,6 +1480,7 @@ __device__ __forceinline__ void elastic_reaction(const SimDev& s, const DevBatch
 // time and test them in lockstep; each lane keeps the candidates of its own
 // k-1..k+1 window, so its accepted sequence is exactly its reference order.
 // ==========================================================================
+constexpr int kSplitThreads = 128;   // threads of the four-lane FP64 pair passes
 constexpr int kSlotBits = 28;
 constexpr int kSlotMask = (1 << kSlotBits) - 1;
 
@@ -1997,6 +1998,125 @@ __device__ __forceinline__ void carry_record(const Particles& P, int p) {
   P.L2[p] = P.L[p];
 }
 
+// The particle's values that its pairs share.
+struct PairSelf {
+  double4 x;
+  double v[3];
+  double rho, p, rcp_rho, mon;   // mon: alfa_mon (2 c) h
+  bool morris;
+  double nu;
+  __device__ __forceinline__ void load(const SimDev& s, const double4& xi, const double4& vi, double rhoi, double pi) {
+    x = xi;
+    v[0] = vi.x;
+    v[1] = vi.y;
+    v[2] = vi.z;
+    rho = rhoi;
+    p = pi;
+    rcp_rho = __drcp_rn(rhoi);
+    mon = s.alfa_mon * (s.celerita + s.celerita) * s.h;
+    nu = s.kin_visc;
+    morris = nu > 1.0e-12;
+  }
+};
+
+// One pair's terms of the momentum equation, component d handed to
+// add(kind, d, term) as each is formed: kind 0 the pressure gradient, 1 ALE1
+// (to be taken from its sum), 2 Monaghan's and 3 Morris's viscosity.
+template <int DIM, class ADD>
+__device__ __forceinline__ void pair_terms(const SimDev& s, const PairSelf& i, const double4& xj, const double4& vj,
+                                           const double2& rpj, ADD&& add) {
+  double r0 = i.x.x - xj.x, r1 = i.x.y - xj.y, r2 = i.x.z - xj.z;
+  double rr = r0 * r0 + r1 * r1 + r2 * r2;
+  double PK1, PK2, PK3;
+  kernel_values(s, rr, PK1, PK2, PK3);
+  double rhoj = rpj.x, pj = rpj.y, amassj = xj.w;
+  double dv0 = vj.x - i.v[0], dv1 = vj.y - i.v[1], dv2 = vj.z - i.v[2];
+  // pressure gradient and ALE1 terms, inter_EqMoto.f90:195-221
+  // the two divisions by rho_i rho_j and the one by rho_i share correctly
+  // rounded reciprocals (the IEEE quotients; the sums start at +0, so the
+  // sign of a zero term is of no account)
+  const double rr_ij = i.rho * rhoj, rcp_rr = __drcp_rn(rr_ij);
+  double alpha = div_rn_unsigned0(pj - i.p, rr_ij, rcp_rr);
+  add(0, 0, -(amassj * alpha * r0 * PK3));
+  if (DIM == 3) add(0, 1, -(amassj * alpha * r1 * PK3));
+  add(0, 2, -(amassj * alpha * r2 * PK3));
+  double alpha2 = div_rn_unsigned0(i.p * (div_rn_unsigned0(rhoj, i.rho, i.rcp_rho) + 1.0) + pj * (i.rho / rhoj - 1.0),
+                                   rr_ij, rcp_rr);
+  add(1, 0, amassj * alpha2 * r0 * PK3);
+  if (DIM == 3) add(1, 1, amassj * alpha2 * r1 * PK3);
+  add(1, 2, amassj * alpha2 * r2 * PK3);
+  // viscomon.f90:54-73
+  double vrij = (DIM == 3) ? -(dv0 * r0) - dv1 * r1 - dv2 * r2 : -(dv0 * r0) - dv2 * r2;
+  double TermMon = i.mon / (i.rho + rhoj);
+  double mtv = amassj * TermMon * vrij;
+  add(2, 0, mtv * r0 * PK2 + 0.0);
+  if (DIM == 3) add(2, 1, mtv * r1 * PK2 + 0.0);
+  add(2, 2, mtv * r2 * PK2 + 0.0);
+  // viscomorris.f90:60-71
+  if (i.morris) {
+    double rt = i.nu * i.rho + i.nu * rhoj + 1.0e-3;
+    double anuitilde = 4.0 * (i.nu * i.nu);
+    double factivis = amassj * anuitilde / rt;
+    add(3, 0, factivis * (-(dv0 * PK2 * rr)));
+    if (DIM == 3) add(3, 1, factivis * (-(dv1 * PK2 * rr)));
+    add(3, 2, factivis * (-(dv2 * PK2 * rr)));
+  }
+}
+
+// The closing of an FP64 momentum pass for particle p from its sums: the
+// laminar flag, gravity, the elastic reaction and, in the fused step, the
+// leapfrog update and the particle's CFL time.
+template <int DIM, bool FUSED>
+__device__ __forceinline__ void momentum_close(const SimDev& s, const DevBatch& b, SimDyn* dyn, int p,
+                                               const double4& xi, const double* vi, double rhoi, double pi,
+                                               const double* tpres, const double* td, const double* tv,
+                                               const double* rs, double& dtc) {
+  const Particles& P = b.P;
+  const double GI = (double)9.80665f;   // Static_allocation_module.f90:72, a default-REAL literal
+  const double* geff = dyn->geff;
+  const int nb = P.bdt_count[p];
+  const int bstart = nb > 0 ? P.bdt_start[p] : 0;
+  // laminar_flag, inter_EqMoto.f90:269-283
+  int lam_new = 0;
+  if (s.kin_visc > 0.0) {
+    double absv_pres = sqrt(tpres[0] * tpres[0] + tpres[1] * tpres[1] + tpres[2] * tpres[2]) + GI;
+    double absv_morris = sqrt(rs[0] * rs[0] + rs[1] * rs[1] + rs[2] * rs[2]);
+    double weight = 0.0;
+    if (absv_pres != 0.0) weight = absv_morris / absv_pres * 100.0;
+    lam_new = (weight > 5.0 || absv_pres == 0.0) ? 1 : 0;
+  }
+  double acc[3];
+  acc[0] = tpres[0] + td[0] + tv[0] + geff[0];
+  acc[1] = tpres[1] + td[1] + tv[1] + geff[1];
+  acc[2] = tpres[2] + td[2] + tv[2] + geff[2];
+  if (nb > 0) {
+    double R[3];
+    const double xa[3] = {xi.x, xi.y, xi.z};
+    elastic_reaction<DIM>(s, b, nb, bstart, xa, vi, R);
+    for (int d = 0; d < 3; ++d) acc[d] = acc[d] + R[d];
+  }
+  if (FUSED) {
+    double dtvel = dyn->dtvel, dt = dyn->dt;
+    double vn[3], xn[3];
+    for (int d = 0; d < 3; ++d) vn[d] = vi[d] + dtvel * acc[d];
+    xn[0] = xi.x + dt * vn[0];
+    xn[1] = xi.y + dt * vn[1];
+    xn[2] = xi.z + dt * vn[2];
+    P.X2[p] = make_double4(xn[0], xn[1], xn[2], xi.w);
+    P.V2[p] = make_double4(vn[0], vn[1], vn[2], rhoi);
+    P.P2[p] = pi;
+    P.I2[p] = P.I[p];
+    P.L2[p] = (uint8_t)lam_new;
+    double U = sqrt(vn[0] * vn[0] + vn[1] * vn[1] + vn[2] * vn[2]);
+    // with velocity smoothing the CFL minimum is taken on the smoothed
+    // velocities (k_velocity_smoothing_apply), which also moves X2
+    if (!(s.teta_v > 1.0e-9)) dtc = s.cfl * 2.0 * s.h / (s.celerita + U);
+  } else {
+    P.ACC[p] = make_double4(acc[0], acc[1], acc[2], 0.0);
+    P.L[p] = (uint8_t)lam_new;
+  }
+}
+
 // C1: with input_any_t%C1_BE the pressure terms are renormalised with
 // B_ren_gradp (3D only).
 // BATCH (not with C1): two list entries' records are requested before the
@@ -2009,7 +2129,6 @@ __global__ void __launch_bounds__(kBlock, 2) k_momentum(DevBatch b) {
   __shared__ double stpres[3][kBlock];   // the wall pressure term, kept out of the pair loop's registers
   int cur = -1;
   const Particles& P = b.P;
-  const double GI = (double)9.80665f;   // Static_allocation_module.f90:72, a default-REAL literal
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
@@ -2062,57 +2181,32 @@ __global__ void __launch_bounds__(kBlock, 2) k_momentum(DevBatch b) {
     double td0 = tdiss[0], td1 = tdiss[1], td2 = tdiss[2];
     double tv0 = tvisc[0], tv1 = tvisc[1], tv2 = tvisc[2];
     double rs0 = 0, rs1 = 0, rs2 = 0;
-    const double celt = s.celerita + s.celerita;
-    const double rcp_rhoi = __drcp_rn(rhoi);
-    const bool morris = s.kin_visc > 1.0e-12;
-    const double nu = s.kin_visc;
+    PairSelf self;
+    self.load(s, xi, make_double4(vi[0], vi[1], vi[2], 0.0), rhoi, pi);
     ListPrefetcher lr;
     lr.init(b.nlist, p, b.list_cap4, cnt);
     const int nmax = __reduce_max_sync(0xffffffffu, (unsigned)cnt);
     prefetch_list_l2(b.nlist, p, b.list_cap4, nmax);
     auto pair = [&](const double4& xj, const double4& vj, const double2& rpj) {
-      double r0 = xi.x - xj.x, r1 = xi.y - xj.y, r2 = xi.z - xj.z;
-      double rr = r0 * r0 + r1 * r1 + r2 * r2;
-      double PK1, PK2, PK3;
-      kernel_values(s, rr, PK1, PK2, PK3);
-      double rhoj = rpj.x, pj = rpj.y, amassj = xj.w;
-      double dv0 = vj.x - vi[0], dv1 = vj.y - vi[1], dv2 = vj.z - vi[2];
-      // pressure gradient and ALE1 terms, inter_EqMoto.f90:195-221
-      // the two divisions by rho_i rho_j and the one by rho_i share correctly
-      // rounded reciprocals (div_rn: the IEEE quotients, bit for bit)
-      const double rr_ij = rhoi * rhoj, rcp_rr = __drcp_rn(rr_ij);
-      double alpha = div_rn_unsigned0(pj - pi, rr_ij, rcp_rr);
-      tp0 = tp0 + -(amassj * alpha * r0 * PK3);
-      if (DIM == 3) tp1 = tp1 + -(amassj * alpha * r1 * PK3);
-      tp2 = tp2 + -(amassj * alpha * r2 * PK3);
-      double alpha2 = div_rn_unsigned0(pi * (div_rn_unsigned0(rhoj, rhoi, rcp_rhoi) + 1.0) + pj * (rhoi / rhoj - 1.0), rr_ij, rcp_rr);
-      al0 = al0 - amassj * alpha2 * r0 * PK3;
-      if (DIM == 3) al1 = al1 - amassj * alpha2 * r1 * PK3;
-      al2 = al2 - amassj * alpha2 * r2 * PK3;
-      // viscomon.f90:54-73
-      double vrij = (DIM == 3) ? -(dv0 * r0) - dv1 * r1 - dv2 * r2 : -(dv0 * r0) - dv2 * r2;
-      double TermMon = s.alfa_mon * celt * s.h / (rhoi + rhoj);
-      double mtv = amassj * TermMon * vrij;
-      td0 = td0 + (mtv * r0 * PK2 + 0.0);
-      if (DIM == 3) td1 = td1 + (mtv * r1 * PK2 + 0.0);
-      td2 = td2 + (mtv * r2 * PK2 + 0.0);
-      // viscomorris.f90:60-71
-      if (morris) {
-        double rt = nu * rhoi + nu * rhoj + 1.0e-3;
-        double anuitilde = 4.0 * (nu * nu);
-        double factivis = amassj * anuitilde / rt;
-        double w0 = factivis * (-(dv0 * PK2 * rr));
-        double w2 = factivis * (-(dv2 * PK2 * rr));
-        tv0 = tv0 + w0;
-        rs0 = rs0 + w0;
-        if (DIM == 3) {
-          double w1 = factivis * (-(dv1 * PK2 * rr));
-          tv1 = tv1 + w1;
-          rs1 = rs1 + w1;
+      pair_terms<DIM>(s, self, xj, vj, rpj, [&](int kind, int d, double a) {
+        if (kind == 0) {
+          if (d == 0) tp0 = tp0 + a;
+          else if (d == 1) tp1 = tp1 + a;
+          else tp2 = tp2 + a;
+        } else if (kind == 1) {
+          if (d == 0) al0 = al0 - a;
+          else if (d == 1) al1 = al1 - a;
+          else al2 = al2 - a;
+        } else if (kind == 2) {
+          if (d == 0) td0 = td0 + a;
+          else if (d == 1) td1 = td1 + a;
+          else td2 = td2 + a;
+        } else {
+          if (d == 0) tv0 = tv0 + a, rs0 = rs0 + a;
+          else if (d == 1) tv1 = tv1 + a, rs1 = rs1 + a;
+          else tv2 = tv2 + a, rs2 = rs2 + a;
         }
-        tv2 = tv2 + w2;
-        rs2 = rs2 + w2;
-      }
+      });
     };
     if (BATCH) {
       for (int k = 0; k < nmax; k += 2) {
@@ -2155,47 +2249,131 @@ __global__ void __launch_bounds__(kBlock, 2) k_momentum(DevBatch b) {
       tpres[0] = stpres[0][threadIdx.x] + tp0 + al0;
       tpres[1] = stpres[1][threadIdx.x] + tp1 + al1;
       tpres[2] = stpres[2][threadIdx.x] + tp2 + al2;
+      const double td[3] = {td0, td1, td2}, tv[3] = {tv0, tv1, tv2}, rs[3] = {rs0, rs1, rs2};
+      momentum_close<DIM, FUSED>(s, b, dyn, p, xi, vi, rhoi, pi, tpres, td, tv, rs, dtc);
+    }
+    if (FUSED) {
+      double m = warp_min(dtc);
+      if ((threadIdx.x & 31) == 0 && m < 1.0e300)
+        atomicMin(&dyn->dtmin_bits, (unsigned long long)__double_as_longlong(m));
+    }
+  }
+}
+
+// The FP64 momentum pass with four lanes to a particle, for simulations too
+// small to fill the SMs with one (launch_momentum): lane j forms the terms of
+// entry j of each list chunk, the chunk's terms change hands through shared
+// memory, and each lane keeps three of the sums (j = 0: pressure gradient,
+// 1: ALE1, 2: Monaghan, 3: Morris) and adds the chunk's four terms to them
+// in list order, so every sum is that of the one-lane pass.  A particle's
+// chain of pairs, each a chain of FP64 divisions and a square root, is what
+// bounds the pass there: one lane took 31 us for the 20 neighbours of a
+// 5,000-particle column.
+template <int DIM, bool FUSED>
+__global__ void __launch_bounds__(kSplitThreads, 4) k_momentum_split(DevBatch b) {
+  constexpr int PARTS = kBlock / (kSplitThreads / 4);   // a tile's parts
+  __shared__ SimDev s;
+  __shared__ double terms[kSplitThreads / 4][4][13];    // [particle][entry][term]; 13: banks
+  int cur = -1;
+  const Particles& P = b.P;
+  const unsigned FULL = 0xffffffffu;
+  const int j = threadIdx.x & 3, g = threadIdx.x >> 2;
+  for (int w = blockIdx.x; w < b.ntiles * PARTS; w += gridDim.x) {
+    const Tile tl = b.tiles[w / PARTS];
+    load_sim(s, b.sims, tl.sim, cur);
+    SimDyn* dyn = b.dyn + tl.sim;
+    const int at = (w % PARTS) * (kSplitThreads / 4) + g;
+    const int p = tl.start + at;
+    bool active = at < tl.count && p < s.p_off + dyn->nag;
+    if (FUSED && active && dyn->frozen) {
+      if (j == 0) carry_record(P, p);
+      active = false;
+    }
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0), v4 = xi;
+    double rhoi = 1.0, pi = 0.0;
+    int cnt = 0;
+    double wall[3] = {0, 0, 0}, tdiss[3] = {0, 0, 0}, tvisc[3] = {0, 0, 0};
+    if (active) {
+      xi = P.X[p];
+      v4 = P.V[p];
+      const double2 rp = P.RP[p];
+      rhoi = rp.x;
+      pi = rp.y;
+      cnt = b.ncount[p];
       const int nb = P.bdt_count[p];
-      const int bstart = nb > 0 ? P.bdt_start[p] : 0;
-      // laminar_flag, inter_EqMoto.f90:269-283
-      int lam_new = 0;
-      if (s.kin_visc > 0.0) {
-        double absv_pres = sqrt(tpres[0] * tpres[0] + tpres[1] * tpres[1] + tpres[2] * tpres[2]) + GI;
-        double absv_morris = sqrt(rs0 * rs0 + rs1 * rs1 + rs2 * rs2);
-        double weight = 0.0;
-        if (absv_pres != 0.0) weight = absv_morris / absv_pres * 100.0;
-        lam_new = (weight > 5.0 || absv_pres == 0.0) ? 1 : 0;
-      }
-      double acc[3];
-      acc[0] = tpres[0] + td0 + tv0 + geff[0];
-      acc[1] = tpres[1] + td1 + tv1 + geff[1];
-      acc[2] = tpres[2] + td2 + tv2 + geff[2];
       if (nb > 0) {
-        double R[3];
-        const double xa[3] = {xi.x, xi.y, xi.z};
-        elastic_reaction<DIM>(s, b, nb, bstart, xa, vi, R);
-        for (int d = 0; d < 3; ++d) acc[d] = acc[d] + R[d];
+        const double vi[3] = {v4.x, v4.y, v4.z};
+        const int lam = P.L[p], bstart = P.bdt_start[p];
+        if (DIM == 3) me_boundary3d(s, b, nb, bstart, vi, rhoi, pi, lam, dyn->geff, wall, tdiss, tvisc);
+        else me_boundary2d(s, b, nb, bstart, vi, rhoi, pi, lam, dyn->geff, wall, tdiss, tvisc);
       }
-      if (FUSED) {
-        double dtvel = dyn->dtvel, dt = dyn->dt;
-        double vn[3], xn[3];
-        for (int d = 0; d < 3; ++d) vn[d] = vi[d] + dtvel * acc[d];
-        xn[0] = xi.x + dt * vn[0];
-        xn[1] = xi.y + dt * vn[1];
-        xn[2] = xi.z + dt * vn[2];
-        P.X2[p] = make_double4(xn[0], xn[1], xn[2], xi.w);
-        P.V2[p] = make_double4(vn[0], vn[1], vn[2], rhoi);
-        P.P2[p] = pi;
-        P.I2[p] = P.I[p];
-        P.L2[p] = (uint8_t)lam_new;
-        double U = sqrt(vn[0] * vn[0] + vn[1] * vn[1] + vn[2] * vn[2]);
-        // with velocity smoothing the CFL minimum is taken on the smoothed
-        // velocities (k_velocity_smoothing_apply), which also moves X2
-        if (!(s.teta_v > 1.0e-9)) dtc = s.cfl * 2.0 * s.h / (s.celerita + U);
-      } else {
-        P.ACC[p] = make_double4(acc[0], acc[1], acc[2], 0.0);
-        P.L[p] = (uint8_t)lam_new;
+    }
+    PairSelf self;
+    self.load(s, xi, v4, rhoi, pi);
+    // this lane's sums; those of Morris twice, from the wall term and from 0
+    double sum[3], rs[3] = {0.0, 0.0, 0.0};
+    for (int d = 0; d < 3; ++d) sum[d] = j == 2 ? tdiss[d] : (j == 3 ? tvisc[d] : 0.0);
+    const int nch = (cnt + 3) >> 2;
+    const int nmax = __reduce_max_sync(FULL, (unsigned)nch);
+    const int* list = b.nlist + 4 * list_base4(p, b.list_cap4) + j;
+    // the records of the next chunk's entry are on their way while this one
+    // is worked on, and the entry of the one after
+    int e1 = (4 + j < cnt) ? __ldg(list + 128) : 0;
+    double4 xj = xi, vj = v4;
+    double2 rpj = make_double2(rhoi, pi);
+    if (j < cnt) {
+      const int q = __ldg(list) & kSlotMask;
+      xj = load_record(P.X + q);
+      vj = load_record(P.V + q);
+      rpj = __ldg(P.RP + q);
+    }
+    for (int c = 0; c < nmax; ++c) {
+      const double4 xc = xj, vc = vj;
+      const double2 rc = rpj;
+      const int k = 4 * c + j;
+      if (k + 4 < cnt) {
+        const int q = e1 & kSlotMask;
+        xj = load_record(P.X + q);
+        vj = load_record(P.V + q);
+        rpj = __ldg(P.RP + q);
       }
+      if (k + 8 < cnt) e1 = __ldg(list + (size_t)(c + 2) * 128);
+      if (k < cnt) {
+        double* o = terms[g][j];
+        pair_terms<DIM>(s, self, xc, vc, rc,
+                        [&](int kind, int d, double a) { o[3 * kind + d] = kind == 1 ? -a : a; });
+      }
+      __syncwarp();
+      const int n = j == 3 && !self.morris ? 0 : min(cnt - 4 * c, 4);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (q >= n) break;
+        const double* o = terms[g][q] + 3 * j;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (DIM == 2 && d == 1) continue;
+          const double a = o[d];
+          sum[d] = sum[d] + a;
+          if (j == 3) rs[d] = rs[d] + a;
+        }
+      }
+      __syncwarp();
+    }
+    // all sums to the particle's first lane
+    double al[3], td[3], tv[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      al[d] = __shfl_down_sync(FULL, sum[d], 1, 4);
+      td[d] = __shfl_down_sync(FULL, sum[d], 2, 4);
+      tv[d] = __shfl_down_sync(FULL, sum[d], 3, 4);
+      rs[d] = __shfl_down_sync(FULL, rs[d], 3, 4);
+    }
+    double dtc = 1.0e300;
+    if (active && j == 0) {
+      const double vi[3] = {v4.x, v4.y, v4.z};
+      double tpres[3];
+      for (int d = 0; d < 3; ++d) tpres[d] = wall[d] + sum[d] + al[d];
+      momentum_close<DIM, FUSED>(s, b, dyn, p, xi, vi, rhoi, pi, tpres, td, tv, rs, dtc);
     }
     if (FUSED) {
       double m = warp_min(dtc);
@@ -2311,6 +2489,38 @@ __device__ __forceinline__ double continuity_boundary_c1(const SimDev& s, const 
   return 0.0 - rhoi * (gu[0] + gv[1] + gw[2]);
 }
 
+// One pair's three terms of the velocity divergence (Continuity_Equation.f90).
+template <int DIM>
+__device__ __forceinline__ void continuity_terms(const SimDev& s, const double4& xi, const double4& vi, double rhoi,
+                                                 const double4& xj, const double4& vj, double* T) {
+  double r0 = xi.x - xj.x, r1 = xi.y - xj.y, r2 = xi.z - xj.z;
+  double rr = r0 * r0 + r1 * r1 + r2 * r2;
+  double PK1, PK2, PK3;
+  kernel_values(s, rr, PK1, PK2, PK3);
+  double c = rhoi * vj.w * PK1;     // rhoi * (amassj / rhoj) * PK1
+  T[0] = c * (vj.x - vi.x) * r0;
+  if (DIM == 3) T[1] = c * (vj.y - vi.y) * r1;
+  T[2] = c * (vj.z - vi.z) * r2;
+}
+
+// drho/dt of particle p; in the fused step Leapfrog_continuity.f90:54-68 and
+// EoS_barotropic_linear.f90:49-55.
+template <bool FUSED>
+__device__ __forceinline__ void continuity_close(const SimDev& s, const DevBatch& b, const SimDyn* dyn, int p,
+                                                 double rhoi, double dden) {
+  if (FUSED) {
+    double rho = rhoi + dyn->dt * dden;
+    if (s.density_thresholds == 1) {
+      if (rho < 0.9 * s.den0) rho = 0.9 * s.den0;
+      if (rho > 1.1 * s.den0) rho = 1.1 * s.den0;
+    }
+    double pr = s.k_over_rho0 * (rho - s.den0) + s.p_ref;
+    b.P.RP[p] = make_double2(rho, pr);
+  } else {
+    b.P.DDEN[p] = dden;
+  }
+}
+
 // Continuity, FP64 form: SASPH_continuity + Continuity_Equation, optionally
 // fused with Leapfrog_continuity and the EoS.  C1 (3D): the renormalised
 // form, Continuity_Equation.f90:119-126,201-217 -- the whole velocity
@@ -2349,12 +2559,12 @@ __global__ void __launch_bounds__(kBlock, 2) k_continuity(DevBatch b) {
     const int nmax = __reduce_max_sync(0xffffffffu, (unsigned)cnt);
     prefetch_list_l2(b.nlist, p, b.list_cap4, nmax);
     auto pair = [&](const double4& xj, const double4& vj) {
-      double r0 = xi.x - xj.x, r1 = xi.y - xj.y, r2 = xi.z - xj.z;
-      double rr = r0 * r0 + r1 * r1 + r2 * r2;
-      double PK1, PK2, PK3;
-      kernel_values(s, rr, PK1, PK2, PK3);
-      double c = rhoi * vj.w * PK1;     // rhoi * (amassj / rhoj) * PK1
       if (C1) {
+        double r0 = xi.x - xj.x, r1 = xi.y - xj.y, r2 = xi.z - xj.z;
+        double rr = r0 * r0 + r1 * r1 + r2 * r2;
+        double PK1, PK2, PK3;
+        kernel_values(s, rr, PK1, PK2, PK3);
+        double c = rhoi * vj.w * PK1;     // rhoi * (amassj / rhoj) * PK1
         const double c0 = c * (vj.x - vi.x), c1 = c * (vj.y - vi.y), c2 = c * (vj.z - vi.z);
         g1[0] = g1[0] + c0 * r0;
         g1[1] = g1[1] + c0 * r1;
@@ -2366,9 +2576,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_continuity(DevBatch b) {
         g3[1] = g3[1] + c2 * r1;
         g3[2] = g3[2] + c2 * r2;
       } else {
-        a1 = a1 + c * (vj.x - vi.x) * r0;
-        if (DIM == 3) a2 = a2 + c * (vj.y - vi.y) * r1;
-        a3 = a3 + c * (vj.z - vi.z) * r2;
+        double T[3];
+        continuity_terms<DIM>(s, xi, vi, rhoi, xj, vj, T);
+        a1 = a1 + T[0];
+        if (DIM == 3) a2 = a2 + T[1];
+        a3 = a3 + T[2];
       }
     };
     if (BATCH) {
@@ -2411,18 +2623,76 @@ __global__ void __launch_bounds__(kBlock, 2) k_continuity(DevBatch b) {
       } else {
         dden = dden - (a1 + a3);
       }
-      if (FUSED) {
-        // Leapfrog_continuity.f90:54-68, EoS_barotropic_linear.f90:49-55
-        double rho = rhoi + dyn->dt * dden;
-        if (s.density_thresholds == 1) {
-          if (rho < 0.9 * s.den0) rho = 0.9 * s.den0;
-          if (rho > 1.1 * s.den0) rho = 1.1 * s.den0;
-        }
-        double pr = s.k_over_rho0 * (rho - s.den0) + s.p_ref;
-        P.RP[p] = make_double2(rho, pr);
-      } else {
-        P.DDEN[p] = dden;
+      continuity_close<FUSED>(s, b, dyn, p, rhoi, dden);
+    }
+  }
+}
+
+// The FP64 continuity pass with four lanes to a particle (k_momentum_split's
+// scheme): lane d keeps the sum of component d.
+template <int DIM, bool FUSED>
+__global__ void __launch_bounds__(kSplitThreads, 4) k_continuity_split(DevBatch b) {
+  constexpr int PARTS = kBlock / (kSplitThreads / 4);
+  __shared__ SimDev s;
+  __shared__ double terms[kSplitThreads / 4][4][3];
+  int cur = -1;
+  const Particles& P = b.P;
+  const unsigned FULL = 0xffffffffu;
+  const int j = threadIdx.x & 3, g = threadIdx.x >> 2;
+  for (int w = blockIdx.x; w < b.ntiles * PARTS; w += gridDim.x) {
+    const Tile tl = b.tiles[w / PARTS];
+    load_sim(s, b.sims, tl.sim, cur);
+    SimDyn* dyn = b.dyn + tl.sim;
+    const int at = (w % PARTS) * (kSplitThreads / 4) + g;
+    const int p = tl.start + at;
+    const bool active = at < tl.count && p < s.p_off + dyn->nag && !(FUSED && dyn->frozen);
+    double4 xi = make_double4(0.0, 0.0, 0.0, 0.0), vi = xi;
+    double rhoi = 1.0;
+    int cnt = 0;
+    if (active) {
+      xi = P.X[p];
+      vi = P.V[p];
+      rhoi = P.RP[p].x;
+      cnt = b.ncount[p];
+    }
+    double sum = 0.0;
+    const int nch = (cnt + 3) >> 2;
+    const int nmax = __reduce_max_sync(FULL, (unsigned)nch);
+    const int* list = b.nlist + 4 * list_base4(p, b.list_cap4) + j;
+    int e1 = (4 + j < cnt) ? __ldg(list + 128) : 0;
+    double4 xj = xi, vj = vi;
+    if (j < cnt) {
+      const int q = __ldg(list) & kSlotMask;
+      xj = load_record(P.X + q);
+      vj = load_record(P.V + q);
+    }
+    for (int c = 0; c < nmax; ++c) {
+      const double4 xc = xj, vc = vj;
+      const int k = 4 * c + j;
+      if (k + 4 < cnt) {
+        const int q = e1 & kSlotMask;
+        xj = load_record(P.X + q);
+        vj = load_record(P.V + q);
       }
+      if (k + 8 < cnt) e1 = __ldg(list + (size_t)(c + 2) * 128);
+      if (k < cnt) continuity_terms<DIM>(s, xi, vi, rhoi, xc, vc, terms[g][j]);
+      __syncwarp();
+      const int n = (j == 3 || (DIM == 2 && j == 1)) ? 0 : min(cnt - 4 * c, 4);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (q >= n) break;
+        sum = sum + terms[g][q][j];
+      }
+      __syncwarp();
+    }
+    const double a2 = __shfl_down_sync(FULL, sum, 1, 4), a3 = __shfl_down_sync(FULL, sum, 2, 4);
+    if (active && j == 0) {
+      const int nb = P.bdt_count[p];
+      double dden = 0.0;
+      if (nb > 0) dden = continuity_boundary<DIM>(s, b, dyn, nb, P.bdt_start[p], vi, rhoi);
+      if (DIM == 3) dden = dden - (sum + a2 + a3);
+      else dden = dden - (sum + a3);
+      continuity_close<FUSED>(s, b, dyn, p, rhoi, dden);
     }
   }
 }
@@ -4376,9 +4646,26 @@ static void c1_frontier_2d(const DevBatch& b, bool gradp_only, cudaStream_t st) 
   else k_c1_frontier_2d<false><<<blocks_for(b), kBlock, 0, st>>>(b);
 }
 
+// Four lanes to a particle in the FP64 pair passes: while one lane each
+// leaves the SMs with fewer than kSplitWarps warps.
+constexpr int kSplitWarps = 7;
+static bool split_pairs(const DevBatch& b) { return !b.c1 && b.ntiles * (kBlock / 32) < b.sms * kSplitWarps; }
+static int split_blocks(const DevBatch& b) { return b.ntiles * (kBlock / (kSplitThreads / 4)); }
+
 void launch_momentum(const DevBatch& b, bool fused, cudaStream_t st) {
   int g = blocks_for(b, kGridMomentum);
   c1_frontier_2d(b, true, st);
+  if (split_pairs(b)) {
+    const int gs = split_blocks(b);
+    if (b.dim == 3) {
+      if (fused) k_momentum_split<3, true><<<gs, kSplitThreads, 0, st>>>(b);
+      else k_momentum_split<3, false><<<gs, kSplitThreads, 0, st>>>(b);
+    } else {
+      if (fused) k_momentum_split<2, true><<<gs, kSplitThreads, 0, st>>>(b);
+      else k_momentum_split<2, false><<<gs, kSplitThreads, 0, st>>>(b);
+    }
+    return;
+  }
   if (b.dim == 3 && b.c1) {
     if (fused) k_momentum<3, true, true><<<g, kBlock, 0, st>>>(b);
     else k_momentum<3, false, true><<<g, kBlock, 0, st>>>(b);
@@ -4473,6 +4760,17 @@ void launch_refresh_f32(const DevBatch& b, cudaStream_t st) { k_refresh_f32<<<bl
 void launch_continuity(const DevBatch& b, bool fused, cudaStream_t st) {
   int g = blocks_for(b, kGridContinuity);
   c1_frontier_2d(b, false, st);
+  if (split_pairs(b)) {
+    const int gs = split_blocks(b);
+    if (b.dim == 3) {
+      if (fused) k_continuity_split<3, true><<<gs, kSplitThreads, 0, st>>>(b);
+      else k_continuity_split<3, false><<<gs, kSplitThreads, 0, st>>>(b);
+    } else {
+      if (fused) k_continuity_split<2, true><<<gs, kSplitThreads, 0, st>>>(b);
+      else k_continuity_split<2, false><<<gs, kSplitThreads, 0, st>>>(b);
+    }
+    return;
+  }
   if (b.dim == 3 && b.c1) {
     if (fused) k_continuity<3, true, true><<<g, kBlock, 0, st>>>(b);
     else k_continuity<3, false, true><<<g, kBlock, 0, st>>>(b);
