@@ -1051,6 +1051,8 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   b.grid_blocks = prop.multiProcessorCount * 8;
   b.sms = prop.multiProcessorCount;
   for (int c = 0; c < kGridClasses; ++c) b.grid[c] = 0;
+  b.fp32c = h->precision == SPH_PREC_FP32C ? 1 : 0;
+  b.smooths = (h->any_teta_v || h->any_teta_p) ? 1 : 0;
   b.c1 = h->any_c1 ? 1 : 0;
   b.c1_divu = h->any_c1_divu ? 1 : 0;
   b.mom_batch = 0;

@@ -527,9 +527,15 @@ __global__ void __launch_bounds__(kBlock) k_rank_permute(DevBatch b) {
       double pr = P.P2[src];
       P.V[fin] = make_double4(v.x, v.y, v.z, vol);
       P.RP[fin] = make_double2(v.w, pr);
-      P.VF[fin] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)vol);
-      P.RF[fin] = make_float4((float)v.w, (float)(pr / (v.w * v.w)), (float)x.w, 0.f);
-      P.RM[fin] = make_float2((float)v.w, (float)(pr / (v.w * v.w)));
+      // the FP32 records only where a pass reads them: the FP64 form has no
+      // use for them, and RF is the smoothing passes' alone (40 of the 225
+      // bytes this launch moves per particle, 16 in the FP32c form)
+      if (b.fp32c) {
+        P.VF[fin] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)vol);
+        const float prr = (float)(pr / (v.w * v.w));
+        P.RM[fin] = make_float2((float)v.w, prr);
+        if (b.smooths) P.RF[fin] = make_float4((float)v.w, prr, (float)x.w, 0.f);
+      }
     }
   }
 }
@@ -3399,10 +3405,11 @@ __global__ void __launch_bounds__(kBlock) k_continuity_f32_finish(DevBatch b) {
     SimDyn* dyn = b.dyn + tl.sim;
     int p = tl.start + threadIdx.x;
     if (!(threadIdx.x < tl.count && p < s.p_off + dyn->nag && !dyn->frozen)) continue;
-    const double4 vi = P.V[p];
     const double rhoi = P.RP[p].x;
     double dden = 0.0;
     const int nb = P.bdt_count[p];
+    double4 vi = make_double4(0.0, 0.0, 0.0, 0.0);   // read by the wall terms alone
+    if (nb > 0) vi = P.V[p];
     if (C1 && DIM == 3 && s.c1_be) {
       dden = continuity_boundary_c1(s, b, dyn, nb, nb > 0 ? P.bdt_start[p] : 0, vi, rhoi, p);
       if (s.c1_divu) {
@@ -3429,7 +3436,7 @@ __global__ void __launch_bounds__(kBlock) k_continuity_f32_finish(DevBatch b) {
       double pr = s.k_over_rho0 * (rho - s.den0) + s.p_ref;
       P.RP[p] = make_double2(rho, pr);
       const double m = P.X[p].w;
-      P.RF[p] = make_float4((float)rho, (float)(pr / (rho * rho)), (float)m, 0.f);
+      if (b.smooths) P.RF[p] = make_float4((float)rho, (float)(pr / (rho * rho)), (float)m, 0.f);
       // the next momentum pass's records: the new density, and m/rho in
       // VF.w (the pair sums of this pass, which read the old one, are done)
       P.RM[p] = make_float2((float)rho, (float)(pr / (rho * rho)));

@@ -37,6 +37,8 @@ struct DevBatch {
   int mom_batch;           // momentum pair loop: 1 = several entries' records loaded together, 2 = the same
                            // with two entries' terms on paired FP32 instructions (FP32c; autotuned)
   int con_batch;           // the same for the continuity pair loop (0, 1, 2)
+  int fp32c;               // the FP32c form: its neighbour records (VF, RM) are kept
+  int smooths;             // some simulation smooths velocities or pressures: RF is kept
   int c1;                  // some simulation renormalises (C1_BE, 3D): P.BG (and P.BD) allocated
   int c1_divu;             // some simulation renormalises its velocity gradients (C1_divu)
 };
