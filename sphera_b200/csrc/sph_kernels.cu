@@ -2880,6 +2880,185 @@ __device__ __forceinline__ void momentum_f32_close(const SimDev& s, const DevBat
   }
 }
 
+// A particle's FP32c momentum pairs: its own values and the sums of the list
+// chunk at hand.
+template <int DIM, bool C1>
+struct MomentumPairs {
+  const SimDev& s;
+  const double2* __restrict__ rp;   // (C1) densities and pressures
+  F32Const fc;
+  RunCursor<DIM> rc;
+  float4 xfi;
+  float ckf, dz, vix, viy, viz, rhof, Pi;
+  double piD;
+  bool morris;
+  float cp0, cp1, cp2, cd0, cd1, cd2, cv0, cv1, cv2, cg0, cg1, cg2;
+  __device__ __forceinline__ MomentumPairs(const SimDev& sim, const double2* r) : s(sim), rp(r) {
+    fc.load(sim);
+    xfi = make_float4(0.f, 0.f, 0.f, 0.f);
+    vix = viy = viz = Pi = ckf = 0.f;
+    rhof = 1.f;
+    piD = 0.0;
+    dz = sim.dcdf[2];
+    morris = sim.kin_visc > 1.0e-12;
+    clear();
+  }
+  __device__ __forceinline__ void load(const float4& x, const double4& v, const double2& r) {
+    xfi = x;
+    ckf = x.w;
+    vix = (float)v.x;
+    viy = (float)v.y;
+    viz = (float)v.z;
+    rhof = (float)r.x;
+    Pi = (float)(r.y / (r.x * r.x));
+    piD = r.y;
+  }
+  __device__ __forceinline__ void clear() {
+    cp0 = cp1 = cp2 = cd0 = cd1 = cd2 = cv0 = cv1 = cv2 = 0.f;
+    if (C1) cg0 = cg1 = cg2 = 0.f;
+  }
+  // a neighbour's record is 40 B: XF (offset, cell k), VF (velocity,
+  // m/rho) and RM (rho, p/rho^2); its mass is rho (m/rho)
+  __device__ __forceinline__ void pair(int e, const float4& xj, const float4& vj, const float2& rmj) {
+    const int q = e & kSlotMask;
+    float d0, d1, d2;
+    separation_f32<DIM>(s, rc, e, xj, xfi, ckf, dz, d0, d1, d2);
+    float rr = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
+    float PK1, PK2, PK3;
+    kernel_values_f32(fc, rr, PK1, PK2, PK3);
+    const float rhoj = rmj.x;
+    const float mj = rhoj * vj.w;
+    // pressure (both accumulators of inter_EqMoto together)
+    float pf = -(mj * (Pi + rmj.y) * PK3);
+    cp0 = fmaf(pf, d0, cp0);
+    if (DIM == 3) cp1 = fmaf(pf, d1, cp1);
+    cp2 = fmaf(pf, d2, cp2);
+    if (C1) {
+      const float dpf = (float)(__ldg(reinterpret_cast<const double*>(rp + q) + 1) - piD);
+      const float gf = -(mj * dpf * rcp_approx(rhof * rhoj) * PK3);
+      cg0 = fmaf(gf, d0, cg0);
+      if (DIM == 3) cg1 = fmaf(gf, d1, cg1);
+      cg2 = fmaf(gf, d2, cg2);
+    }
+    float dv0 = vj.x - vix, dv1 = vj.y - viy, dv2 = vj.z - viz;
+    // viscomon amon / rsum and viscomorris nu4 / (nu rsum + 1e-3) from one
+    // reciprocal of their denominators' product
+    const float rsum = rhof + rhoj;
+    const float bm = fmaf(fc.nu, rsum, 1.0e-3f);
+    const float iv = rcp_approx(rsum * bm);
+    float vr = -fmaf(dv2, d2, fmaf(dv1, d1, dv0 * d0));
+    float df = mj * (fc.amon * (bm * iv)) * vr * PK2;
+    cd0 = fmaf(df, d0, cd0);
+    if (DIM == 3) cd1 = fmaf(df, d1, cd1);
+    cd2 = fmaf(df, d2, cd2);
+    if (morris) {
+      float vf = -((mj * fc.nu4) * (rsum * iv) * PK2 * rr);
+      cv0 = fmaf(vf, dv0, cv0);
+      if (DIM == 3) cv1 = fmaf(vf, dv1, cv1);
+      cv2 = fmaf(vf, dv2, cv2);
+    }
+  }
+  // `pair` for entries ea, eb on paired instructions: every half rounds as
+  // the scalar instruction does (x - y as fma(y, -1, x), one rounding
+  // either way; products and sums in the scalar code's association, no
+  // contraction), the special-function values, the cubic spline's branch
+  // and the accumulations stay scalar, ea's accumulated before eb's.
+  __device__ __forceinline__ void pair2(int ea, int eb, const float4& xa, const float4& va, const float2& ra,
+                                        const float4& xb, const float4& vb, const float2& rb) {
+    const float2 m1 = make_float2(-1.f, -1.f);
+    rc.update(s, (int)((unsigned)ea >> kSlotBits));
+    const float dxa = rc.Dx, dya = rc.Dy;
+    rc.update(s, (int)((unsigned)eb >> kSlotBits));
+    const float2 Dx = make_float2(dxa, rc.Dx), Dy = make_float2(dya, rc.Dy);
+    const float2 d0 = __fadd2_rn(Dx, __ffma2_rn(make_float2(xa.x, xb.x), m1, make_float2(xfi.x, xfi.x)));
+    const float2 d1 = (DIM == 3) ? __fadd2_rn(Dy, __ffma2_rn(make_float2(xa.y, xb.y), m1, make_float2(xfi.y, xfi.y)))
+                                 : make_float2(0.f, 0.f);
+    const float2 dk = __ffma2_rn(make_float2(xa.w, xb.w), m1, make_float2(ckf, ckf));
+    const float2 d2 = __fadd2_rn(__fmul2_rn(dk, make_float2(dz, dz)),
+                                 __ffma2_rn(make_float2(xa.z, xb.z), m1, make_float2(xfi.z, xfi.z)));
+    const float2 rr = __ffma2_rn(d2, d2, __ffma2_rn(d1, d1, __fmul2_rn(d0, d0)));
+    // kernel_values_f32
+    const float2 rq = make_float2(fmaxf(rr.x, 1.0e-30f), fmaxf(rr.y, 1.0e-30f));
+    const float2 r = __fmul2_rn(rq, make_float2(rsqrt_approx(rq.x), rsqrt_approx(rq.y)));
+    const float2 q = __fmul2_rn(r, make_float2(fc.hinv, fc.hinv));
+    const float2 q2 = __fmul2_rn(rr, make_float2(fc.h2inv, fc.h2inv));
+    const float2 a = __fadd2_rn(r, make_float2(fc.eta, fc.eta));
+    const float2 bq = __fadd2_rn(rr, make_float2(fc.eta2, fc.eta2));
+    const float2 ab = __fmul2_rn(a, bq);
+    const float2 inv = make_float2(rcp_approx(ab.x), rcp_approx(ab.y));
+    const float2 denom = __fmul2_rn(bq, inv);
+    const float2 glo = __ffma2_rn(make_float2(1.5f, 1.5f), q2, __fmul2_rn(make_float2(-2.0f, -2.0f), q));
+    const float2 ghi = __ffma2_rn(make_float2(-0.5f, -0.5f), q2,
+                                  __ffma2_rn(make_float2(2.0f, 2.0f), q, make_float2(-2.0f, -2.0f)));
+    const float2 g = make_float2(q.x < 1.0f ? glo.x : ghi.x, q.y < 1.0f ? glo.y : ghi.y);
+    const float2 gw = __ffma2_rn(make_float2(12.0f, 12.0f), q,
+                                 __ffma2_rn(make_float2(-3.0f, -3.0f), q2, make_float2(-12.0f, -12.0f)));
+    const float2 PK1 = __fmul2_rn(__fmul2_rn(g, make_float2(fc.ke, fc.ke)), denom);
+    const float2 PK2 = __fmul2_rn(PK1, __fmul2_rn(a, inv));
+    const float2 PK3 = __fmul2_rn(__fmul2_rn(gw, make_float2(fc.kacl, fc.kacl)), denom);
+    const float2 mj = __fmul2_rn(make_float2(ra.x, rb.x), make_float2(va.w, vb.w));
+    // pressure: pf = -t
+    const float2 t = __fmul2_rn(__fmul2_rn(mj, __fadd2_rn(make_float2(Pi, Pi), make_float2(ra.y, rb.y))), PK3);
+    // viscosity
+    const float2 dv0 = __ffma2_rn(make_float2(vix, vix), m1, make_float2(va.x, vb.x));
+    const float2 dv1 = __ffma2_rn(make_float2(viy, viy), m1, make_float2(va.y, vb.y));
+    const float2 dv2 = __ffma2_rn(make_float2(viz, viz), m1, make_float2(va.z, vb.z));
+    const float2 rsum = __fadd2_rn(make_float2(rhof, rhof), make_float2(ra.x, rb.x));
+    const float2 bm = __ffma2_rn(make_float2(fc.nu, fc.nu), rsum, make_float2(1.0e-3f, 1.0e-3f));
+    const float2 rb2 = __fmul2_rn(rsum, bm);
+    const float2 iv = make_float2(rcp_approx(rb2.x), rcp_approx(rb2.y));
+    // vr = -u; df = -w
+    const float2 u = __ffma2_rn(dv2, d2, __ffma2_rn(dv1, d1, __fmul2_rn(dv0, d0)));
+    const float2 w = __fmul2_rn(
+        __fmul2_rn(__fmul2_rn(mj, __fmul2_rn(make_float2(fc.amon, fc.amon), __fmul2_rn(bm, iv))), u), PK2);
+    cp0 = fmaf(-t.x, d0.x, cp0);
+    if (DIM == 3) cp1 = fmaf(-t.x, d1.x, cp1);
+    cp2 = fmaf(-t.x, d2.x, cp2);
+    cd0 = fmaf(-w.x, d0.x, cd0);
+    if (DIM == 3) cd1 = fmaf(-w.x, d1.x, cd1);
+    cd2 = fmaf(-w.x, d2.x, cd2);
+    cp0 = fmaf(-t.y, d0.y, cp0);
+    if (DIM == 3) cp1 = fmaf(-t.y, d1.y, cp1);
+    cp2 = fmaf(-t.y, d2.y, cp2);
+    cd0 = fmaf(-w.y, d0.y, cd0);
+    if (DIM == 3) cd1 = fmaf(-w.y, d1.y, cd1);
+    cd2 = fmaf(-w.y, d2.y, cd2);
+    if (morris) {
+      // vf = -z
+      const float2 z = __fmul2_rn(
+          __fmul2_rn(__fmul2_rn(__fmul2_rn(mj, make_float2(fc.nu4, fc.nu4)), __fmul2_rn(rsum, iv)), PK2), rr);
+      cv0 = fmaf(-z.x, dv0.x, cv0);
+      if (DIM == 3) cv1 = fmaf(-z.x, dv1.x, cv1);
+      cv2 = fmaf(-z.x, dv2.x, cv2);
+      cv0 = fmaf(-z.y, dv0.y, cv0);
+      if (DIM == 3) cv1 = fmaf(-z.y, dv1.y, cv1);
+      cv2 = fmaf(-z.y, dv2.y, cv2);
+    }
+  }
+  // the entries of a chunk, rem of them, their records requested together
+  template <bool PAIRED>
+  __device__ __forceinline__ void chunk(const Particles& P, const int4& ch, int rem) {
+    float4 x0, v0, x1, v1, x2, v2, x3, v3;
+    float2 r0, r1, r2, r3;
+    const int q0 = ch.x & kSlotMask, q1 = ch.y & kSlotMask, q2 = ch.z & kSlotMask, q3 = ch.w & kSlotMask;
+    x0 = __ldg(P.XF + q0); v0 = __ldg(P.VF + q0); r0 = __ldg(P.RM + q0);
+    if (rem > 1) { x1 = __ldg(P.XF + q1); v1 = __ldg(P.VF + q1); r1 = __ldg(P.RM + q1); }
+    if (rem > 2) { x2 = __ldg(P.XF + q2); v2 = __ldg(P.VF + q2); r2 = __ldg(P.RM + q2); }
+    if (rem > 3) { x3 = __ldg(P.XF + q3); v3 = __ldg(P.VF + q3); r3 = __ldg(P.RM + q3); }
+    if (PAIRED) {
+      if (rem > 1) pair2(ch.x, ch.y, x0, v0, r0, x1, v1, r1);
+      else pair(ch.x, x0, v0, r0);
+      if (rem > 3) pair2(ch.z, ch.w, x2, v2, r2, x3, v3, r3);
+      else if (rem > 2) pair(ch.z, x2, v2, r2);
+    } else {
+      pair(ch.x, x0, v0, r0);
+      if (rem > 1) pair(ch.y, x1, v1, r1);
+      if (rem > 2) pair(ch.z, x2, v2, r2);
+      if (rem > 3) pair(ch.w, x3, v3, r3);
+    }
+  }
+};
+
 // Momentum, FP32c form, in two launches.  k_momentum_f32 holds only what
 // the pair loop needs -- the particle's FP32 values, the compensated sums,
 // the list chunk being read and the next one -- so that it runs at 3 blocks
@@ -2913,37 +3092,20 @@ __global__ void __launch_bounds__(kBlock, (C1 || BATCH) ? 2 : 3) k_momentum_f32(
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
-    F32Const fc;
-    fc.load(s);
     SimDyn* dyn = b.dyn + tl.sim;
     int p = tl.start + threadIdx.x;
     const bool active = threadIdx.x < tl.count && p < s.p_off + dyn->nag && !dyn->frozen;
     int cnt = 0;
-    float4 xfi = make_float4(0.f, 0.f, 0.f, 0.f);
-    float vix = 0.f, viy = 0.f, viz = 0.f, rhof = 1.f, Pi = 0.f;
-    double piD = 0.0;
+    MomentumPairs<DIM, C1> m(s, P.RP);
     if (active) {
-      double4 v4 = P.V[p];
-      double2 rp = P.RP[p];
-      xfi = P.XF[p];
-      vix = (float)v4.x;
-      viy = (float)v4.y;
-      viz = (float)v4.z;
-      rhof = (float)rp.x;
-      Pi = (float)(rp.y / (rp.x * rp.x));
-      piD = rp.y;
+      m.load(P.XF[p], P.V[p], P.RP[p]);
       cnt = b.ncount[p];
     }
-    const float ckf = xfi.w, dz = s.dcdf[2];
-    RunCursor<DIM> rc;
-    const bool morris = s.kin_visc > 1.0e-12;
     // compensated sums of 4-entry partial sums (one list chunk each)
     Kahan tp0, tp1, tp2, td0, td1, td2, tv0, tv1, tv2;
     tp0.zero(); tp1.zero(); tp2.zero(); td0.zero(); td1.zero(); td2.zero(); tv0.zero(); tv1.zero(); tv2.zero();
-    float cp0 = 0.f, cp1 = 0.f, cp2 = 0.f, cd0 = 0.f, cd1 = 0.f, cd2 = 0.f, cv0 = 0.f, cv1 = 0.f, cv2 = 0.f;
     Kahan tg0, tg1, tg2;
     tg0.zero(); tg1.zero(); tg2.zero();
-    float cg0 = 0.f, cg1 = 0.f, cg2 = 0.f;
     // one list chunk (4 entries) per iteration: entries, compensation and
     // the next chunk's load handled once per chunk
     const int nch = (cnt + 3) >> 2;
@@ -2951,166 +3113,30 @@ __global__ void __launch_bounds__(kBlock, (C1 || BATCH) ? 2 : 3) k_momentum_f32(
     prefetch_list_l2(b.nlist, p, b.list_cap4, nchmax * 4);
     const int4* lbase = reinterpret_cast<const int4*>(b.nlist) + list_base4(p, b.list_cap4);
     int4 nxt = nch > 0 ? __ldg(lbase) : make_int4(0, 0, 0, 0);
-    // a neighbour's record is 40 B: XF (offset, cell k), VF (velocity,
-    // m/rho) and RM (rho, p/rho^2); its mass is rho (m/rho)
-    auto pair = [&](int e, const float4& xj, const float4& vj, const float2& rmj) {
-      const int q = e & kSlotMask;
-      float d0, d1, d2;
-      separation_f32<DIM>(s, rc, e, xj, xfi, ckf, dz, d0, d1, d2);
-      float rr = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
-      float PK1, PK2, PK3;
-      kernel_values_f32(fc, rr, PK1, PK2, PK3);
-      const float rhoj = rmj.x;
-      const float mj = rhoj * vj.w;
-      // pressure (both accumulators of inter_EqMoto together)
-      float pf = -(mj * (Pi + rmj.y) * PK3);
-      cp0 = fmaf(pf, d0, cp0);
-      if (DIM == 3) cp1 = fmaf(pf, d1, cp1);
-      cp2 = fmaf(pf, d2, cp2);
-      if (C1) {
-        const float dpf = (float)(__ldg(reinterpret_cast<const double*>(P.RP + q) + 1) - piD);
-        const float gf = -(mj * dpf * rcp_approx(rhof * rhoj) * PK3);
-        cg0 = fmaf(gf, d0, cg0);
-        if (DIM == 3) cg1 = fmaf(gf, d1, cg1);
-        cg2 = fmaf(gf, d2, cg2);
-      }
-      float dv0 = vj.x - vix, dv1 = vj.y - viy, dv2 = vj.z - viz;
-      // viscomon amon / rsum and viscomorris nu4 / (nu rsum + 1e-3) from one
-      // reciprocal of their denominators' product
-      const float rsum = rhof + rhoj;
-      const float bm = fmaf(fc.nu, rsum, 1.0e-3f);
-      const float iv = rcp_approx(rsum * bm);
-      float vr = -fmaf(dv2, d2, fmaf(dv1, d1, dv0 * d0));
-      float df = mj * (fc.amon * (bm * iv)) * vr * PK2;
-      cd0 = fmaf(df, d0, cd0);
-      if (DIM == 3) cd1 = fmaf(df, d1, cd1);
-      cd2 = fmaf(df, d2, cd2);
-      if (morris) {
-        float vf = -((mj * fc.nu4) * (rsum * iv) * PK2 * rr);
-        cv0 = fmaf(vf, dv0, cv0);
-        if (DIM == 3) cv1 = fmaf(vf, dv1, cv1);
-        cv2 = fmaf(vf, dv2, cv2);
-      }
-    };
-    // `pair` for entries ea, eb on paired instructions: every half rounds as
-    // the scalar instruction does (x - y as fma(y, -1, x), one rounding
-    // either way; products and sums in the scalar code's association, no
-    // contraction), the special-function values, the cubic spline's branch
-    // and the accumulations stay scalar, ea's accumulated before eb's.
-    auto pair2 = [&](int ea, int eb, const float4& xa, const float4& va, const float2& ra, const float4& xb,
-                     const float4& vb, const float2& rb) {
-      const float2 m1 = make_float2(-1.f, -1.f);
-      rc.update(s, (int)((unsigned)ea >> kSlotBits));
-      const float dxa = rc.Dx, dya = rc.Dy;
-      rc.update(s, (int)((unsigned)eb >> kSlotBits));
-      const float2 Dx = make_float2(dxa, rc.Dx), Dy = make_float2(dya, rc.Dy);
-      const float2 d0 = __fadd2_rn(Dx, __ffma2_rn(make_float2(xa.x, xb.x), m1, make_float2(xfi.x, xfi.x)));
-      const float2 d1 = (DIM == 3) ? __fadd2_rn(Dy, __ffma2_rn(make_float2(xa.y, xb.y), m1, make_float2(xfi.y, xfi.y)))
-                                   : make_float2(0.f, 0.f);
-      const float2 dk = __ffma2_rn(make_float2(xa.w, xb.w), m1, make_float2(ckf, ckf));
-      const float2 d2 = __fadd2_rn(__fmul2_rn(dk, make_float2(dz, dz)),
-                                   __ffma2_rn(make_float2(xa.z, xb.z), m1, make_float2(xfi.z, xfi.z)));
-      const float2 rr = __ffma2_rn(d2, d2, __ffma2_rn(d1, d1, __fmul2_rn(d0, d0)));
-      // kernel_values_f32
-      const float2 rq = make_float2(fmaxf(rr.x, 1.0e-30f), fmaxf(rr.y, 1.0e-30f));
-      const float2 r = __fmul2_rn(rq, make_float2(rsqrt_approx(rq.x), rsqrt_approx(rq.y)));
-      const float2 q = __fmul2_rn(r, make_float2(fc.hinv, fc.hinv));
-      const float2 q2 = __fmul2_rn(rr, make_float2(fc.h2inv, fc.h2inv));
-      const float2 a = __fadd2_rn(r, make_float2(fc.eta, fc.eta));
-      const float2 bq = __fadd2_rn(rr, make_float2(fc.eta2, fc.eta2));
-      const float2 ab = __fmul2_rn(a, bq);
-      const float2 inv = make_float2(rcp_approx(ab.x), rcp_approx(ab.y));
-      const float2 denom = __fmul2_rn(bq, inv);
-      const float2 glo = __ffma2_rn(make_float2(1.5f, 1.5f), q2, __fmul2_rn(make_float2(-2.0f, -2.0f), q));
-      const float2 ghi = __ffma2_rn(make_float2(-0.5f, -0.5f), q2,
-                                    __ffma2_rn(make_float2(2.0f, 2.0f), q, make_float2(-2.0f, -2.0f)));
-      const float2 g = make_float2(q.x < 1.0f ? glo.x : ghi.x, q.y < 1.0f ? glo.y : ghi.y);
-      const float2 gw = __ffma2_rn(make_float2(12.0f, 12.0f), q,
-                                   __ffma2_rn(make_float2(-3.0f, -3.0f), q2, make_float2(-12.0f, -12.0f)));
-      const float2 PK1 = __fmul2_rn(__fmul2_rn(g, make_float2(fc.ke, fc.ke)), denom);
-      const float2 PK2 = __fmul2_rn(PK1, __fmul2_rn(a, inv));
-      const float2 PK3 = __fmul2_rn(__fmul2_rn(gw, make_float2(fc.kacl, fc.kacl)), denom);
-      const float2 mj = __fmul2_rn(make_float2(ra.x, rb.x), make_float2(va.w, vb.w));
-      // pressure: pf = -t
-      const float2 t = __fmul2_rn(__fmul2_rn(mj, __fadd2_rn(make_float2(Pi, Pi), make_float2(ra.y, rb.y))), PK3);
-      // viscosity
-      const float2 dv0 = __ffma2_rn(make_float2(vix, vix), m1, make_float2(va.x, vb.x));
-      const float2 dv1 = __ffma2_rn(make_float2(viy, viy), m1, make_float2(va.y, vb.y));
-      const float2 dv2 = __ffma2_rn(make_float2(viz, viz), m1, make_float2(va.z, vb.z));
-      const float2 rsum = __fadd2_rn(make_float2(rhof, rhof), make_float2(ra.x, rb.x));
-      const float2 bm = __ffma2_rn(make_float2(fc.nu, fc.nu), rsum, make_float2(1.0e-3f, 1.0e-3f));
-      const float2 rb2 = __fmul2_rn(rsum, bm);
-      const float2 iv = make_float2(rcp_approx(rb2.x), rcp_approx(rb2.y));
-      // vr = -u; df = -w
-      const float2 u = __ffma2_rn(dv2, d2, __ffma2_rn(dv1, d1, __fmul2_rn(dv0, d0)));
-      const float2 w = __fmul2_rn(
-          __fmul2_rn(__fmul2_rn(mj, __fmul2_rn(make_float2(fc.amon, fc.amon), __fmul2_rn(bm, iv))), u), PK2);
-      cp0 = fmaf(-t.x, d0.x, cp0);
-      if (DIM == 3) cp1 = fmaf(-t.x, d1.x, cp1);
-      cp2 = fmaf(-t.x, d2.x, cp2);
-      cd0 = fmaf(-w.x, d0.x, cd0);
-      if (DIM == 3) cd1 = fmaf(-w.x, d1.x, cd1);
-      cd2 = fmaf(-w.x, d2.x, cd2);
-      cp0 = fmaf(-t.y, d0.y, cp0);
-      if (DIM == 3) cp1 = fmaf(-t.y, d1.y, cp1);
-      cp2 = fmaf(-t.y, d2.y, cp2);
-      cd0 = fmaf(-w.y, d0.y, cd0);
-      if (DIM == 3) cd1 = fmaf(-w.y, d1.y, cd1);
-      cd2 = fmaf(-w.y, d2.y, cd2);
-      if (morris) {
-        // vf = -z
-        const float2 z = __fmul2_rn(
-            __fmul2_rn(__fmul2_rn(__fmul2_rn(mj, make_float2(fc.nu4, fc.nu4)), __fmul2_rn(rsum, iv)), PK2), rr);
-        cv0 = fmaf(-z.x, dv0.x, cv0);
-        if (DIM == 3) cv1 = fmaf(-z.x, dv1.x, cv1);
-        cv2 = fmaf(-z.x, dv2.x, cv2);
-        cv0 = fmaf(-z.y, dv0.y, cv0);
-        if (DIM == 3) cv1 = fmaf(-z.y, dv1.y, cv1);
-        cv2 = fmaf(-z.y, dv2.y, cv2);
-      }
-    };
     for (int c = 0; c < nchmax; ++c) {
       const int4 ch = nxt;
       if (c + 1 < nch) nxt = __ldg(lbase + (size_t)(c + 1) * 32);
       if (c >= nch) continue;
       const int rem = cnt - 4 * c;   // >= 1
       if (BATCH) {
-        float4 x0, v0, x1, v1, x2, v2, x3, v3;
-        float2 r0, r1, r2, r3;
-        const int q0 = ch.x & kSlotMask, q1 = ch.y & kSlotMask, q2 = ch.z & kSlotMask, q3 = ch.w & kSlotMask;
-        x0 = __ldg(P.XF + q0); v0 = __ldg(P.VF + q0); r0 = __ldg(P.RM + q0);
-        if (rem > 1) { x1 = __ldg(P.XF + q1); v1 = __ldg(P.VF + q1); r1 = __ldg(P.RM + q1); }
-        if (rem > 2) { x2 = __ldg(P.XF + q2); v2 = __ldg(P.VF + q2); r2 = __ldg(P.RM + q2); }
-        if (rem > 3) { x3 = __ldg(P.XF + q3); v3 = __ldg(P.VF + q3); r3 = __ldg(P.RM + q3); }
-        if (PAIRED) {
-          if (rem > 1) pair2(ch.x, ch.y, x0, v0, r0, x1, v1, r1);
-          else pair(ch.x, x0, v0, r0);
-          if (rem > 3) pair2(ch.z, ch.w, x2, v2, r2, x3, v3, r3);
-          else if (rem > 2) pair(ch.z, x2, v2, r2);
-        } else {
-          pair(ch.x, x0, v0, r0);
-          if (rem > 1) pair(ch.y, x1, v1, r1);
-          if (rem > 2) pair(ch.z, x2, v2, r2);
-          if (rem > 3) pair(ch.w, x3, v3, r3);
-        }
+        m.template chunk<PAIRED>(P, ch, rem);
       } else {
         auto one = [&](int e) {
           const int q = e & kSlotMask;
-          pair(e, __ldg(P.XF + q), __ldg(P.VF + q), __ldg(P.RM + q));
+          m.pair(e, __ldg(P.XF + q), __ldg(P.VF + q), __ldg(P.RM + q));
         };
         one(ch.x);
         if (rem > 1) one(ch.y);
         if (rem > 2) one(ch.z);
         if (rem > 3) one(ch.w);
       }
-      tp0.add(cp0); tp1.add(cp1); tp2.add(cp2);
-      td0.add(cd0); td1.add(cd1); td2.add(cd2);
-      tv0.add(cv0); tv1.add(cv1); tv2.add(cv2);
-      cp0 = cp1 = cp2 = cd0 = cd1 = cd2 = cv0 = cv1 = cv2 = 0.f;
+      tp0.add(m.cp0); tp1.add(m.cp1); tp2.add(m.cp2);
+      td0.add(m.cd0); td1.add(m.cd1); td2.add(m.cd2);
+      tv0.add(m.cv0); tv1.add(m.cv1); tv2.add(m.cv2);
       if (C1) {
-        tg0.add(cg0); tg1.add(cg1); tg2.add(cg2);
-        cg0 = cg1 = cg2 = 0.f;
+        tg0.add(m.cg0); tg1.add(m.cg1); tg2.add(m.cg2);
       }
+      m.clear();
     }
     bool close_here = false;
     if (!C1 && fused && active) close_here = P.bdt_count[p] == 0;
@@ -3126,9 +3152,9 @@ __global__ void __launch_bounds__(kBlock, (C1 || BATCH) ? 2 : 3) k_momentum_f32(
       momentum_f32_close<DIM, true>(s, b, dyn, p, ms, tpres, tdiss, tvisc, vi, rp.x, rp.y, 0, 0, dtc);
     }
     if (!C1 && fused) {
-      const double m = warp_min(dtc);
-      if ((threadIdx.x & 31) == 0 && m < 1.0e300)
-        atomicMin(&dyn->dtmin_bits, (unsigned long long)__double_as_longlong(m));
+      const double least = warp_min(dtc);
+      if ((threadIdx.x & 31) == 0 && least < 1.0e300)
+        atomicMin(&dyn->dtmin_bits, (unsigned long long)__double_as_longlong(least));
     }
     if (active && !close_here) {
       double* o = P.MSUM + p;
@@ -3151,9 +3177,136 @@ __global__ void __launch_bounds__(kBlock, (C1 || BATCH) ? 2 : 3) k_momentum_f32(
   }
 }
 
+// k_momentum_f32 with four lanes to a particle, for simulations too small to
+// fill the SMs with one (split_pairs): lane j of a particle sums list
+// chunks j, j + 4, ... and the chunk sums change hands through shared
+// memory; lane j < 3 keeps the compensated sums of one kind (pressure,
+// Monaghan, Morris) and adds the chunks to them in list order, so every sum
+// is that of the one-lane pass.  Lanes 8 j .. 8 j + 7 of a warp hold lane j of
+// its eight particles: neighbouring lanes read neighbouring records.
+template <int DIM>
+__global__ void __launch_bounds__(kBlock, 2) k_momentum_f32_split(DevBatch b, int fused) {
+  constexpr int PARTS = 4;                             // 64 particles a block
+  __shared__ SimDev s;
+  __shared__ float sums[kBlock / 32][8][4][9 + 1];     // [warp][particle][chunk][sum]
+  int cur = -1;
+  const Particles& P = b.P;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane >> 3, g = lane & 7;
+  for (int w = blockIdx.x; w < b.ntiles * PARTS; w += gridDim.x) {
+    const Tile tl = b.tiles[w / PARTS];
+    load_sim(s, b.sims, tl.sim, cur);
+    SimDyn* dyn = b.dyn + tl.sim;
+    const int at = (w % PARTS) * (kBlock / 4) + warp * 8 + g;
+    const int p = tl.start + at;
+    const bool active = at < tl.count && p < s.p_off + dyn->nag && !dyn->frozen;
+    int cnt = 0;
+    MomentumPairs<DIM, false> m(s, P.RP);
+    if (active) {
+      m.load(P.XF[p], P.V[p], P.RP[p]);
+      cnt = b.ncount[p];
+    }
+    Kahan k0, k1, k2;
+    k0.zero();
+    k1.zero();
+    k2.zero();
+    const int nch = (cnt + 3) >> 2;
+    const int rounds = (int)(__reduce_max_sync(FULL, (unsigned)nch) + 3) >> 2;
+    const int4* lbase = reinterpret_cast<const int4*>(b.nlist) + list_base4(p, b.list_cap4);
+    int4 nxt = j < nch ? __ldg(lbase + (size_t)j * 32) : make_int4(0, 0, 0, 0);
+    for (int r = 0; r < rounds; ++r) {
+      const int c = 4 * r + j;
+      const int4 ch = nxt;
+      if (c + 4 < nch) nxt = __ldg(lbase + (size_t)(c + 4) * 32);
+      if (c < nch) {
+        m.template chunk<true>(P, ch, cnt - 4 * c);
+        float* o = sums[warp][g][j];
+        o[0] = m.cp0; o[1] = m.cp1; o[2] = m.cp2;
+        o[3] = m.cd0; o[4] = m.cd1; o[5] = m.cd2;
+        o[6] = m.cv0; o[7] = m.cv1; o[8] = m.cv2;
+        m.clear();
+      }
+      __syncwarp();
+      const int n = j < 3 ? min(nch - 4 * r, 4) : 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (q >= n) break;
+        const float* o = sums[warp][g][q] + 3 * j;
+        k0.add(o[0]);
+        k1.add(o[1]);
+        k2.add(o[2]);
+      }
+      __syncwarp();
+    }
+    double ms[9] = {k0.val(), k1.val(), k2.val()};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      ms[3 + d] = __shfl_down_sync(FULL, ms[d], 8);
+      ms[6 + d] = __shfl_down_sync(FULL, ms[d], 16);
+    }
+    const bool close_here = fused && active && j == 0 && P.bdt_count[p] == 0;
+    double dtc = 1.0e300;
+    if (close_here) {
+      double tpres[3] = {0, 0, 0};
+      const double zero[3] = {0, 0, 0};
+      const double4 v4 = P.V[p];
+      const double2 rp = P.RP[p];
+      const double vi[3] = {v4.x, v4.y, v4.z};
+      momentum_f32_close<DIM, true>(s, b, dyn, p, ms, tpres, zero, zero, vi, rp.x, rp.y, 0, 0, dtc);
+    }
+    if (fused) {
+      const double least = warp_min(dtc);
+      if (lane == 0 && least < 1.0e300)
+        atomicMin(&dyn->dtmin_bits, (unsigned long long)__double_as_longlong(least));
+    }
+    if (active && j == 0 && !close_here)
+      for (int k = 0; k < 9; ++k) P.MSUM[(size_t)k * P.total_slots + p] = ms[k];
+  }
+}
+
+// The finishing of particle p: its wall terms and closing.
 // C1: as the FP64 form (k_momentum<3, F, true>): the first step completes
 // and inverts B_ren_gradp in the wall pass; the renormalised pressure-
 // gradient accumulator joins the ALE1 accumulator and the wall terms.
+template <int DIM, bool FUSED, bool C1>
+__device__ __forceinline__ void momentum_f32_finish(const SimDev& s, const DevBatch& b, SimDyn* dyn, int p,
+                                                    double& dtc) {
+  const Particles& P = b.P;
+  double ms[9];
+  for (int c = 0; c < 9; ++c) ms[c] = P.MSUM[(size_t)c * P.total_slots + p];
+  double4 v4 = P.V[p];
+  double2 rp = P.RP[p];
+  const double vi[3] = {v4.x, v4.y, v4.z};
+  const double rhoi = rp.x, pi = rp.y;
+  const int nb = P.bdt_count[p];
+  const int bstart = nb > 0 ? P.bdt_start[p] : 0;
+  double tpres[3] = {0, 0, 0}, tdiss[3] = {0, 0, 0}, tvisc[3] = {0, 0, 0};
+  const double* geff = dyn->geff;
+  const bool c1 = C1 && DIM == 3 && s.c1_be;
+  if (c1) {
+    double B[9];
+    const bool first = dyn->step == 0;
+    load_b(P.BG, P.total_slots, p, B);
+    if (nb > 0)
+      me_boundary3d<true>(s, b, nb, bstart, vi, rhoi, pi, P.L[p], geff, tpres, tdiss, tvisc, B, first);
+    else if (first)
+      b_inversion(B, s.invb_det_thresh);
+    if (first) store_b(P.BG, P.total_slots, p, B);
+    // inter_EqMoto.f90:255-260: the pressure-gradient sum renormalised,
+    // the ALE1 sum (the symmetric sum less it) as it is
+    double g[3];
+    for (int d = 0; d < 3; ++d) g[d] = P.MSUM[(size_t)(9 + d) * P.total_slots + p];
+    const double al[3] = {ms[0] - g[0], ms[1] - g[1], ms[2] - g[2]};
+    b_renormalise(B, g);
+    for (int d = 0; d < 3; ++d) ms[d] = g[d] + al[d];
+  } else if (nb > 0) {
+    const int lam = P.L[p];
+    if (DIM == 3) me_boundary3d(s, b, nb, bstart, vi, rhoi, pi, lam, geff, tpres, tdiss, tvisc);
+    else me_boundary2d(s, b, nb, bstart, vi, rhoi, pi, lam, geff, tpres, tdiss, tvisc);
+  }
+  momentum_f32_close<DIM, FUSED>(s, b, dyn, p, ms, tpres, tdiss, tvisc, vi, rhoi, pi, nb, bstart, dtc);
+}
+
 template <int DIM, bool FUSED, bool C1 = false>
 __global__ void __launch_bounds__(kBlock) k_momentum_f32_finish(DevBatch b) {
   __shared__ SimDev s;
@@ -3173,41 +3326,7 @@ __global__ void __launch_bounds__(kBlock) k_momentum_f32_finish(DevBatch b) {
     // in the fused step the pair launch has closed the particles without
     // close faces already (k_momentum_f32)
     if (FUSED && !C1 && active && P.bdt_count[p] == 0) active = false;
-    if (active) {
-      double ms[9];
-      for (int c = 0; c < 9; ++c) ms[c] = P.MSUM[(size_t)c * P.total_slots + p];
-      double4 v4 = P.V[p];
-      double2 rp = P.RP[p];
-      const double vi[3] = {v4.x, v4.y, v4.z};
-      const double rhoi = rp.x, pi = rp.y;
-      const int nb = P.bdt_count[p];
-      const int bstart = nb > 0 ? P.bdt_start[p] : 0;
-      double tpres[3] = {0, 0, 0}, tdiss[3] = {0, 0, 0}, tvisc[3] = {0, 0, 0};
-      const double* geff = dyn->geff;
-      const bool c1 = C1 && DIM == 3 && s.c1_be;
-      if (c1) {
-        double B[9];
-        const bool first = dyn->step == 0;
-        load_b(P.BG, P.total_slots, p, B);
-        if (nb > 0)
-          me_boundary3d<true>(s, b, nb, bstart, vi, rhoi, pi, P.L[p], geff, tpres, tdiss, tvisc, B, first);
-        else if (first)
-          b_inversion(B, s.invb_det_thresh);
-        if (first) store_b(P.BG, P.total_slots, p, B);
-        // inter_EqMoto.f90:255-260: the pressure-gradient sum renormalised,
-        // the ALE1 sum (the symmetric sum less it) as it is
-        double g[3];
-        for (int d = 0; d < 3; ++d) g[d] = P.MSUM[(size_t)(9 + d) * P.total_slots + p];
-        const double al[3] = {ms[0] - g[0], ms[1] - g[1], ms[2] - g[2]};
-        b_renormalise(B, g);
-        for (int d = 0; d < 3; ++d) ms[d] = g[d] + al[d];
-      } else if (nb > 0) {
-        const int lam = P.L[p];
-        if (DIM == 3) me_boundary3d(s, b, nb, bstart, vi, rhoi, pi, lam, geff, tpres, tdiss, tvisc);
-        else me_boundary2d(s, b, nb, bstart, vi, rhoi, pi, lam, geff, tpres, tdiss, tvisc);
-      }
-      momentum_f32_close<DIM, FUSED>(s, b, dyn, p, ms, tpres, tdiss, tvisc, vi, rhoi, pi, nb, bstart, dtc);
-    }
+    if (active) momentum_f32_finish<DIM, FUSED, C1>(s, b, dyn, p, dtc);
     if (FUSED) {
       double m = warp_min(dtc);
       if ((threadIdx.x & 31) == 0 && m < 1.0e300)
@@ -3215,6 +3334,99 @@ __global__ void __launch_bounds__(kBlock) k_momentum_f32_finish(DevBatch b) {
     }
   }
 }
+
+// A particle's FP32c continuity pairs: its own values and the sum of the
+// list chunk at hand.
+template <int DIM>
+struct ContinuityPairs {
+  const SimDev& s;
+  F32Const fc;
+  RunCursor<DIM> rc;
+  float4 xfi;
+  float ckf, dz, vix, viy, viz, rhof, part;
+  __device__ __forceinline__ ContinuityPairs(const SimDev& sim) : s(sim) {
+    fc.load(sim);
+    xfi = make_float4(0.f, 0.f, 0.f, 0.f);
+    vix = viy = viz = ckf = part = 0.f;
+    rhof = 1.f;
+    dz = sim.dcdf[2];
+  }
+  __device__ __forceinline__ void load(const float4& x, const double4& v, double rho) {
+    xfi = x;
+    ckf = x.w;
+    vix = (float)v.x;
+    viy = (float)v.y;
+    viz = (float)v.z;
+    rhof = (float)rho;
+  }
+  __device__ __forceinline__ void pair(int e, const float4& xj, const float4& vj) {
+    float d0, d1, d2;
+    separation_f32<DIM>(s, rc, e, xj, xfi, ckf, dz, d0, d1, d2);
+    float rr = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
+    const float PK1 = kernel_pk1_f32(fc, rr);
+    float c = rhof * vj.w * PK1;
+    part = fmaf(c, fmaf(vj.z - viz, d2, fmaf(vj.y - viy, d1, (vj.x - vix) * d0)), part);
+  }
+  // pair for entries ea, eb on paired instructions (each half rounds
+  // as the scalar instruction; x - y as fma(y, -1, x)), ea's term
+  // accumulated before eb's
+  __device__ __forceinline__ void pair2(int ea, int eb, const float4& xa, const float4& va, const float4& xb,
+                                        const float4& vb) {
+    const float2 m1 = make_float2(-1.f, -1.f);
+    rc.update(s, (int)((unsigned)ea >> kSlotBits));
+    const float dxa = rc.Dx, dya = rc.Dy;
+    rc.update(s, (int)((unsigned)eb >> kSlotBits));
+    const float2 Dx = make_float2(dxa, rc.Dx), Dy = make_float2(dya, rc.Dy);
+    const float2 d0 = __fadd2_rn(Dx, __ffma2_rn(make_float2(xa.x, xb.x), m1, make_float2(xfi.x, xfi.x)));
+    const float2 d1 = (DIM == 3)
+                          ? __fadd2_rn(Dy, __ffma2_rn(make_float2(xa.y, xb.y), m1, make_float2(xfi.y, xfi.y)))
+                          : make_float2(0.f, 0.f);
+    const float2 dk = __ffma2_rn(make_float2(xa.w, xb.w), m1, make_float2(ckf, ckf));
+    const float2 d2 = __fadd2_rn(__fmul2_rn(dk, make_float2(dz, dz)),
+                                 __ffma2_rn(make_float2(xa.z, xb.z), m1, make_float2(xfi.z, xfi.z)));
+    const float2 rr = __ffma2_rn(d2, d2, __ffma2_rn(d1, d1, __fmul2_rn(d0, d0)));
+    // kernel_pk1_f32
+    const float2 rq = make_float2(fmaxf(rr.x, 1.0e-30f), fmaxf(rr.y, 1.0e-30f));
+    const float2 r = __fmul2_rn(rq, make_float2(rsqrt_approx(rq.x), rsqrt_approx(rq.y)));
+    const float2 q = __fmul2_rn(r, make_float2(fc.hinv, fc.hinv));
+    const float2 q2 = __fmul2_rn(rr, make_float2(fc.h2inv, fc.h2inv));
+    const float2 glo = __ffma2_rn(make_float2(1.5f, 1.5f), q2, __fmul2_rn(make_float2(-2.0f, -2.0f), q));
+    const float2 ghi = __ffma2_rn(make_float2(-0.5f, -0.5f), q2,
+                                  __ffma2_rn(make_float2(2.0f, 2.0f), q, make_float2(-2.0f, -2.0f)));
+    const float2 g = make_float2(q.x < 1.0f ? glo.x : ghi.x, q.y < 1.0f ? glo.y : ghi.y);
+    const float2 ra = __fadd2_rn(r, make_float2(fc.eta, fc.eta));
+    const float2 PK1 = __fmul2_rn(__fmul2_rn(g, make_float2(fc.ke, fc.ke)),
+                                  make_float2(rcp_approx(ra.x), rcp_approx(ra.y)));
+    const float2 c = __fmul2_rn(__fmul2_rn(make_float2(rhof, rhof), make_float2(va.w, vb.w)), PK1);
+    const float2 dv0 = __ffma2_rn(make_float2(vix, vix), m1, make_float2(va.x, vb.x));
+    const float2 dv1 = __ffma2_rn(make_float2(viy, viy), m1, make_float2(va.y, vb.y));
+    const float2 dv2 = __ffma2_rn(make_float2(viz, viz), m1, make_float2(va.z, vb.z));
+    const float2 u = __ffma2_rn(dv2, d2, __ffma2_rn(dv1, d1, __fmul2_rn(dv0, d0)));
+    part = fmaf(c.x, u.x, part);
+    part = fmaf(c.y, u.y, part);
+  }
+  // the entries of a chunk, rem of them, their records requested together
+  template <bool PAIRED>
+  __device__ __forceinline__ void chunk(const Particles& P, const int4& ch, int rem) {
+    const int q0 = ch.x & kSlotMask, q1 = ch.y & kSlotMask, q2 = ch.z & kSlotMask, q3 = ch.w & kSlotMask;
+    float4 x0, v0, x1, v1, x2, v2, x3, v3;
+    x0 = __ldg(P.XF + q0); v0 = __ldg(P.VF + q0);
+    if (rem > 1) { x1 = __ldg(P.XF + q1); v1 = __ldg(P.VF + q1); }
+    if (rem > 2) { x2 = __ldg(P.XF + q2); v2 = __ldg(P.VF + q2); }
+    if (rem > 3) { x3 = __ldg(P.XF + q3); v3 = __ldg(P.VF + q3); }
+    if (PAIRED) {
+      if (rem > 1) pair2(ch.x, ch.y, x0, v0, x1, v1);
+      else pair(ch.x, x0, v0);
+      if (rem > 3) pair2(ch.z, ch.w, x2, v2, x3, v3);
+      else if (rem > 2) pair(ch.z, x2, v2);
+    } else {
+      pair(ch.x, x0, v0);
+      if (rem > 1) pair(ch.y, x1, v1);
+      if (rem > 2) pair(ch.z, x2, v2);
+      if (rem > 3) pair(ch.w, x3, v3);
+    }
+  }
+};
 
 // Continuity, FP32c form, in two launches so that the pair sum need not
 // wait for the boundary data: k_continuity_f32 writes the compensated pair
@@ -3239,29 +3451,18 @@ __global__ void __launch_bounds__(kBlock, DIVU ? 2 : (BATCH ? 3 : 5)) k_continui
   for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
     Tile tl = b.tiles[t];
     load_sim(s, b.sims, tl.sim, cur);
-    F32Const fc;
-    fc.load(s);
     SimDyn* dyn = b.dyn + tl.sim;
     int p = tl.start + threadIdx.x;
     bool active = threadIdx.x < tl.count && p < s.p_off + dyn->nag && !dyn->frozen;
     int cnt = 0;
-    float4 xfi = make_float4(0.f, 0.f, 0.f, 0.f);
-    float vix = 0.f, viy = 0.f, viz = 0.f, rhof = 1.f;
+    ContinuityPairs<DIM> m(s);
     if (active) {
-      double4 vi = P.V[p];
-      xfi = P.XF[p];
-      vix = (float)vi.x;
-      viy = (float)vi.y;
-      viz = (float)vi.z;
-      rhof = (float)P.RP[p].x;
+      m.load(P.XF[p], P.V[p], P.RP[p].x);
       cnt = b.ncount[p];
     }
-    const float ckf = xfi.w, dz = s.dcdf[2];
-    RunCursor<DIM> rc;
     const bool tensor = DIVU && DIM == 3 && s.c1_be && s.c1_divu;
     Kahan sum;
     sum.zero();
-    float part = 0.f;   // 4-entry partial sum, compensated into sum per chunk
     Kahan gs[9];
     float gp[9];
 #pragma unroll
@@ -3272,51 +3473,6 @@ __global__ void __launch_bounds__(kBlock, DIVU ? 2 : (BATCH ? 3 : 5)) k_continui
     const int nmax = __reduce_max_sync(0xffffffffu, (unsigned)cnt);
     prefetch_list_l2(b.nlist, p, b.list_cap4, nmax);
     if (BATCH && !DIVU) {
-      auto contrib = [&](int e, const float4& xj, const float4& vj) {
-        float d0, d1, d2;
-        separation_f32<DIM>(s, rc, e, xj, xfi, ckf, dz, d0, d1, d2);
-        float rr = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
-        const float PK1 = kernel_pk1_f32(fc, rr);
-        float c = rhof * vj.w * PK1;
-        part = fmaf(c, fmaf(vj.z - viz, d2, fmaf(vj.y - viy, d1, (vj.x - vix) * d0)), part);
-      };
-      // contrib for entries ea, eb on paired instructions (each half rounds
-      // as the scalar instruction; x - y as fma(y, -1, x)), ea's term
-      // accumulated before eb's
-      auto contrib2 = [&](int ea, int eb, const float4& xa, const float4& va, const float4& xb, const float4& vb) {
-        const float2 m1 = make_float2(-1.f, -1.f);
-        rc.update(s, (int)((unsigned)ea >> kSlotBits));
-        const float dxa = rc.Dx, dya = rc.Dy;
-        rc.update(s, (int)((unsigned)eb >> kSlotBits));
-        const float2 Dx = make_float2(dxa, rc.Dx), Dy = make_float2(dya, rc.Dy);
-        const float2 d0 = __fadd2_rn(Dx, __ffma2_rn(make_float2(xa.x, xb.x), m1, make_float2(xfi.x, xfi.x)));
-        const float2 d1 = (DIM == 3)
-                              ? __fadd2_rn(Dy, __ffma2_rn(make_float2(xa.y, xb.y), m1, make_float2(xfi.y, xfi.y)))
-                              : make_float2(0.f, 0.f);
-        const float2 dk = __ffma2_rn(make_float2(xa.w, xb.w), m1, make_float2(ckf, ckf));
-        const float2 d2 = __fadd2_rn(__fmul2_rn(dk, make_float2(dz, dz)),
-                                     __ffma2_rn(make_float2(xa.z, xb.z), m1, make_float2(xfi.z, xfi.z)));
-        const float2 rr = __ffma2_rn(d2, d2, __ffma2_rn(d1, d1, __fmul2_rn(d0, d0)));
-        // kernel_pk1_f32
-        const float2 rq = make_float2(fmaxf(rr.x, 1.0e-30f), fmaxf(rr.y, 1.0e-30f));
-        const float2 r = __fmul2_rn(rq, make_float2(rsqrt_approx(rq.x), rsqrt_approx(rq.y)));
-        const float2 q = __fmul2_rn(r, make_float2(fc.hinv, fc.hinv));
-        const float2 q2 = __fmul2_rn(rr, make_float2(fc.h2inv, fc.h2inv));
-        const float2 glo = __ffma2_rn(make_float2(1.5f, 1.5f), q2, __fmul2_rn(make_float2(-2.0f, -2.0f), q));
-        const float2 ghi = __ffma2_rn(make_float2(-0.5f, -0.5f), q2,
-                                      __ffma2_rn(make_float2(2.0f, 2.0f), q, make_float2(-2.0f, -2.0f)));
-        const float2 g = make_float2(q.x < 1.0f ? glo.x : ghi.x, q.y < 1.0f ? glo.y : ghi.y);
-        const float2 ra = __fadd2_rn(r, make_float2(fc.eta, fc.eta));
-        const float2 PK1 = __fmul2_rn(__fmul2_rn(g, make_float2(fc.ke, fc.ke)),
-                                      make_float2(rcp_approx(ra.x), rcp_approx(ra.y)));
-        const float2 c = __fmul2_rn(__fmul2_rn(make_float2(rhof, rhof), make_float2(va.w, vb.w)), PK1);
-        const float2 dv0 = __ffma2_rn(make_float2(vix, vix), m1, make_float2(va.x, vb.x));
-        const float2 dv1 = __ffma2_rn(make_float2(viy, viy), m1, make_float2(va.y, vb.y));
-        const float2 dv2 = __ffma2_rn(make_float2(viz, viz), m1, make_float2(va.z, vb.z));
-        const float2 u = __ffma2_rn(dv2, d2, __ffma2_rn(dv1, d1, __fmul2_rn(dv0, d0)));
-        part = fmaf(c.x, u.x, part);
-        part = fmaf(c.y, u.y, part);
-      };
       const int nch = (cnt + 3) >> 2, nchmax = (nmax + 3) >> 2;
       const int4* lbase = reinterpret_cast<const int4*>(b.nlist) + list_base4(p, b.list_cap4);
       int4 nxt = nch > 0 ? __ldg(lbase) : make_int4(0, 0, 0, 0);
@@ -3325,25 +3481,9 @@ __global__ void __launch_bounds__(kBlock, DIVU ? 2 : (BATCH ? 3 : 5)) k_continui
         if (c + 1 < nch) nxt = __ldg(lbase + (size_t)(c + 1) * 32);
         if (c >= nch) continue;
         const int rem = cnt - 4 * c;
-        const int q0 = ch.x & kSlotMask, q1 = ch.y & kSlotMask, q2 = ch.z & kSlotMask, q3 = ch.w & kSlotMask;
-        float4 x0, v0, x1, v1, x2, v2, x3, v3;
-        x0 = __ldg(P.XF + q0); v0 = __ldg(P.VF + q0);
-        if (rem > 1) { x1 = __ldg(P.XF + q1); v1 = __ldg(P.VF + q1); }
-        if (rem > 2) { x2 = __ldg(P.XF + q2); v2 = __ldg(P.VF + q2); }
-        if (rem > 3) { x3 = __ldg(P.XF + q3); v3 = __ldg(P.VF + q3); }
-        if (PAIRED) {
-          if (rem > 1) contrib2(ch.x, ch.y, x0, v0, x1, v1);
-          else contrib(ch.x, x0, v0);
-          if (rem > 3) contrib2(ch.z, ch.w, x2, v2, x3, v3);
-          else if (rem > 2) contrib(ch.z, x2, v2);
-        } else {
-          contrib(ch.x, x0, v0);
-          if (rem > 1) contrib(ch.y, x1, v1);
-          if (rem > 2) contrib(ch.z, x2, v2);
-          if (rem > 3) contrib(ch.w, x3, v3);
-        }
-        sum.add(part);
-        part = 0.f;
+        m.template chunk<PAIRED>(P, ch, rem);
+        sum.add(m.part);   // 4-entry partial sums, compensated into sum
+        m.part = 0.f;
       }
     }
     ListPrefetcher lr;
@@ -3353,13 +3493,13 @@ __global__ void __launch_bounds__(kBlock, DIVU ? 2 : (BATCH ? 3 : 5)) k_continui
       if (k >= cnt) continue;
       const float4 xj = __ldg(P.XF + (e & kSlotMask)), vj = __ldg(P.VF + (e & kSlotMask));
       float d0, d1, d2;
-      separation_f32<DIM>(s, rc, e, xj, xfi, ckf, dz, d0, d1, d2);
+      separation_f32<DIM>(s, m.rc, e, xj, m.xfi, m.ckf, m.dz, d0, d1, d2);
       float rr = fmaf(d2, d2, fmaf(d1, d1, d0 * d0));
-      const float PK1 = kernel_pk1_f32(fc, rr);
-      float c = rhof * vj.w * PK1;    // rho_i (m_j / rho_j) PK1
+      const float PK1 = kernel_pk1_f32(m.fc, rr);
+      float c = m.rhof * vj.w * PK1;    // rho_i (m_j / rho_j) PK1
       const bool flush = (k & 3) == 3 || k == cnt - 1;
       if (DIVU && tensor) {
-        const float cv[3] = {c * (vj.x - vix), c * (vj.y - viy), c * (vj.z - viz)};
+        const float cv[3] = {c * (vj.x - m.vix), c * (vj.y - m.viy), c * (vj.z - m.viz)};
         const float dd[3] = {d0, d1, d2};
 #pragma unroll
         for (int a = 0; a < 3; ++a)
@@ -3373,10 +3513,10 @@ __global__ void __launch_bounds__(kBlock, DIVU ? 2 : (BATCH ? 3 : 5)) k_continui
           }
         }
       } else {
-        part = fmaf(c, fmaf(vj.z - viz, d2, fmaf(vj.y - viy, d1, (vj.x - vix) * d0)), part);
+        m.part = fmaf(c, fmaf(vj.z - m.viz, d2, fmaf(vj.y - m.viy, d1, (vj.x - m.vix) * d0)), m.part);
         if (flush) {
-          sum.add(part);
-          part = 0.f;
+          sum.add(m.part);
+          m.part = 0.f;
         }
       }
     }
@@ -3388,6 +3528,51 @@ __global__ void __launch_bounds__(kBlock, DIVU ? 2 : (BATCH ? 3 : 5)) k_continui
         P.DDEN[p] = sum.val();
       }
     }
+  }
+}
+
+// k_continuity_f32 with four lanes to a particle (k_momentum_f32_split's
+// scheme); the chunk sums go round by shuffles.
+template <int DIM>
+__global__ void __launch_bounds__(kBlock, 3) k_continuity_f32_split(DevBatch b) {
+  constexpr int PARTS = 4;
+  __shared__ SimDev s;
+  int cur = -1;
+  const Particles& P = b.P;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane >> 3, g = lane & 7;
+  for (int w = blockIdx.x; w < b.ntiles * PARTS; w += gridDim.x) {
+    const Tile tl = b.tiles[w / PARTS];
+    load_sim(s, b.sims, tl.sim, cur);
+    const SimDyn* dyn = b.dyn + tl.sim;
+    const int at = (w % PARTS) * (kBlock / 4) + warp * 8 + g;
+    const int p = tl.start + at;
+    const bool active = at < tl.count && p < s.p_off + dyn->nag && !dyn->frozen;
+    int cnt = 0;
+    ContinuityPairs<DIM> m(s);
+    if (active) {
+      m.load(P.XF[p], P.V[p], P.RP[p].x);
+      cnt = b.ncount[p];
+    }
+    Kahan sum;
+    sum.zero();
+    const int nch = (cnt + 3) >> 2;
+    const int rounds = (int)(__reduce_max_sync(FULL, (unsigned)nch) + 3) >> 2;
+    const int4* lbase = reinterpret_cast<const int4*>(b.nlist) + list_base4(p, b.list_cap4);
+    int4 nxt = j < nch ? __ldg(lbase + (size_t)j * 32) : make_int4(0, 0, 0, 0);
+    for (int r = 0; r < rounds; ++r) {
+      const int c = 4 * r + j;
+      const int4 ch = nxt;
+      if (c + 4 < nch) nxt = __ldg(lbase + (size_t)(c + 4) * 32);
+      m.part = 0.f;
+      if (c < nch) m.template chunk<true>(P, ch, cnt - 4 * c);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float v = __shfl_sync(FULL, m.part, 8 * q + g);
+        if (4 * r + q < nch) sum.add(v);
+      }
+    }
+    if (active && j == 0) P.DDEN[p] = sum.val();
   }
 }
 
@@ -4653,16 +4838,16 @@ static void c1_frontier_2d(const DevBatch& b, bool gradp_only, cudaStream_t st) 
   else k_c1_frontier_2d<false><<<blocks_for(b), kBlock, 0, st>>>(b);
 }
 
-// Four lanes to a particle in the FP64 pair passes: while one lane each
-// leaves the SMs with fewer than kSplitWarps warps.
-constexpr int kSplitWarps = 7;
-static bool split_pairs(const DevBatch& b) { return !b.c1 && b.ntiles * (kBlock / 32) < b.sms * kSplitWarps; }
+// Four lanes to a particle in a pair pass (without C1): while one lane each
+// would leave an SM with fewer than `warps` warps.
+constexpr int kSplitFp64 = 7, kSplitMomentumF32 = 5, kSplitContinuityF32 = 8;
+static bool split_pairs(const DevBatch& b, int warps) { return !b.c1 && b.ntiles * (kBlock / 32) < b.sms * warps; }
 static int split_blocks(const DevBatch& b) { return b.ntiles * (kBlock / (kSplitThreads / 4)); }
 
 void launch_momentum(const DevBatch& b, bool fused, cudaStream_t st) {
   int g = blocks_for(b, kGridMomentum);
   c1_frontier_2d(b, true, st);
-  if (split_pairs(b)) {
+  if (split_pairs(b, kSplitFp64)) {
     const int gs = split_blocks(b);
     if (b.dim == 3) {
       if (fused) k_momentum_split<3, true><<<gs, kSplitThreads, 0, st>>>(b);
@@ -4717,13 +4902,15 @@ void launch_momentum_f32(const DevBatch& b, bool fused, cudaStream_t st) {
     if (fused) k_momentum_f32_finish<3, true, true><<<gf, kBlock, 0, st>>>(b);
     else k_momentum_f32_finish<3, false, true><<<gf, kBlock, 0, st>>>(b);
   } else if (b.dim == 3) {
-    if (b.mom_batch == 2) k_momentum_f32<3, false, true, true><<<g, kBlock, 0, st>>>(b, f);
+    if (split_pairs(b, kSplitMomentumF32)) k_momentum_f32_split<3><<<b.ntiles * 4, kBlock, 0, st>>>(b, f);
+    else if (b.mom_batch == 2) k_momentum_f32<3, false, true, true><<<g, kBlock, 0, st>>>(b, f);
     else if (b.mom_batch) k_momentum_f32<3, false, true><<<g, kBlock, 0, st>>>(b, f);
     else k_momentum_f32<3><<<g, kBlock, 0, st>>>(b, f);
     if (fused) k_momentum_f32_finish<3, true><<<gf, kBlock, 0, st>>>(b);
     else k_momentum_f32_finish<3, false><<<gf, kBlock, 0, st>>>(b);
   } else {
-    if (b.mom_batch == 2) k_momentum_f32<2, false, true, true><<<g, kBlock, 0, st>>>(b, f);
+    if (split_pairs(b, kSplitMomentumF32)) k_momentum_f32_split<2><<<b.ntiles * 4, kBlock, 0, st>>>(b, f);
+    else if (b.mom_batch == 2) k_momentum_f32<2, false, true, true><<<g, kBlock, 0, st>>>(b, f);
     else if (b.mom_batch) k_momentum_f32<2, false, true><<<g, kBlock, 0, st>>>(b, f);
     else k_momentum_f32<2><<<g, kBlock, 0, st>>>(b, f);
     if (fused) k_momentum_f32_finish<2, true><<<gf, kBlock, 0, st>>>(b);
@@ -4734,6 +4921,8 @@ void launch_momentum_f32(const DevBatch& b, bool fused, cudaStream_t st) {
 void launch_continuity_f32_pairs(const DevBatch& b, cudaStream_t st) {
   int g = blocks_for(b, kGridContinuity);
   if (b.dim == 3 && b.c1_divu) k_continuity_f32<3, true><<<g, kBlock, 0, st>>>(b);
+  else if (split_pairs(b, kSplitContinuityF32) && b.dim == 3) k_continuity_f32_split<3><<<b.ntiles * 4, kBlock, 0, st>>>(b);
+  else if (split_pairs(b, kSplitContinuityF32)) k_continuity_f32_split<2><<<b.ntiles * 4, kBlock, 0, st>>>(b);
   else if (b.dim == 3 && b.con_batch == 2) k_continuity_f32<3, false, true, true><<<g, kBlock, 0, st>>>(b);
   else if (b.dim == 3 && b.con_batch) k_continuity_f32<3, false, true><<<g, kBlock, 0, st>>>(b);
   else if (b.dim == 3) k_continuity_f32<3><<<g, kBlock, 0, st>>>(b);
@@ -4767,7 +4956,7 @@ void launch_refresh_f32(const DevBatch& b, cudaStream_t st) { k_refresh_f32<<<bl
 void launch_continuity(const DevBatch& b, bool fused, cudaStream_t st) {
   int g = blocks_for(b, kGridContinuity);
   c1_frontier_2d(b, false, st);
-  if (split_pairs(b)) {
+  if (split_pairs(b, kSplitFp64)) {
     const int gs = split_blocks(b);
     if (b.dim == 3) {
       if (fused) k_continuity_split<3, true><<<gs, kSplitThreads, 0, st>>>(b);
