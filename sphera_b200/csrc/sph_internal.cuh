@@ -30,6 +30,7 @@ constexpr int kBitRows = 256;        // BITrows = FI_STEPS * TETA_STEPS
 constexpr int kKtRows = 40;          // INT_KERNELTABLE
 constexpr int kMaxCloseSides = 4;    // MAXCLOSEBOUNDSIDES
 constexpr int kMaxLocalFaces = 16;   // per-thread close-face buffer (3D)
+constexpr int kMostSpan = 14;        // z cells between the particles that the list pass screens together
 
 // Per-simulation constants (read-only during a step).
 struct SimDev {

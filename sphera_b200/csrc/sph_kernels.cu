@@ -1546,73 +1546,31 @@ struct ListPrefetcher {
 };
 
 // r^2 <= (2h)^2 (CalcVarLength.f90:223-228) is decided on the FP32
-// screening copies outside [rr_lo, rr_hi], a band the host derives from the
-// copies' rounding bounds, and in FP64, exactly as the reference, inside it.
-// A group of lanes whose z cells span at most kRebaseSpan stages candidate z
-// values re-based on the group's lowest cell, (kj - kmin) dcd + f_j, so the
-// z difference costs one subtraction; the band covers that form's rounding
-// too.  Candidates are rejected on the FP32 value alone; the window test
-// (the candidate's z cell within one of the lane's), the NMAXPARTJ cap and
-// the acceptance run only for the few that pass.
-constexpr int kRebaseSpan = 6;
+// screening copies outside a band around (2h)^2 that the host derives from
+// the copies' rounding bounds ([rr_lo, rr_hi]), and in FP64, exactly as the
+// reference, inside it (one particle in 40 has such a candidate).  Candidates
+// are staged in the frame of the group's lowest cell, f_j + D in x and y and
+// (kj - kmin) dcd + f_j in z, so each difference costs one addition; the band
+// covers that form's rounding for groups that span up to kMostSpan cells
+// (sph_api.cu).
 
-// FP32 r^2 of the lane and staged candidate xj.  REBASE: staged z values
-// are (kj - kmin) dcdf + f_j and zi the lane's own; otherwise the raw
-// offsets f_j with the cell difference formed here.
-template <int DIM, bool REBASE>
-__device__ __forceinline__ float screen_rf(const float4& xj, float ax, float ay, float zi, float fz, int ck, float dz) {
-  float d0 = ax - xj.x;
-  float d1 = (DIM == 3) ? ay - xj.y : 0.f;
-  float d2 = REBASE ? zi - xj.z : (((float)ck - xj.w) * dz + fz) - xj.z;
-  return __fmaf_rn(d2, d2, __fmaf_rn(d1, d1, __fmul_rn(d0, d0)));
-}
-
-// Screens the staged tile of nt candidates for one lane, branch-free: bit u
-// of hitm is set unless candidate u's FP32 r^2 exceeds rr_hi (a certain
-// rejection), bit u of lom when it is below rr_lo (a certain acceptance of
-// the distance test; the caller still masks the lane's own 3-cell window,
-// which a candidate closer than 2h can lie outside where cells are narrower
-// than 2h).  Hits are about one candidate in nine; the band cases (hit, not
-// low) are left to the caller.  Entries past nt are staged far away and
-// never hit, so the tile is screened in blocks of 8.
-template <int DIM, bool REBASE>
-__device__ __forceinline__ void screen_tile(const float4* wbuf, int nt, float ax, float ay, float zi, float fz, int ck,
-                                            float dz, float rr_lo, float rr_hi, unsigned& hitm, unsigned& lom) {
-  unsigned hm = 0u, lm = 0u;
-  for (int u0 = 0; u0 < nt; u0 += 8) {
-    unsigned h8 = 0u, l8 = 0u;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      float rf = screen_rf<DIM, REBASE>(wbuf[u0 + c], ax, ay, zi, fz, ck, dz);
-      if (!(rf > rr_hi)) h8 |= 1u << c;
-      if (rf < rr_lo) l8 |= 1u << c;
-    }
-    hm |= h8 << u0;
-    lm |= l8 << u0;
-  }
-  hitm = hm;
-  lom = lm;
-}
-
-// screen_tile<DIM, true> on Blackwell's paired FP32 instructions: the tile
-// is staged a second time as negated x, y, z arrays, and candidates u, u+1
-// share each add, multiply and fused multiply-add (__fadd2_rn, __fmul2_rn,
-// __ffma2_rn round each half as the scalar instruction does, x + (-y)
-// rounds as x - y and fma(r, -1, y) as y - r, so every r^2 and both masks
-// are bit-identical to screen_tile's).
+// Screens the staged tile of nt >= 1 candidates (negated x, y, z arrays) for
+// one lane: bit 31 - u of the result is the sign of r^2 - mid of candidate u,
+// and `near` falls to the least |r^2 - mid|, so that outside the band the
+// sign is the test.  Candidates u, u + 1 share each paired FP32 instruction
+// (__fadd2_rn, __fmul2_rn, __ffma2_rn), and one funnel shift moves a sign in.
+// Entries past nt are staged far away and never hit.
 template <int DIM>
-__device__ __forceinline__ void screen_tile_x2(const float* nx, const float* ny, const float* nz, int nt, float ax,
-                                               float ay, float zi, float rr_lo, float rr_hi, unsigned& hitm,
-                                               unsigned& lom) {
+__device__ __forceinline__ unsigned screen_tile(const float* nx, const float* ny, const float* nz, int nt, float ax,
+                                                float ay, float zi, float mid, float& near) {
   const float2 ax2 = make_float2(ax, ax), ay2 = make_float2(ay, ay), zi2 = make_float2(zi, zi);
-  const float2 hi2 = make_float2(rr_hi, rr_hi), nlo2 = make_float2(-rr_lo, -rr_lo), m1 = make_float2(-1.f, -1.f);
-  unsigned hm = 0u, lm = 0u;
+  const float2 nm2 = make_float2(-mid, -mid);
+  unsigned m = 0u;
 #pragma unroll
   for (int u0 = 0; u0 < 32; u0 += 8) {
     if (u0 >= nt) break;
-    unsigned h8 = 0u, l8 = 0u;
 #pragma unroll
-    for (int c = 4; c >= 0; c -= 4) {
+    for (int c = 0; c < 8; c += 4) {
       const float4 X = *reinterpret_cast<const float4*>(nx + u0 + c);
       const float4 Z = *reinterpret_cast<const float4*>(nz + u0 + c);
       float2 ra = __fadd2_rn(ax2, make_float2(X.x, X.y));
@@ -1628,227 +1586,478 @@ __device__ __forceinline__ void screen_tile_x2(const float* nx, const float* ny,
         ra = __ffma2_rn(ya, ya, ra);
         rb = __ffma2_rn(yb, yb, rb);
       }
-      ra = __ffma2_rn(za, za, ra);
-      rb = __ffma2_rn(zb, zb, rb);
-      // sign bits: rr_hi - r^2 < 0 exactly when r^2 > rr_hi, r^2 - rr_lo < 0
-      // exactly when r^2 < rr_lo (finite inputs; a difference of two floats
-      // is zero only when they are equal); one funnel shift per candidate
-      // and mask moves the sign in, candidate u ending in bit u
-      const float2 ha = __ffma2_rn(ra, m1, hi2), hb = __ffma2_rn(rb, m1, hi2);
-      const float2 la = __fadd2_rn(ra, nlo2), lb = __fadd2_rn(rb, nlo2);
-      h8 = __funnelshift_l(__float_as_uint(hb.y), h8, 1);
-      h8 = __funnelshift_l(__float_as_uint(hb.x), h8, 1);
-      h8 = __funnelshift_l(__float_as_uint(ha.y), h8, 1);
-      h8 = __funnelshift_l(__float_as_uint(ha.x), h8, 1);
-      l8 = __funnelshift_l(__float_as_uint(lb.y), l8, 1);
-      l8 = __funnelshift_l(__float_as_uint(lb.x), l8, 1);
-      l8 = __funnelshift_l(__float_as_uint(la.y), l8, 1);
-      l8 = __funnelshift_l(__float_as_uint(la.x), l8, 1);
+      ra = __fadd2_rn(__ffma2_rn(za, za, ra), nm2);
+      rb = __fadd2_rn(__ffma2_rn(zb, zb, rb), nm2);
+      near = fminf(near, fminf(fabsf(ra.x), fabsf(ra.y)));
+      near = fminf(near, fminf(fabsf(rb.x), fabsf(rb.y)));
+      m = __funnelshift_l(__float_as_uint(ra.x), m, 1);
+      m = __funnelshift_l(__float_as_uint(ra.y), m, 1);
+      m = __funnelshift_l(__float_as_uint(rb.x), m, 1);
+      m = __funnelshift_l(__float_as_uint(rb.y), m, 1);
     }
-    hm |= (~h8 & 0xffu) << u0;   // h8: rejected; l8: below rr_lo
-    lm |= (l8 & 0xffu) << u0;
   }
-  hitm = hm;
-  lom = lm;
+  return m << (32 - ((nt + 7) & ~7));
 }
 
-// Whether any staged candidate u0 <= u < nt lies in the lane's 3-cell z
-// window (the truncation test once NMAXPARTJ is reached; rare).
-__device__ __forceinline__ bool in_window(float kj, int ck) { return fabsf(kj - (float)ck) <= 1.0f; }
+// Run r of a cell's block: its candidates end before `end`, candidate c of
+// the block is slot base + c, (dx, dy) the run's column origin in the cell's
+// frame.
+struct ListRun {
+  int end, base;
+  float dx, dy;
+};
 
-// Bits u of a 32-candidate tile with lo <= u < hi (lo, hi relative to the
-// tile's first slot, any sign).
-__device__ __forceinline__ unsigned window_mask(int lo, int hi) {
-  lo = lo < 0 ? 0 : lo;
-  hi = hi > 32 ? 32 : hi;
-  if (hi <= lo) return 0u;
-  const unsigned upto = hi == 32 ? 0xffffffffu : (1u << hi) - 1u;
-  return upto & ~((1u << lo) - 1u);
+// The list of particle q, FP32 copy xq in cell (ci, cj, ck), by the whole
+// warp: its own 27-cell block, 32 candidates at a time, the entries ranked by
+// ballots and written one by one; the first NMAXPARTJ accepted are kept, the
+// particle itself among them (CalcVarLength.f90:197-205), and trunc tells
+// that candidates follow them.  For groups of few lanes, and for those whose
+// common window is many times a particle's own.
+template <int DIM>
+__device__ __forceinline__ void list_by_ballots(const SimDev& s, const DevBatch& b, int q, const float4& xq, int ci,
+                                                int cj, int ck, ListRun* runs, int& cnt, int& acc, int& cand,
+                                                bool& trunc) {
+  constexpr int NR = (DIM == 3) ? 9 : 3, UN = (DIM == 3) ? 4 : 2;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const Particles& P = b.P;
+  const int cap = s.nmaxpartj;
+  int nb = 0, ne = 0;
+  if (lane < NR) neighbour_run<DIM>(s, P.cell_start, ci, cj, ck, lane, nb, ne);
+  int inc = ne - nb;
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const int v = __shfl_up_sync(FULL, inc, o, 16);
+    if ((lane & 15) >= o) inc += v;
+  }
+  __syncwarp();
+  if (lane < NR) {
+    const int rx = (DIM == 3) ? lane % 3 : lane;
+    runs[lane] = ListRun{inc, nb - (inc - (ne - nb)), (float)(rx - 1) * s.dcdf[0],
+                         (DIM == 3) ? (float)(lane / 3 - 1) * s.dcdf[1] : 0.f};
+  }
+  __syncwarp();
+  const int W = __shfl_sync(FULL, inc, NR - 1);
+  int* const list = b.nlist + 4 * list_base4(q, b.list_cap4);
+  int total = 0, last = -1, r = 0;
+  bool self_seen = false, self_kept = false;
+  for (int g0 = 0; g0 < W; g0 += 32 * UN) {
+    // UN candidates a lane, their loads in flight together
+    int e[UN];
+    float4 f[UN];
+#pragma unroll
+    for (int k = 0; k < UN; ++k) {
+      const int c = g0 + 32 * k + lane;
+      e[k] = -1;
+      if (c < W) {
+        while (c >= runs[r].end) ++r;
+        e[k] = (runs[r].base + c) | (r << kSlotBits);
+        f[k] = __ldg(P.XF + (runs[r].base + c));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < UN; ++k) {
+      const int c0 = g0 + 32 * k;
+      if (c0 >= W) break;
+      bool hit = false, self = false;
+      const int slot = e[k] & kSlotMask;
+      if (e[k] != -1) {
+        const int rk = (int)((unsigned)e[k] >> kSlotBits);
+        const float d0 = xq.x - (f[k].x + runs[rk].dx), d1 = (DIM == 3) ? xq.y - (f[k].y + runs[rk].dy) : 0.f;
+        const float d2 = xq.z - ((f[k].w - (float)ck) * s.dcdf[2] + f[k].z);
+        const float rr = __fmaf_rn(d2, d2, __fmaf_rn(d1, d1, __fmul_rn(d0, d0)));
+        hit = !(rr > s.rr_hi);
+        if (hit && !(rr < s.rr_lo)) {
+          const double4 xj = P.X[slot], xi = P.X[q];
+          const double r0 = xi.x - xj.x, r1 = xi.y - xj.y, r2 = xi.z - xj.z;
+          hit = !(r0 * r0 + r1 * r1 + r2 * r2 > s.square_doubleh);
+        }
+        self = hit && slot == q;
+      }
+      const unsigned m = __ballot_sync(FULL, hit), ms = __ballot_sync(FULL, self);
+      const int rank = total + __popc(m & below);
+      if (hit && !self && rank < cap) {
+        const int pos = rank - ((self_seen || (ms & below)) ? 1 : 0);
+        list[(size_t)(pos >> 2) * 128 + (pos & 3)] = e[k];
+      }
+      if (ms) {
+        self_seen = true;
+        self_kept = total + __popc(m & (ms - 1u)) < cap;
+      }
+      total += __popc(m);
+      if (m) last = c0 + 31 - __clz(m);
+    }
+  }
+  acc = min(total, cap);
+  cnt = acc - (self_kept ? 1 : 0);
+  cand = W;
+  trunc = total > cap || (total == cap && last < W - 1);
 }
 
-__device__ __forceinline__ bool window_candidate(const float4* wbuf, int u0, int nt, int ck) {
-  for (int u = u0; u < nt; ++u)
-    if (in_window(wbuf[u].w, ck)) return true;
-  return false;
-}
+// A lane's accepted entries wait in shared memory (kListWait rows of 32
+// lanes) until some lane of the warp has no room for its next tile, and then
+// go out in chunks of four: an entry costs a leading-zero count, a mask, a
+// load and a store, 9 instructions where collecting four in registers and
+// testing for a full chunk took about 25 and was half of the pass (a warp
+// waits in every tile for the lane with the most hits).
+constexpr int kListWait = 36;   // a tile's 32 and the up to 3 of an unfinished chunk
+
+// What a warp stages: the next candidates to be screened, a ring of two
+// tiles (negated x, y, z in the frame of the group's lowest cell, the list
+// entry, the z cell less that cell's predecessor), where the lanes' own
+// particles went, and each z cell's candidates of a tile.
+struct ListStage {
+  float nx[64], ny[64], nz[64];
+  int entry[64];
+  unsigned kmask[32];
+  int self_at[32];
+  unsigned char krel[64];
+};
+
+// The neighbour lists.  The lanes of a warp whose particles share a column of
+// cells, up to SPAN z cells apart, form a group.  The runs of the group's
+// common window are read as one sequence, 32 candidates at a time; the lane
+// that reads a candidate drops it if it is farther than 2h from the box around
+// the group's particles (a fifth of a dense 3D window: its edges and corners),
+// and what is left fills tiles of 32 across the runs, which every lane screens
+// (screen_tile).  A dense 3D group takes 16 tiles where a tile for each part of
+// each run took 27.
+//
+// Bound by instruction issue and, in small simulations, by a warp's chain of
+// tiles.  Blocks of two warps: small simulations spread over the SMs, and a
+// block does not wait for its slowest of eight warps.  Registers decide the
+// rest: 96 in 3D and 80 in 2D (9 and 12 blocks an SM asked for) keep the loop
+// out of local memory and beat fewer and more (box of 10^6, 8, 9, 12 and 16
+// blocks: 630, 568, 598 and 675 us; 2D, 1.02 10^6 particles, 9, 12 and 16:
+// 137, 122 and 131).  Against one tile for each run part and eight warps a
+// block, on one B200: 735 -> 568 us for that box, 483 -> 379 at 864,000
+// particles of the dam break, 68 -> 53 at 62,500, 157 -> 96 at 94,221 (columns
+// of about a warp's particles, where a warp spans a whole column), 133 -> 122
+// in 2D.
+constexpr int kListBlock = 64;
 
 template <int DIM>
-__global__ void __launch_bounds__(kBlock, 4) k_neighbour_lists(DevBatch b) {
+__global__ void __launch_bounds__(kListBlock, DIM == 3 ? 9 : 12) k_neighbour_lists(DevBatch b) {
+  constexpr int T = kListBlock, PARTS = kBlock / T;   // a tile's parts
+  constexpr int NR = (DIM == 3) ? 9 : 3, RY = (DIM == 3) ? 3 : 1, SPAN = (DIM == 3) ? 9 : kMostSpan;
+  static_assert((SPAN + 1) * RY <= 32, "one lane for each z cell and y column");
   __shared__ SimDev s;
-  __shared__ float4 cbuf[kBlock];
-  __shared__ __align__(16) float cneg[3][kBlock];   // the tile again: -x, -y, -z (paired screening)
+  __shared__ __align__(16) ListStage stage[T / 32];
+  __shared__ int wait[T / 32][kListWait][32];
+  __shared__ __align__(16) ListRun run_table[T / 32][NR];
   int cur = -1;
   const Particles& P = b.P;
-  const int lane = threadIdx.x & 31;
-  float4* wbuf = cbuf + (threadIdx.x & ~31);
-  float* wnx = &cneg[0][threadIdx.x & ~31];
-  float* wny = &cneg[1][threadIdx.x & ~31];
-  float* wnz = &cneg[2][threadIdx.x & ~31];
-  constexpr int NR = (DIM == 3) ? 9 : 3;
-  const unsigned FULL = 0xffffffffu;
-  for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-    Tile tl = b.tiles[t];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned FULL = 0xffffffffu, below = (1u << lane) - 1u;
+  ListStage& g = stage[warp];
+  ListRun* const runs = run_table[warp];
+  int* const mine_wait = &wait[warp][0][lane];
+  const int alone = b.ntiles < 2 * b.sms ? 20 : 6;   // quarters: the weight of a particle taken singly
+  for (int t = blockIdx.x; t < b.ntiles * PARTS; t += gridDim.x) {
+    const Tile tl = b.tiles[t / PARTS];
     load_sim(s, b.sims, tl.sim, cur);
     SimDyn* dyn = b.dyn + tl.sim;
-    int p = tl.start + threadIdx.x;
-    bool active = threadIdx.x < tl.count && p < s.p_off + dyn->nag && !dyn->frozen;
-    double4 xd = make_double4(0.0, 0.0, 0.0, 0.0);
+    const int at = (t % PARTS) * T + threadIdx.x;
+    const int p = tl.start + at;
+    const bool active = at < tl.count && p < s.p_off + dyn->nag && !dyn->frozen;
     float4 xf = make_float4(0.f, 0.f, 0.f, 0.f);
     int ci = 0, cj = 0, ck = 0;
     bool on = false;
     if (active) {
-      xd = P.X[p];
+      const double4 xd = P.X[p];
       xf = P.XF[p];
       on = particle_cell(s, xd.x, xd.y, xd.z, ci, cj, ck);
       if (!on) set_status(dyn, SPH_ERR_INVALID_ARGUMENT);   // state not re-sorted after a move
     }
-    int colkey = on ? (cj * s.ncd[0] + ci) : -1;
+    const int colkey = on ? (cj * s.ncd[0] + ci) : -1;
     unsigned remaining = __ballot_sync(FULL, on);
-    int cnt = 0, nacc = 0, cand = 0;
+    int done = 0, n = 0, nacc = 0, cand = 0;         // entries written, waiting; accepted, candidates
     bool trunc = false;
     const int cap = s.nmaxpartj;
     int4* out = reinterpret_cast<int4*>(b.nlist) + list_base4(p, b.list_cap4);
-    int4 pend = make_int4(0, 0, 0, 0);   // entries not yet written, oldest in x
-    const float rr_lo = s.rr_lo, rr_hi = s.rr_hi, dz = s.dcdf[2];
-    bool full = cap <= 0;                            // NMAXPARTJ reached
-    while (remaining) {
-      int leader = __ffs(remaining) - 1;
-      int key = __shfl_sync(FULL, colkey, leader);
-      unsigned group = __ballot_sync(FULL, on && colkey == key) & remaining;
-      remaining &= ~group;
-      bool mine = (group >> lane) & 1u;
-      int kmin = __reduce_min_sync(FULL, mine ? ck : 0x7fffffff);
-      int kmax = __reduce_max_sync(FULL, mine ? ck : -0x7fffffff);
-      int gci = __shfl_sync(FULL, ci, leader);
-      int gcj = __shfl_sync(FULL, cj, leader);
-      const bool rebase = kmax - kmin <= kRebaseSpan;          // uniform over the warp
-      const float zi = rebase ? (float)(ck - kmin) * dz + xf.z : 0.f;
-      for (int r = 0; r < NR; ++r) {
-        int jr = (DIM == 3) ? gcj - 1 + r / 3 : gcj;
-        int ir = gci - 1 + ((DIM == 3) ? r % 3 : r);
-        if (ir < 1 || ir > s.ncd[0] || jr < 1 || jr > s.ncd[1]) continue;
-        int klo = kmin > 1 ? kmin - 1 : 1;
-        int khi = kmax < s.ncd[2] ? kmax + 1 : s.ncd[2];
-        int base = s.cell_off + ((jr - 1) * s.ncd[0] + (ir - 1)) * s.ncd[2];
-        int ub = __ldg(P.cell_start + base + klo - 1);
-        int ue = __ldg(P.cell_start + base + khi);
-        // this lane's own window in the run, cells ck-1..ck+1: the slots the
-        // reference visits (CalcVarLength.f90's 27-cell block)
-        int wlo = 0, whi = 0;
-        if (mine) {
-          int ml = ck > 1 ? ck - 1 : 1, mh = ck < s.ncd[2] ? ck + 1 : s.ncd[2];
-          wlo = __ldg(P.cell_start + base + ml - 1);
-          whi = __ldg(P.cell_start + base + mh);
-          cand += whi - wlo;
+    const float mid = 0.5f * (s.rr_lo + s.rr_hi), delta = 0.5f * (s.rr_hi - s.rr_lo) * 1.01f, dz = s.dcdf[2];
+    // the waiting chunks of all lanes; what is left moves to the front
+    auto flush = [&]() {
+      const int chunks = n >> 2;
+      const int most = (int)__reduce_max_sync(FULL, (unsigned)chunks);
+      int4* o = out + (size_t)(done >> 2) * 32;
+      for (int k = 0; k < most; ++k) {
+        if (k < chunks) {
+          const int* e = mine_wait + 128 * k;
+          o[(size_t)k * 32] = make_int4(e[0], e[32], e[64], e[96]);
         }
-        float Dx = (float)(gci - ir) * s.dcdf[0];
-        float Dy = (DIM == 3) ? (float)(gcj - jr) * s.dcdf[1] : 0.f;
-        float ax = Dx + xf.x, ay = Dy + xf.y;
-        const int tag = r << kSlotBits;
-        for (int c0 = ub; c0 < ue; c0 += 32) {
-          int cidx = c0 + lane;
-          float4 st = (cidx < ue) ? P.XF[cidx] : make_float4(3.0e18f, 3.0e18f, 3.0e18f, -1.0e9f);
-          if (rebase && cidx < ue) st.z = (st.w - (float)kmin) * dz + st.z;
-          __syncwarp();
-          wbuf[lane] = st;
-          if (rebase) {
-            wnx[lane] = -st.x;
-            wny[lane] = -st.y;
-            wnz[lane] = -st.z;
-          }
-          __syncwarp();
-          if (!mine) continue;
-          int nt = ue - c0 < 32 ? ue - c0 : 32;
-          // phase 1: screening masks of the tile
-          unsigned hitm, lom;
-          if (rebase) screen_tile_x2<DIM>(wnx, wny, wnz, nt, ax, ay, zi, rr_lo, rr_hi, hitm, lom);
-          else screen_tile<DIM, false>(wbuf, nt, ax, ay, zi, xf.z, ck, dz, rr_lo, rr_hi, hitm, lom);
-          if (full) {
-            // NMAXPARTJ reached: every later candidate of the window is refused
-            if (!trunc && window_candidate(wbuf, 0, nt, ck)) trunc = true;
-            continue;
-          }
-          // only the lane's own window counts: the warp's union of runs
-          // reaches two z cells away from some lanes, and where the cells are
-          // narrower than 2h (CreaGrid rounds the cell count to nearest) a
-          // candidate there can lie within 2h without being the reference's
-          // neighbour; with cells at least 2h wide such a candidate is never
-          // a hit below the band, and band hits are tested below
-          if (s.narrow_z) hitm &= window_mask(wlo - c0, whi - c0);
-          // phase 2a (rare): resolve band hits -- outside the lane's window
-          // (the reference never visits those) or failing the FP64 test
-          // they are dropped; hitm then holds exactly the accepted ones
-          unsigned band = hitm & ~lom;
-          while (band) {
-            int u = __ffs(band) - 1;
-            band &= band - 1;
-            bool keep = in_window(wbuf[u].w, ck);
-            if (keep) {
-              double4 xq = P.X[c0 + u], xi = P.X[p];
-              double r0 = xi.x - xq.x, r1 = xi.y - xq.y, r2 = xi.z - xq.z;
-              double rr = r0 * r0 + r1 * r1 + r2 * r2;
-              keep = !(rr > s.square_doubleh);
-            }
-            if (!keep) hitm &= ~(1u << u);
-          }
-          if (nacc + __popc(hitm) >= cap) {
-            // reaching NMAXPARTJ in this tile (rare): accepted ones in
-            // visiting order up to the cap, then the truncation test
-            while (hitm) {
-              int u = __ffs(hitm) - 1;
-              hitm &= hitm - 1;
-              nacc++;
-              int q = c0 + u;
-              if (q != p) {
-                pend.x = pend.y;
-                pend.y = pend.z;
-                pend.z = pend.w;
-                pend.w = q | tag;
-                cnt++;
-                if ((cnt & 3) == 0) out[(size_t)((cnt >> 2) - 1) * 32] = pend;
-              }
-              if (nacc >= cap) {
-                full = true;
-                if (window_candidate(wbuf, u + 1, nt, ck)) trunc = true;   // window candidates follow
-                break;
-              }
-            }
-            continue;
-          }
-          // phase 2b: append the accepted ones in visiting order (the lane
-          // itself counted, not stored)
-          nacc += __popc(hitm);
-          unsigned self = (unsigned)(p - c0) < (unsigned)nt ? 1u << (p - c0) : 0u;
-          hitm &= ~self;
-          const int qbase = c0 | tag;                 // c0 + u < 2^28: no carry into the run bits
-          while (hitm) {
-            int u = __ffs(hitm) - 1;
-            hitm &= hitm - 1;
-            pend.x = pend.y;
-            pend.y = pend.z;
-            pend.z = pend.w;
-            pend.w = qbase + u;
-            cnt++;
-            if ((cnt & 3) == 0) out[(size_t)((cnt >> 2) - 1) * 32] = pend;
+      }
+      const int* e = mine_wait + 128 * chunks;
+      const int left = n & 3;
+      if (left > 0) mine_wait[0] = e[0];
+      if (left > 1) mine_wait[32] = e[32];
+      if (left > 2) mine_wait[64] = e[64];
+      done += 4 * chunks;
+      n = left;
+    };
+    while (remaining) {
+      const int leader = __ffs(remaining) - 1;
+      const int key = __shfl_sync(FULL, colkey, leader);
+      bool mine = ((remaining >> lane) & 1u) && colkey == key;
+      const int kmin = __reduce_min_sync(FULL, mine ? ck : 0x7fffffff);
+      mine = mine && ck - kmin <= SPAN;
+      const int kmax = __reduce_max_sync(FULL, mine ? ck : -0x7fffffff);
+      const unsigned group = __ballot_sync(FULL, mine);
+      remaining &= ~group;
+      const int gci = __shfl_sync(FULL, ci, leader);
+      const int gcj = __shfl_sync(FULL, cj, leader);
+      // the runs of the common window, and each z cell's candidates
+      const int klo = kmin > 1 ? kmin - 1 : 1, khi = kmax < s.ncd[2] ? kmax + 1 : s.ncd[2];
+      int ub = 0, ue = 0;
+      if (lane < NR) {
+        const int jr = (DIM == 3) ? gcj - 1 + lane / 3 : gcj, ir = gci - 1 + ((DIM == 3) ? lane % 3 : lane);
+        if (ir >= 1 && ir <= s.ncd[0] && jr >= 1 && jr <= s.ncd[1]) {
+          const int base = s.cell_off + ((jr - 1) * s.ncd[0] + (ir - 1)) * s.ncd[2];
+          ub = __ldg(P.cell_start + base + klo - 1);
+          ue = __ldg(P.cell_start + base + khi);
+        }
+      }
+      int part = 0;
+      {
+        const int k = kmin + lane / RY, jr = (DIM == 3) ? gcj - 1 + lane % RY : gcj;
+        if (k <= kmax && jr >= 1 && jr <= s.ncd[1]) {
+          const int ml = k > 1 ? k - 1 : 1, mh = k < s.ncd[2] ? k + 1 : s.ncd[2];
+#pragma unroll
+          for (int x = -1; x <= 1; ++x) {
+            if (gci + x < 1 || gci + x > s.ncd[0]) continue;
+            const int base = s.cell_off + ((jr - 1) * s.ncd[0] + (gci + x - 1)) * s.ncd[2];
+            part += __ldg(P.cell_start + base + mh) - __ldg(P.cell_start + base + ml - 1);
           }
         }
       }
+      int inc = ue - ub;
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, inc, o, 16);
+        if ((lane & 15) >= o) inc += v;
+      }
+      const int W = __shfl_sync(FULL, inc, NR - 1);
+      {
+        const int kr = mine ? (ck - kmin) * RY : 0;
+        int c = __shfl_sync(FULL, part, kr);
+        if (DIM == 3) c += __shfl_sync(FULL, part, kr + 1) + __shfl_sync(FULL, part, kr + 2);
+        if (mine) cand = c;
+      }
+      // few lanes, or a common window many times their own: a particle at a
+      // time (list_by_ballots).  Both sides are instruction counts: 160 and
+      // one a candidate for a particle, 256 and eight a candidate for the
+      // group's window, a particle's weighted 1.5 (127,008 particles: 133 us
+      // with 1, 128 with 1.5; 176,435: 126 and 109) and, where an SM has few
+      // warps and each waits for its own loads, 5 (13,500 particles: 60 us
+      // with groups of up to 7 taken singly, 47 with up to 2).
+      if (__popc(group) * (160 + __shfl_sync(FULL, cand, leader)) * alone < 4 * (256 + 8 * W)) {
+        for (unsigned left = group; left; left &= left - 1) {
+          const int o = __ffs(left) - 1;
+          const float4 xo = make_float4(__shfl_sync(FULL, xf.x, o), __shfl_sync(FULL, xf.y, o),
+                                        __shfl_sync(FULL, xf.z, o), 0.f);
+          int cn, ac, ca;
+          bool tr;
+          list_by_ballots<DIM>(s, b, p - lane + o, xo, gci, gcj, __shfl_sync(FULL, ck, o), runs, cn, ac, ca, tr);
+          if (lane == o) {
+            done = cn;
+            nacc = ac;
+            cand = ca;
+            trunc = tr;
+          }
+        }
+        continue;
+      }
+      __syncwarp();
+      if (lane < NR)
+        runs[lane] = ListRun{inc, ub - (inc - (ue - ub)), (float)(((DIM == 3) ? lane % 3 : lane) - 1) * s.dcdf[0],
+                             (DIM == 3) ? (float)(lane / 3 - 1) * s.dcdf[1] : 0.f};
+      g.self_at[lane] = -1;
+      // the box of the group's particles, offsets from its lowest cell's
+      // origin (not below 0: float bits order as integers), and the distance
+      // beyond which no lane's FP32 value can be within the band
+      const float zi = (float)(ck - kmin) * dz + xf.z;
+      const int far_lo = 0x7f000000;
+      const float bx0 = __int_as_float(__reduce_min_sync(FULL, mine ? __float_as_int(fmaxf(xf.x, 0.f)) : far_lo));
+      const float bx1 = __int_as_float(__reduce_max_sync(FULL, mine ? __float_as_int(fmaxf(xf.x, 0.f)) : 0));
+      const float bz0 = __int_as_float(__reduce_min_sync(FULL, mine ? __float_as_int(fmaxf(zi, 0.f)) : far_lo));
+      const float bz1 = __int_as_float(__reduce_max_sync(FULL, mine ? __float_as_int(fmaxf(zi, 0.f)) : 0));
+      float by0 = 0.f, by1 = 0.f;
+      if (DIM == 3) {
+        by0 = __int_as_float(__reduce_min_sync(FULL, mine ? __float_as_int(fmaxf(xf.y, 0.f)) : far_lo));
+        by1 = __int_as_float(__reduce_max_sync(FULL, mine ? __float_as_int(fmaxf(xf.y, 0.f)) : 0));
+      }
+      const float far2 = s.rr_hi * 1.001f;
+      bool full = cap <= 0;                          // NMAXPARTJ reached
+      if (full && mine) trunc = cand > 0;
+      __syncwarp();
+      // one tile of nt staged candidates, the first of them number c0
+      auto tile = [&](int c0, int nt) {
+        const int h = c0 & 32;
+        float near = 3.0e38f;
+        unsigned hitm = screen_tile<DIM>(g.nx + h, g.ny + h, g.nz + h, nt, xf.x, xf.y, zi, mid, near);
+        if (!mine) hitm = 0u;
+        // only the lane's own window counts: the group's common window
+        // reaches beyond some lanes', and where the cells are narrower than
+        // 2h (CreaGrid rounds the cell count to nearest) a candidate there
+        // can lie within 2h without being the reference's neighbour; with
+        // cells at least 2h wide such a candidate is never a hit below the
+        // band, and band hits are tested below
+        if (s.narrow_z) {
+          g.kmask[lane] = 0u;
+          __syncwarp();
+          const int kr = lane < nt ? g.krel[h + lane] & 31 : 31;
+          g.kmask[kr] = __brev(__match_any_sync(FULL, kr));
+          __syncwarp();
+          const unsigned* w = g.kmask + (mine ? ck - kmin : 0);
+          hitm &= w[0] | w[1] | w[2];
+        }
+        if (mine && near <= delta) {
+          // rare: candidates in the band -- outside the lane's window (the
+          // reference never visits those) or failing the FP64 test they
+          // are dropped; hitm then holds exactly the accepted ones
+          for (int u = 0; u < nt; ++u) {
+            const float d0 = xf.x + g.nx[h + u], d1 = (DIM == 3) ? xf.y + g.ny[h + u] : 0.f, d2 = zi + g.nz[h + u];
+            float rr = __fmul_rn(d0, d0);
+            if (DIM == 3) rr = __fmaf_rn(d1, d1, rr);
+            rr = __fmaf_rn(d2, d2, rr);
+            if (!(fabsf(rr - mid) <= delta)) continue;
+            const int slot = g.entry[h + u] & kSlotMask;
+            bool keep = fabsf(P.XF[slot].w - (float)ck) <= 1.0f;
+            if (keep) {
+              const double4 xq = P.X[slot], xi = P.X[p];
+              const double r0 = xi.x - xq.x, r1 = xi.y - xq.y, r2 = xi.z - xq.z;
+              keep = !(r0 * r0 + r1 * r1 + r2 * r2 > s.square_doubleh);
+            }
+            const unsigned bit = 0x80000000u >> u;
+            hitm = keep ? (hitm | bit) : (hitm & ~bit);
+          }
+        }
+        if (full) hitm = 0u;                         // every later candidate is refused
+        const int more = __popc(hitm);
+        if (nacc + more >= cap && more > 0) {
+          // reaching NMAXPARTJ in this tile (rare): the accepted ones in
+          // visiting order up to the cap; candidates of the window that
+          // follow the last of them are refused
+          unsigned keep = 0u;
+          int u = 0;
+          for (unsigned m = hitm; m && nacc < cap; ++nacc) {
+            u = __clz(m);
+            m &= 0x7fffffffu >> u;
+            keep |= 0x80000000u >> u;
+          }
+          hitm = keep;
+          if (nacc >= cap) {
+            full = true;
+            const int e = g.entry[h + u], last = (int)((unsigned)e >> kSlotBits);
+            const int ml = ck > 1 ? ck - 1 : 1, mh = ck < s.ncd[2] ? ck + 1 : s.ncd[2];
+            int seen = 0;
+            for (int r = 0; r <= last; ++r) {
+              const int jr = (DIM == 3) ? gcj - 1 + r / 3 : gcj, ir = gci - 1 + ((DIM == 3) ? r % 3 : r);
+              if (ir < 1 || ir > s.ncd[0] || jr < 1 || jr > s.ncd[1]) continue;
+              const int base = s.cell_off + ((jr - 1) * s.ncd[0] + (ir - 1)) * s.ncd[2];
+              const int wlo = P.cell_start[base + ml - 1];
+              seen += (r == last ? (e & kSlotMask) + 1 : P.cell_start[base + mh]) - wlo;
+            }
+            trunc = seen < cand;
+          }
+        } else {
+          nacc += more;
+        }
+        // the lane itself: counted, not stored
+        const unsigned self = (unsigned)(g.self_at[lane] - c0);
+        if (self < 32u) hitm &= ~(0x80000000u >> self);
+        const int add = __popc(hitm);
+        if (__any_sync(FULL, n + add > kListWait)) flush();
+        int* dst = mine_wait + 32 * n;
+        n += add;
+        const int* ent = g.entry + h;
+        while (hitm) {
+          const int u = __clz(hitm);
+          hitm &= 0x7fffffffu >> u;
+          *dst = ent[u];
+          dst += 32;
+        }
+      };
+      int staged = 0, screened = 0, r = 0, e = -1;
+      float4 f;
+      float dx = 0.f, dy = 0.f;
+      auto fetch = [&](int c) {                      // candidate c of the runs
+        e = -1;
+        if (c < W) {
+          while (c >= runs[r].end) ++r;
+          const ListRun q = runs[r];
+          e = (q.base + c) | (r << kSlotBits);
+          dx = q.dx;
+          dy = q.dy;
+          f = __ldg(P.XF + (q.base + c));
+        }
+      };
+      fetch(lane);
+      for (int c = lane; c - lane < W; c += 32) {
+        const int e0 = e;
+        bool keep = false;
+        float x = 0.f, y = 0.f, z = 0.f;
+        int kr = 0;
+        if (e0 != -1) {
+          x = f.x + dx;
+          y = f.y + dy;
+          z = (f.w - (float)kmin) * dz + f.z;
+          kr = (int)f.w - kmin + 1;
+          const float gx = fmaxf(fmaxf(bx0 - x, x - bx1), 0.f), gz = fmaxf(fmaxf(bz0 - z, z - bz1), 0.f);
+          float d = __fmaf_rn(gx, gx, gz * gz);
+          if (DIM == 3) {
+            const float gy = fmaxf(fmaxf(by0 - y, y - by1), 0.f);
+            d = __fmaf_rn(gy, gy, d);
+          }
+          keep = d <= far2;
+        }
+        fetch(c + 32);
+        const unsigned m = __ballot_sync(FULL, keep);
+        const int pos = staged + __popc(m & below), w = pos & 63;
+        if (keep) {
+          g.nx[w] = -x;
+          g.ny[w] = -y;
+          g.nz[w] = -z;
+          g.entry[w] = e0;
+          if (s.narrow_z) g.krel[w] = (unsigned char)kr;
+          const unsigned o = (unsigned)((e0 & kSlotMask) - (p - lane));
+          if (o < 32u && (int)((unsigned)e0 >> kSlotBits) == NR / 2) g.self_at[o] = pos;
+        }
+        staged += __popc(m);
+        __syncwarp();
+        if (staged - screened >= 32) {
+          tile(screened, 32);
+          screened += 32;
+          __syncwarp();
+        }
+      }
+      if (staged > screened) {
+        const int nt = staged - screened, w = (screened & 32) + lane;
+        if (lane >= nt) {
+          g.nx[w] = -3.0e18f;
+          g.ny[w] = -3.0e18f;
+          g.nz[w] = -3.0e18f;
+        }
+        __syncwarp();
+        tile(screened, nt);
+      }
+      __syncwarp();
     }
-    if (cnt & 3) {
-      // flush the last partial chunk, entries moved to its front
-      int rem = cnt & 3;
-      int4 w = pend;
-      if (rem == 1) w = make_int4(pend.w, 0, 0, 0);
-      else if (rem == 2) w = make_int4(pend.z, pend.w, 0, 0);
-      else w = make_int4(pend.y, pend.z, pend.w, 0);
-      out[(size_t)(cnt >> 2) * 32] = w;
+    flush();
+    if (n > 0) {
+      // the last, partial chunk
+      int4 w = make_int4(mine_wait[0], 0, 0, 0);
+      if (n > 1) w.y = mine_wait[32];
+      if (n > 2) w.z = mine_wait[64];
+      out[(size_t)(done >> 2) * 32] = w;
     }
     if (active) {
-      b.ncount[p] = cnt;
+      b.ncount[p] = done + n;
       if (trunc) atomicOr(&dyn->warnings, SPH_WARN_NEIGHBOURS_TRUNCATED);
     }
     block_count2(b.counters, cand, nacc);
-    int m = warp_max(nacc);
+    const int m = warp_max(nacc);
     if (lane == 0 && m > 0) atomicMax(&dyn->max_neigh, m);
   }
 }
@@ -4881,9 +5090,11 @@ void launch_momentum(const DevBatch& b, bool fused, cudaStream_t st) {
 }
 
 void launch_neighbour_lists(const DevBatch& b, cudaStream_t st) {
-  int g = blocks_for(b, kGridLists);
-  if (b.dim == 3) k_neighbour_lists<3><<<g, kBlock, 0, st>>>(b);
-  else k_neighbour_lists<2><<<g, kBlock, 0, st>>>(b);
+  // a chosen grid counts blocks of kBlock threads, as for the other passes
+  const int tiles = b.grid[kGridLists] > 0 && b.grid[kGridLists] < b.ntiles ? b.grid[kGridLists] : b.ntiles;
+  const int g = tiles * (kBlock / kListBlock);
+  if (b.dim == 3) k_neighbour_lists<3><<<g, kListBlock, 0, st>>>(b);
+  else k_neighbour_lists<2><<<g, kListBlock, 0, st>>>(b);
 }
 
 void launch_renormalisation(const DevBatch& b, cudaStream_t st) {
