@@ -1056,8 +1056,15 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   b.smooths = (h->any_teta_v || h->any_teta_p) ? 1 : 0;
   b.c1 = h->any_c1 ? 1 : 0;
   b.c1_divu = h->any_c1_divu ? 1 : 0;
-  b.mom_batch = 0;
-  b.con_batch = 0;
+  // the pair loops until they are chosen: with six tiles or more to an SM the
+  // lean FP32c momentum loop, of more warps an SM, hides the gathers better
+  // than the batched ones (dam break of 127,008 particles
+  // 94 us lean, 89 paired; 256,000: 155 and 156; 500,000: 261 and 272; box of
+  // 10^6: 483 and 542); the FP32c continuity loop is best paired at every size
+  // (62,500: 46 us lean, 38 paired; 864,000: 274 and 265), the FP64 one batched,
+  // the FP64 momentum loop lean.
+  b.mom_batch = h->precision == SPH_PREC_FP32C && b.ntiles < 6 * b.sms ? 2 : 0;
+  b.con_batch = h->precision == SPH_PREC_FP32C ? 2 : 1;
   *out = h;
   return SPH_OK;
 }
