@@ -86,8 +86,12 @@ __device__ __forceinline__ double div_rn_unsigned0(double a, double b, double y)
 }
 
 // q >= 1 and q >= 2 for q >= 0, from its upper word (integer instructions).
+// A NaN is not at or beyond 2 (its upper word lies past infinity's): a pair
+// with a NaN separation goes on to NaN terms, it is not passed over.
 __device__ __forceinline__ bool at_least_one(double q) { return __double2hiint(q) >= 0x3ff00000; }
-__device__ __forceinline__ bool at_least_two(double q) { return __double2hiint(q) >= 0x40000000; }
+__device__ __forceinline__ bool at_least_two(double q) {
+  return (unsigned)__double2hiint(q) - 0x40000000u <= 0x7ff00000u - 0x40000000u;
+}
 
 __device__ __forceinline__ bool particle_cell(const SimDev& s, double x, double y, double z, int& i, int& j,
                                               int& k) {
