@@ -303,9 +303,12 @@ int  sph_idle(SphHandle* h, int32_t* idle);
  * [6] the momentum and continuity shapes.                                 */
 int  sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out);
 /* Applies a launch configuration in sph_autotune's 7-entry layout (blocks
- * per kernel class, 0 = the default, then the two loop shapes), e.g. one
- * tuned earlier on a similar state; the next step rebuilds its graph.
- * Launch shapes change no result.                                          */
+ * per kernel class, 0 = the default, then the two loop shapes, -1 = the
+ * default for the simulation's size and form), e.g. one tuned earlier on a
+ * similar state; the next step rebuilds its graph.  The loop shapes and
+ * pair grids are those of the passes with one lane to a particle: without
+ * C1, simulations too small to fill the SMs so run four lanes to a
+ * particle instead, whatever the shape.  Launch shapes change no result.   */
 int  sph_set_launch_shape(SphHandle* h, const int32_t* shape);
 
 /* ---------------------------------------------------------------------- */

@@ -118,7 +118,8 @@ def _autotune(h, reps):
 
 
 def _set_launch_shape(h, shape):
-    g = np.array([int(shape.get(k, 0)) for k in _SHAPE_KEYS], np.int32)
+    # 0 blocks and loop shape -1: the defaults (a loop shape of 0 is the lean loop)
+    g = np.array([int(shape.get(k, -1 if k.endswith("_shape") else 0)) for k in _SHAPE_KEYS], np.int32)
     _chk(lib().sph_set_launch_shape(h, abi.iptr(g)), "sph_set_launch_shape")
 
 
@@ -302,7 +303,7 @@ class Simulation:
         return _autotune(self._h, reps)
 
     def set_launch_shape(self, shape):
-        """Applies a launch configuration (autotune's dict; missing keys 0)."""
+        """Applies a launch configuration (autotune's dict; a missing key is the default)."""
         _set_launch_shape(self._h, shape)
 
     # ------------------------------------------------------------ profiling

@@ -845,6 +845,16 @@ int build_graph(SphHandle* h) {
   return cuda_status(e);
 }
 
+// The pair loops until they are chosen: with six tiles or more to an SM the
+// lean FP32c momentum loop, of more warps an SM, hides the gathers better
+// than the batched ones (dam break of 127,008 particles
+// 94 us lean, 89 paired; 256,000: 155 and 156; 500,000: 261 and 272; box of
+// 10^6: 483 and 542); the FP32c continuity loop is best paired at every size
+// (62,500: 46 us lean, 38 paired; 864,000: 274 and 265), the FP64 one batched,
+// the FP64 momentum loop lean.
+int default_momentum_loop(const DevBatch& b) { return b.fp32c && b.ntiles < 6 * b.sms ? 2 : 0; }
+int default_continuity_loop(const DevBatch& b) { return b.fp32c ? 2 : 1; }
+
 // With bytes_out set, nothing touches the device: the arrays are sized,
 // their total goes to *bytes_out and no handle is returned.
 int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, const int32_t* caps,
@@ -1056,15 +1066,8 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   b.smooths = (h->any_teta_v || h->any_teta_p) ? 1 : 0;
   b.c1 = h->any_c1 ? 1 : 0;
   b.c1_divu = h->any_c1_divu ? 1 : 0;
-  // the pair loops until they are chosen: with six tiles or more to an SM the
-  // lean FP32c momentum loop, of more warps an SM, hides the gathers better
-  // than the batched ones (dam break of 127,008 particles
-  // 94 us lean, 89 paired; 256,000: 155 and 156; 500,000: 261 and 272; box of
-  // 10^6: 483 and 542); the FP32c continuity loop is best paired at every size
-  // (62,500: 46 us lean, 38 paired; 864,000: 274 and 265), the FP64 one batched,
-  // the FP64 momentum loop lean.
-  b.mom_batch = h->precision == SPH_PREC_FP32C && b.ntiles < 6 * b.sms ? 2 : 0;
-  b.con_batch = h->precision == SPH_PREC_FP32C ? 2 : 1;
+  b.mom_batch = default_momentum_loop(b);
+  b.con_batch = default_continuity_loop(b);
   *out = h;
   return SPH_OK;
 }
@@ -1730,19 +1733,19 @@ int sph_dump_renormalisation(SphHandle* h, double* b_gradp, double* b_divu) {
 // grid_out[5..6] the FP32c momentum and continuity loop shapes.
 
 // Applies a launch configuration (sph_autotune's output, or a chosen one):
-// blocks per kernel class (0 = the default) and the two pair-loop shapes.
+// blocks per kernel class (0 = the default) and the two pair-loop shapes
+// (-1 = the default).
 int sph_set_launch_shape(SphHandle* h, const int32_t* shape) {
   DeviceGuard dev_guard_(h);
   if (!h || !shape) return SPH_ERR_INVALID_ARGUMENT;
   for (int c = 0; c < kGridClasses; ++c)
     if (shape[c] < 0) return SPH_ERR_INVALID_ARGUMENT;
-  if (shape[kGridClasses] < 0 || shape[kGridClasses] > 2 || shape[kGridClasses + 1] < 0 ||
-      shape[kGridClasses + 1] > 2)
-    return SPH_ERR_INVALID_ARGUMENT;
+  const int mom = shape[kGridClasses], con = shape[kGridClasses + 1];
+  if (mom < -1 || mom > 2 || con < -1 || con > 2) return SPH_ERR_INVALID_ARGUMENT;
   SPH_CUDA(cudaStreamSynchronize(h->stream));
   for (int c = 0; c < kGridClasses; ++c) h->db.grid[c] = shape[c];
-  h->db.mom_batch = shape[kGridClasses];
-  h->db.con_batch = shape[kGridClasses + 1];
+  h->db.mom_batch = mom < 0 ? default_momentum_loop(h->db) : mom;
+  h->db.con_batch = con < 0 ? default_continuity_loop(h->db) : con;
   if (h->graph) {
     cudaGraphExecDestroy(h->graph);
     h->graph = nullptr;
