@@ -1084,18 +1084,33 @@ __device__ __forceinline__ void corner_integrals2d(const SimDev& s, const SideDe
 // particle close to one side finishes its entry itself; the corner particles
 // of the block (neighbours in the cell order) are then shared out over its
 // warps (corner_integrals2d).
-__global__ void __launch_bounds__(kBlock) k_boundary2d(DevBatch b) {
+//
+// It runs beside the list pass, whose blocks of 64 threads leave room for one
+// of their own kind at a time: a block of 256 found a place late, and the pass,
+// hidden before those small blocks came, cost its own time again (256 columns,
+// 4.48 10^6 particles in FP32c: 2.305 ms a step with blocks of 256, 2.261 of 128,
+// 2.253 of 64; 2.307 with lists in blocks of 256 as well).  Few tiles want the
+// corners shared over more warps, and the FP64 form, which has no pair sums
+// beside the pass, more of them: T = 128 from 8 tiles an SM in FP32c (80,000
+// particles: 76.6 us a step with 128, 75.3 with 256; 320,000: 179.1 and 180.3;
+// 500,000: 263.1 and 268.1; 1.02 10^6: 479 and 484) and from 32 in FP64 (80,000:
+// 120.0 and 117.1; 500,000: 418 and 411; 1.02 10^6: 773 and 769; 2.28 10^6 in 128
+// columns: 1723 and 1743).
+template <int T>
+__global__ void __launch_bounds__(T) k_boundary2d(DevBatch b) {
   chain_wait();
+  constexpr int PARTS = kBlock / T;   // a tile's parts
   __shared__ SimDev s;
-  __shared__ int ncorner, corner_ib[kBlock][2], corner_base[kBlock];
-  __shared__ double corner_xy[kBlock][4];   // x of both entries, y of both
+  __shared__ int ncorner, corner_ib[T][2], corner_base[T];
+  __shared__ double corner_xy[T][4];   // x of both entries, y of both
   int cur = -1;
   const Particles& P = b.P;
-  for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
-    Tile tl = b.tiles[t];
+  for (int t = blockIdx.x; t < b.ntiles * PARTS; t += gridDim.x) {
+    Tile tl = b.tiles[t / PARTS];
     load_sim(s, b.sims, tl.sim, cur);
-    const int p = tl.start + threadIdx.x;
-    const bool slot = threadIdx.x < tl.count;
+    const int at = (t % PARTS) * T + threadIdx.x;
+    const int p = tl.start + at;
+    const bool slot = at < tl.count;
     SimDyn* dyn = b.dyn + tl.sim;
     if (slot) P.bdt_count[p] = 0;
     const bool on = slot && p < s.p_off + dyn->nag && s.nsides > 0;
@@ -1202,7 +1217,7 @@ __global__ void __launch_bounds__(kBlock) k_boundary2d(DevBatch b) {
       corner_base[c] = gbase;
     }
     __syncthreads();
-    for (int c = threadIdx.x >> 5; c < ncorner; c += kBlock / 32)
+    for (int c = threadIdx.x >> 5; c < ncorner; c += T / 32)
       corner_integrals2d(s, sd, dyn, corner_ib[c], corner_xy[c], corner_xy[c] + 2, P.bdt + corner_base[c]);
     __syncthreads();
   }
@@ -5101,7 +5116,10 @@ void launch_boundary(const DevBatch& b, bool cleared, cudaStream_t st) {
     k_boundary3d<<<blocks_for(b, kGridBoundary), kBlock, 0, st>>>(b);
     launch_next(k_boundary3d_integrals, b.grid[kGridIntegrals] > 0 ? b.grid[kGridIntegrals] : b.grid_blocks, 128, st, b);
   } else {
-    k_boundary2d<<<blocks_for(b, kGridBoundary), kBlock, 0, st>>>(b);
+    // a chosen grid counts blocks of kBlock threads, as for the other passes
+    const int g = blocks_for(b, kGridBoundary);
+    if (b.ntiles >= (b.fp32c ? 8 : 32) * b.sms) k_boundary2d<128><<<2 * g, 128, 0, st>>>(b);
+    else k_boundary2d<kBlock><<<g, kBlock, 0, st>>>(b);
   }
 }
 
