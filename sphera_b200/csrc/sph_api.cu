@@ -845,15 +845,22 @@ int build_graph(SphHandle* h) {
   return cuda_status(e);
 }
 
-// The pair loops until they are chosen: with six tiles or more to an SM the
-// lean FP32c momentum loop, of more warps an SM, hides the gathers better
-// than the batched ones (dam break of 127,008 particles
-// 94 us lean, 89 paired; 256,000: 155 and 156; 500,000: 261 and 272; box of
-// 10^6: 483 and 542); the FP32c continuity loop is best paired at every size
-// (62,500: 46 us lean, 38 paired; 864,000: 274 and 265), the FP64 one batched,
-// the FP64 momentum loop lean.
-int default_momentum_loop(const DevBatch& b) { return b.fp32c && b.ntiles < 6 * b.sms ? 2 : 0; }
-int default_continuity_loop(const DevBatch& b) { return b.fp32c ? 2 : 1; }
+// The pair loops until they are chosen.  The FP64 form: momentum lean,
+// continuity batched, in 2D and 3D.  The FP32c form in 3D: with six tiles or
+// more to an SM the lean momentum loop, of more warps an SM, hides the gathers
+// better than the batched ones (dam break of 62,500 particles 53 us lean, 50
+// paired; 94,221: 66 and 71; 127,008: 89 and 86; 256,000: 152 and 151; 500,000:
+// 257 and 264; box of 10^6: 483 and 542); the continuity loop is best paired
+// (62,500: 46 us lean, 38 paired; 256,000: 109 and 101; 864,000: 274 and 265).
+// In 2D, with 20 neighbours instead of 78, both are lean from two tiles an SM
+// on (55,611 particles: momentum 24.9 us lean, 23.8 paired, continuity 21.5 and
+// 19.4; 80,000: 28.1 and 32.6, 21.7 and 21.3; 222,111: 48 and 52, 34 and 31;
+// 500,000: 96 and 110, 56 and 60; 1.02 10^6: 171 and 204, 99 and 107).
+int default_momentum_loop(const DevBatch& b) { return b.fp32c && b.ntiles < (b.dim == 3 ? 6 : 2) * b.sms ? 2 : 0; }
+int default_continuity_loop(const DevBatch& b) {
+  if (!b.fp32c) return 1;
+  return b.dim == 3 || b.ntiles < 2 * b.sms ? 2 : 0;
+}
 
 // With bytes_out set, nothing touches the device: the arrays are sized,
 // their total goes to *bytes_out and no handle is returned.
