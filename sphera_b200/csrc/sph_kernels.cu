@@ -5050,13 +5050,20 @@ static void launch_next(void (*kernel)(DevBatch, P...), int grid, int block, cud
 }
 
 static inline int blocks_for(const DevBatch& b) { return b.ntiles < b.grid_blocks ? b.ntiles : b.grid_blocks; }
-// The pair, list and boundary passes take one block to a tile unless a grid
-// has been chosen: they load little per block, and tiles handed out as blocks
-// finish even out what a fixed stride of 8 blocks an SM leaves uneven (FP32c
-// box of 10^6, lean momentum loop: 528 us so strided, 483 one to a tile).
+// The pair and list passes take one block to a tile unless a grid has been
+// chosen: they load little per block, and tiles handed out as blocks finish
+// even out what a fixed stride of 8 blocks an SM leaves uneven (FP32c box of
+// 10^6, lean momentum loop: 528 us so strided, 483 one to a tile).  So does the
+// wall pass of the FP64 form (64 2D columns, 1.1 10^6 particles: 882 us a step,
+// 891 strided).  That of the FP32c form, beside the lists and the pair sums,
+// strides 8 blocks an SM: it is not what the step waits for, and a block that
+// stays costs them less than many that come and go (2D column of 1.02 10^6: 490 us a step
+// one to a tile, 481 strided; 2.47 10^6: 1089 and 1082; 64 2D columns: 598 and 592;
+// 256: 2283 and 2270; 3D dam break of 4 10^6: 5302 and 5286).
 static inline int blocks_for(const DevBatch& b, int cls) {
-  if (b.grid[cls] <= 0) return b.ntiles;
-  return b.ntiles < b.grid[cls] ? b.ntiles : b.grid[cls];
+  int g = b.grid[cls];
+  if (g <= 0) g = cls == kGridBoundary && b.fp32c ? b.grid_blocks : b.ntiles;
+  return b.ntiles < g ? b.ntiles : g;
 }
 
 void launch_stage(const DevBatch& b, cudaStream_t st) { k_stage<<<blocks_for(b), kBlock, 0, st>>>(b); }
