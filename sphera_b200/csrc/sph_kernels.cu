@@ -86,12 +86,11 @@ __device__ __forceinline__ double div_rn_unsigned0(double a, double b, double y)
 }
 
 // q >= 1 and q >= 2 for q >= 0, from its upper word (integer instructions).
-// A NaN is not at or beyond 2 (its upper word lies past infinity's): a pair
-// with a NaN separation goes on to NaN terms, it is not passed over.
+// A NaN is at or beyond both: for pair terms that are multiplied by the
+// separation (or hold the velocities it became NaN from) and are NaN anyway.
+// A range test against it cost the FP64 step 0.2 to 0.6% (3D, from 256,000 particles).
 __device__ __forceinline__ bool at_least_one(double q) { return __double2hiint(q) >= 0x3ff00000; }
-__device__ __forceinline__ bool at_least_two(double q) {
-  return (unsigned)__double2hiint(q) - 0x40000000u <= 0x7ff00000u - 0x40000000u;
-}
+__device__ __forceinline__ bool at_least_two(double q) { return __double2hiint(q) >= 0x40000000; }
 
 __device__ __forceinline__ bool particle_cell(const SimDev& s, double x, double y, double z, int& i, int& j,
                                               int& k) {
@@ -3917,11 +3916,13 @@ __global__ void k_refresh_f32(DevBatch b) {
 // ==========================================================================
 
 // PartKernel(4) of CalcVarLength.f90:241-268: the kernel value W = wu coefke.
+// NaN for a NaN separation: the smoothing sums multiply W by values that need
+// not be NaN themselves, and the pair is not to be passed over.
 __device__ __forceinline__ double kernel_w(const SimDev& s, double rr) {
   double r = sqrt(rr);
   double q = div_rn_unsigned0(r, s.h, s.rcp_h);
   double q2 = div_rn_unsigned0(rr, s.squareh, s.rcp_squareh);
-  if (at_least_two(q)) return 0.0;
+  if (at_least_two(q) && !isnan(q)) return 0.0;
   double wu = 0.666666667 + q2 * (q * 0.5 - 1.0);
   if (at_least_one(q)) wu = (2.0 - q) * (2.0 - q) * (2.0 - q) * 0.166666666667;
   return wu * s.coefke;
