@@ -288,10 +288,12 @@ int  sph_memory_required(int32_t nsims, const SphParams* params, const SphGeomet
  * 0 while some is still running; never waits.                             */
 int  sph_idle(SphHandle* h, int32_t* idle);
 
-/* Autotuner (no reference counterpart): sizes the persistent grid of the
+/* Autotuner (no reference counterpart): sizes the grid of the
  * neighbour-list, momentum, continuity and boundary kernels on the live
  * state by timing `reps` launches of each candidate (1 to 32 blocks per
- * SM) of variants that leave the state unchanged, and for the momentum
+ * SM, and one block to a tile of 256 particles; the lists and the boundary
+ * pass beside each other, as a step runs them) of variants that leave the
+ * state unchanged, and for the momentum
  * and continuity pair loops also picks their shape (0: lean, one pair's
  * records at a time; 1: several list entries' records loaded together --
  * a list chunk's in the FP32c form, two entries' in the FP64 form; 2, FP32c
@@ -300,7 +302,9 @@ int  sph_idle(SphHandle* h, int32_t* idle);
  * in both forms.
  * grid_out (may be NULL; 7 entries) receives in [0..4] the chosen blocks
  * of lists, momentum, continuity, boundary find and integrals, in [5] and
- * [6] the momentum and continuity shapes.                                 */
+ * [6] the momentum and continuity shapes; a pair pass that runs four lanes
+ * to a particle (small simulations without C1) has nothing to choose and
+ * reports one block to a tile and its present shape.                       */
 int  sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out);
 /* Applies a launch configuration in sph_autotune's 7-entry layout (blocks
  * per kernel class, 0 = the default, then the two loop shapes, -1 = the

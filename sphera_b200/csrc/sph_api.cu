@@ -818,7 +818,7 @@ void step_sequence(SphHandle* h, cudaStream_t st, EarlyCopy* early = nullptr) {
   sort_sequence(h, true, st);
   cudaEventRecord(h->ev_fork, st);
   cudaStreamWaitEvent(h->stream2, h->ev_fork, 0);
-  launch_boundary(h->db, true, h->stream2);
+  launch_boundary(h->db, h->stream2);
   cudaEventRecord(h->ev_join, h->stream2);
   lists_pass(h, st);
   if (h->precision == SPH_PREC_FP32C) {
@@ -1158,7 +1158,7 @@ int upload_and_initialise(SphHandle* h, const SphState* states) {
   SPH_CUDA(cudaEventRecord(h->ev_rest, q3));
   SPH_CUDA(cudaEventRecord(h->ev_fork, q));
   SPH_CUDA(cudaStreamWaitEvent(h->stream2, h->ev_fork, 0));
-  launch_boundary(h->db, true, h->stream2);
+  launch_boundary(h->db, h->stream2);
   SPH_CUDA(cudaEventRecord(h->ev_join, h->stream2));
   launch_neighbour_lists(h->db, q);
   SPH_CUDA(cudaStreamWaitEvent(q, h->ev_join, 0));
@@ -1446,7 +1446,7 @@ int sph_replace_particles(SphHandle* h, const SphState* state, const int32_t* la
   launch_init_from_caller(h->db, h->d_cx, h->d_cv, h->d_crho, h->d_cp, h->d_cm, q);
   sort_sequence(h, true, q);
   if (laminar && state->n > 0) launch_load_laminar(h->db, h->d_ci1, q);
-  launch_boundary(h->db, true, q);
+  launch_boundary(h->db, q);
   lists_pass(h, q);
   SPH_CUDA(cudaGetLastError());
   return sync_dyn(h);
@@ -1575,7 +1575,8 @@ int sph_boundary_data_tab(SphHandle* h) {
   DeviceGuard dev_guard_(h);
   NvtxRange range_("ComputeBoundaryDataTab");
   if (!h || !h->uploaded) return SPH_ERR_INVALID_ARGUMENT;
-  launch_boundary(h->db, false, h->stream);
+  launch_boundary_reset(h->db, h->stream);
+  launch_boundary(h->db, h->stream);
   SPH_CUDA(cudaGetLastError());
   return sync_dyn(h);
 }
@@ -1730,11 +1731,12 @@ int sph_dump_renormalisation(SphHandle* h, double* b_gradp, double* b_divu) {
 }
 
 // ---------------------------------------------------------------- autotuner
-// Sizes the persistent grid of each kernel class on the live state: every
-// candidate (1 to 32 blocks per SM) is timed over `reps` launches of a
-// variant that leaves the state unchanged -- the rate-only momentum and
+// Sizes the grid of each kernel class on the live state: every candidate (1
+// to 32 blocks per SM, and one block to a tile) is timed over `reps` launches
+// of a variant that leaves the state unchanged -- the rate-only momentum and
 // continuity passes (their laminar-flag write is saved and restored), the
-// neighbour-list and boundary passes (idempotent) -- and the fastest kept.
+// neighbour-list and boundary passes (idempotent, timed beside each other) --
+// and the fastest kept.
 // The step graph is rebuilt with the choice.  grid_out[0..4] receives the
 // chosen blocks of lists, momentum, continuity, boundary find, integrals,
 // grid_out[5..6] the FP32c momentum and continuity loop shapes.
@@ -1766,7 +1768,6 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
   if (!h || !h->uploaded || reps <= 0) return SPH_ERR_INVALID_ARGUMENT;
   cudaStream_t q = h->stream;
   DevBatch& b = h->db;
-  const int mult[] = {1, 2, 4, 8, 16, 32};
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) { cudaGetLastError(); return SPH_ERR_CUDA; }
   // the rate-only momentum pass rewrites the laminar flags: keep them
@@ -1787,27 +1788,47 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
   // the momentum and continuity pair loops come in two shapes (lean, or
   // several list entries' records loaded together), the FP32c loops in a
   // third (batched, two entries' terms on paired FP32 instructions): all
-  // are timed
+  // are timed, but not where the passes run four lanes to a particle, which
+  // have neither a grid nor a shape to choose
   const bool two_shapes = !h->any_c1;
   const int pair_shapes = h->precision == SPH_PREC_FP32C ? 3 : 2;
   int best_batch = b.mom_batch, best_cbatch = b.con_batch;
+  // the lists and the wall pass as the step runs them: beside each other,
+  // and the FP32c pair sums of the continuity pass after the lists
+  auto search = [&]() {
+    launch_boundary_reset(b, q);
+    cudaEventRecord(h->ev_fork, q);
+    cudaStreamWaitEvent(h->stream2, h->ev_fork, 0);
+    launch_boundary(b, h->stream2);
+    cudaEventRecord(h->ev_join, h->stream2);
+    launch_neighbour_lists(b, q);
+    if (h->precision == SPH_PREC_FP32C) launch_continuity_f32_pairs(b, q);
+    cudaStreamWaitEvent(q, h->ev_join, 0);
+  };
+  // blocks: multiples of the SMs and, for a pass over tiles, one to a tile
+  auto grids = [&](int cls) {
+    std::vector<int> g;
+    for (int m = 1; m <= 32 && (cls == kGridIntegrals || b.sms * m < b.ntiles); m *= 2) g.push_back(b.sms * m);
+    if (cls != kGridIntegrals) g.push_back(b.ntiles);
+    return g;
+  };
   for (int cls = 0; cls < kGridClasses && e == cudaSuccess; ++cls) {
     if (cls == kGridIntegrals && h->dim != 3) continue;
     float best = 1e30f;
-    int best_g = 0;
+    int best_g = b.ntiles;
+    const bool split = (cls == kGridMomentum && momentum_split(b)) || (cls == kGridContinuity && continuity_split(b));
     const int nshapes = (two_shapes && (cls == kGridMomentum || cls == kGridContinuity)) ? pair_shapes : 1;
-    for (int cand = 0; cand < nshapes * 6; ++cand) {
-      const int m = mult[cand % 6];
-      if (nshapes > 1 && cls == kGridMomentum) b.mom_batch = cand / 6;
-      if (nshapes > 1 && cls == kGridContinuity) b.con_batch = cand / 6;
-      int g = b.sms * m;
-      b.grid[cls] = g;
+    const std::vector<int> g = grids(cls);
+    const int ng = (int)g.size();
+    for (int cand = 0; cand < nshapes * ng && !split; ++cand) {
+      if (nshapes > 1 && cls == kGridMomentum) b.mom_batch = cand / ng;
+      if (nshapes > 1 && cls == kGridContinuity) b.con_batch = cand / ng;
+      b.grid[cls] = g[cand % ng];
       auto run = [&]() {
         switch (cls) {
-          case kGridLists: launch_neighbour_lists(b, q); break;
           case kGridMomentum: momentum_pass(h, false, q); break;
           case kGridContinuity: continuity_pass(h, false, q); break;
-          default: launch_boundary(b, false, q); break;
+          default: search(); break;
         }
       };
       run();   // warm-up
@@ -1820,7 +1841,7 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
       if (e != cudaSuccess) break;
       if (ms < best) {
         best = ms;
-        best_g = g;
+        best_g = b.grid[cls];
         if (nshapes > 1 && cls == kGridMomentum) best_batch = b.mom_batch;
         if (nshapes > 1 && cls == kGridContinuity) best_cbatch = b.con_batch;
       }
@@ -1876,7 +1897,7 @@ int sph_profile_phases(SphHandle* h, int32_t nsteps, double* ms) {
     cudaEventRecord(ev[1], q);
     sort_sequence(h, true, q);
     cudaEventRecord(ev[2], q);
-    launch_boundary(h->db, true, q);
+    launch_boundary(h->db, q);
     cudaEventRecord(ev[3], q);
     lists_pass(h, q);
     cudaEventRecord(ev[4], q);

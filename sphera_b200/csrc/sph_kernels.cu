@@ -5118,8 +5118,11 @@ void launch_rank_reference(const DevBatch& b, const int* cell_start_ref, int* np
   k_rank_reference<<<blocks_for(b), kBlock, 0, st>>>(b, cell_start_ref, npartord);
 }
 
-void launch_boundary(const DevBatch& b, bool cleared, cudaStream_t st) {
-  if (!cleared) k_bdt_reset<<<(b.nsims + 127) / 128, 128, 0, st>>>(b);
+void launch_boundary_reset(const DevBatch& b, cudaStream_t st) {
+  k_bdt_reset<<<(b.nsims + 127) / 128, 128, 0, st>>>(b);
+}
+
+void launch_boundary(const DevBatch& b, cudaStream_t st) {
   if (b.dim == 3) {
     k_boundary3d<<<blocks_for(b, kGridBoundary), kBlock, 0, st>>>(b);
     launch_next(k_boundary3d_integrals, b.grid[kGridIntegrals] > 0 ? b.grid[kGridIntegrals] : b.grid_blocks, 128, st, b);
@@ -5143,12 +5146,14 @@ static void c1_frontier_2d(const DevBatch& b, bool gradp_only, cudaStream_t st) 
 // would leave an SM with fewer than `warps` warps.
 constexpr int kSplitFp64 = 7, kSplitMomentumF32 = 5, kSplitContinuityF32 = 8;
 static bool split_pairs(const DevBatch& b, int warps) { return !b.c1 && b.ntiles * (kBlock / 32) < b.sms * warps; }
+bool momentum_split(const DevBatch& b) { return split_pairs(b, b.fp32c ? kSplitMomentumF32 : kSplitFp64); }
+bool continuity_split(const DevBatch& b) { return split_pairs(b, b.fp32c ? kSplitContinuityF32 : kSplitFp64); }
 static int split_blocks(const DevBatch& b) { return b.ntiles * (kBlock / (kSplitThreads / 4)); }
 
 void launch_momentum(const DevBatch& b, bool fused, cudaStream_t st) {
   int g = blocks_for(b, kGridMomentum);
   c1_frontier_2d(b, true, st);
-  if (split_pairs(b, kSplitFp64)) {
+  if (momentum_split(b)) {
     const int gs = split_blocks(b);
     if (b.dim == 3) {
       if (fused) k_momentum_split<3, true><<<gs, kSplitThreads, 0, st>>>(b);
@@ -5205,14 +5210,14 @@ void launch_momentum_f32(const DevBatch& b, bool fused, cudaStream_t st) {
     if (fused) launch_next(k_momentum_f32_finish<3, true, true>, gf, kBlock, st, b);
     else launch_next(k_momentum_f32_finish<3, false, true>, gf, kBlock, st, b);
   } else if (b.dim == 3) {
-    if (split_pairs(b, kSplitMomentumF32)) k_momentum_f32_split<3><<<b.ntiles * 4, kBlock, 0, st>>>(b, f);
+    if (momentum_split(b)) k_momentum_f32_split<3><<<b.ntiles * 4, kBlock, 0, st>>>(b, f);
     else if (b.mom_batch == 2) k_momentum_f32<3, false, true, true><<<g, kBlock, 0, st>>>(b, f);
     else if (b.mom_batch) k_momentum_f32<3, false, true><<<g, kBlock, 0, st>>>(b, f);
     else k_momentum_f32<3><<<g, kBlock, 0, st>>>(b, f);
     if (fused) launch_next(k_momentum_f32_finish<3, true>, gf, kBlock, st, b);
     else launch_next(k_momentum_f32_finish<3, false>, gf, kBlock, st, b);
   } else {
-    if (split_pairs(b, kSplitMomentumF32)) k_momentum_f32_split<2><<<b.ntiles * 4, kBlock, 0, st>>>(b, f);
+    if (momentum_split(b)) k_momentum_f32_split<2><<<b.ntiles * 4, kBlock, 0, st>>>(b, f);
     else if (b.mom_batch == 2) k_momentum_f32<2, false, true, true><<<g, kBlock, 0, st>>>(b, f);
     else if (b.mom_batch) k_momentum_f32<2, false, true><<<g, kBlock, 0, st>>>(b, f);
     else k_momentum_f32<2><<<g, kBlock, 0, st>>>(b, f);
@@ -5224,8 +5229,8 @@ void launch_momentum_f32(const DevBatch& b, bool fused, cudaStream_t st) {
 void launch_continuity_f32_pairs(const DevBatch& b, cudaStream_t st) {
   int g = blocks_for(b, kGridContinuity);
   if (b.dim == 3 && b.c1_divu) launch_next(k_continuity_f32<3, true>, g, kBlock, st, b);
-  else if (split_pairs(b, kSplitContinuityF32) && b.dim == 3) launch_next(k_continuity_f32_split<3>, b.ntiles * 4, kBlock, st, b);
-  else if (split_pairs(b, kSplitContinuityF32)) launch_next(k_continuity_f32_split<2>, b.ntiles * 4, kBlock, st, b);
+  else if (continuity_split(b) && b.dim == 3) launch_next(k_continuity_f32_split<3>, b.ntiles * 4, kBlock, st, b);
+  else if (continuity_split(b)) launch_next(k_continuity_f32_split<2>, b.ntiles * 4, kBlock, st, b);
   else if (b.dim == 3 && b.con_batch == 2) launch_next(k_continuity_f32<3, false, true, true>, g, kBlock, st, b);
   else if (b.dim == 3 && b.con_batch) launch_next(k_continuity_f32<3, false, true>, g, kBlock, st, b);
   else if (b.dim == 3) launch_next(k_continuity_f32<3>, g, kBlock, st, b);
@@ -5259,7 +5264,7 @@ void launch_refresh_f32(const DevBatch& b, cudaStream_t st) { k_refresh_f32<<<bl
 void launch_continuity(const DevBatch& b, bool fused, cudaStream_t st) {
   int g = blocks_for(b, kGridContinuity);
   c1_frontier_2d(b, false, st);
-  if (split_pairs(b, kSplitFp64)) {
+  if (continuity_split(b)) {
     const int gs = split_blocks(b);
     if (b.dim == 3) {
       if (fused) k_continuity_split<3, true><<<gs, kSplitThreads, 0, st>>>(b);

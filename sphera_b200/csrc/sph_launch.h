@@ -61,9 +61,13 @@ void launch_rank_reference(const DevBatch& b, const int* cell_start_ref, int* np
 void launch_neighbour_lists(const DevBatch& b, cudaStream_t st);
 void launch_renormalisation(const DevBatch& b, cudaStream_t st);   // C1: fluid part of the matrices
 // physics (FP64)
-// cleared: the sort before it has cleared its counters
-void launch_boundary(const DevBatch& b, bool cleared, cudaStream_t st);
+// its counters are cleared by the sort before it, or by launch_boundary_reset
+void launch_boundary(const DevBatch& b, cudaStream_t st);
+void launch_boundary_reset(const DevBatch& b, cudaStream_t st);
 void launch_momentum(const DevBatch& b, bool fused, cudaStream_t st);
+// whether the momentum / continuity pair pass runs four lanes to a particle
+bool momentum_split(const DevBatch& b);
+bool continuity_split(const DevBatch& b);
 void launch_continuity(const DevBatch& b, bool fused, cudaStream_t st);
 // physics (FP32-compensated form)
 void launch_momentum_f32(const DevBatch& b, bool fused, cudaStream_t st);
