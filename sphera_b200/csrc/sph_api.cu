@@ -530,8 +530,9 @@ int prepare_sim(const SphParams& prm, const SphGeometry& g, int cap, HostSim& hs
     }
     // FindCloseBoundaryFaces3D visits the 27 cells around a particle's (x,
     // then y, then z) and takes a face at its first visit: one list per
-    // cell, in that order
+    // cell, in that order (taken[nf]: the last cell that took face nf)
     std::vector<uint8_t> near(s.ncells, 0);
+    std::vector<int> taken(g.n_faces + 1, -1);
     auto around = [&](int key, auto&& visit) {
       const int k = key % s.ncd[2] + 1, i = key / s.ncd[2] % s.ncd[0] + 1, j = key / s.ncd[2] / s.ncd[0] + 1;
       for (int a = std::max(i - 1, 1); a <= std::min(i + 1, s.ncd[0]); ++a)
@@ -544,9 +545,11 @@ int prepare_sim(const SphParams& prm, const SphGeometry& g, int cap, HostSim& hs
       hs.cf_start[key] = (int)hs.cf_list.size();
       if (!near[key]) continue;
       around(key, [&](int q) {
-        for (int nf : per[q])
-          if (std::find(hs.cf_list.begin() + hs.cf_start[key], hs.cf_list.end(), nf) == hs.cf_list.end())
-            hs.cf_list.push_back(nf);
+        for (int nf : per[q]) {
+          if (taken[nf] == key) continue;
+          taken[nf] = key;
+          hs.cf_list.push_back(nf);
+        }
       });
       hs.cf_count[key] = (int)hs.cf_list.size() - hs.cf_start[key];
     }
