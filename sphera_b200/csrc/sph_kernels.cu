@@ -288,6 +288,7 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanPer = 4;
 constexpr int kScanChunk = kScanThreads * kScanPer;
 constexpr int kBinChunks = 8;            // chunks around a block's first that k_bin gathers
+constexpr int kMostOwnSums = 16384;      // chunks (67 10^6 cells) up to which k_scan's blocks add up the sums before them
 
 // Cell key of every slot + atomic histogram, and the histogram's sums over
 // chunks of kScanChunk cells that the scan starts from.  KeyKind::Sort bins the
@@ -384,7 +385,7 @@ __device__ void replay_removals(const DevBatch& b, int sim) {
   d->warnings |= SPH_WARN_PARTICLES_REMOVED;
 }
 
-// Exclusive scan of the cell histogram (3 phases), clearing the histogram.
+// Exclusive scan of v over the block, and its total.
 __device__ __forceinline__ int block_excl_scan(int v, int* warp_sums, int& total) {
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int x = v;
@@ -417,7 +418,13 @@ __device__ __forceinline__ int block_excl_scan(int v, int* warp_sums, int& total
 // neither needs the other, so one launch holds what were four (chunk sums,
 // their scan, the scan, the removals).  These launches are latency alone:
 // at 5,000 particles the sort took 35 us in eight launches.
-__global__ void __launch_bounds__(kScanThreads) k_scan(DevBatch b, int n, int nb, int* cell_start, int removals) {
+//
+// summed: the chunk sums have been made prefix sums already (k_scan_sums).
+// Each block adding up all sums before its own is nothing for a few thousand
+// chunks and grows with their square (a sort in 151 10^6 cells 885 us so and 816
+// with prefix sums, in 302 10^6 1955 and 1591).
+__global__ void __launch_bounds__(kScanThreads) k_scan(DevBatch b, int n, int nb, int* cell_start, int removals,
+                                                       int summed) {
   chain_wait();
   if (blockIdx.x >= nb) {
     const int sim = blockIdx.x - nb;
@@ -435,7 +442,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(DevBatch b, int n, int nb
     v += vals[q];
   }
   int prev = 0;
-  for (int c = threadIdx.x; c < (int)blockIdx.x; c += kScanThreads) prev += b.scan_block_sums[c];
+  if (summed) prev = threadIdx.x == 0 ? b.scan_block_sums[blockIdx.x] : 0;
+  else
+    for (int c = threadIdx.x; c < (int)blockIdx.x; c += kScanThreads) prev += b.scan_block_sums[c];
   if (threadIdx.x == 0) before = 0;
   __syncthreads();
   prev = __reduce_add_sync(0xffffffffu, prev);
@@ -450,6 +459,21 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(DevBatch b, int n, int nb
     }
     ex += vals[q];
     if (base + q == n - 1) cell_start[n] = ex;
+  }
+}
+
+// The chunk sums in place of their exclusive prefix sums, by one block, for the
+// grids of very many chunks (kMostOwnSums).
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(int* sums, int nb) {
+  __shared__ int ws[32];
+  int carry = 0;
+  for (int c0 = 0; c0 < nb; c0 += kScanThreads) {
+    const int c = c0 + threadIdx.x;
+    const int v = c < nb ? sums[c] : 0;
+    int total;
+    const int ex = block_excl_scan(v, ws, total);
+    if (c < nb) sums[c] = carry + ex;
+    carry += total;
   }
 }
 
@@ -5076,7 +5100,10 @@ void launch_bin(const DevBatch& b, KeyKind kind, cudaStream_t st) {
 
 void launch_scan(const DevBatch& b, int* cell_start, bool removals, cudaStream_t st) {
   const int n = b.P.total_cells, nb = (n + kScanChunk - 1) / kScanChunk;
-  launch_next(k_scan, nb + (removals ? b.nsims : 0), kScanThreads, st, b, n, nb, cell_start, removals ? 1 : 0);
+  const bool summed = nb > kMostOwnSums;
+  if (summed) k_scan_sums<<<1, kScanThreads, 0, st>>>(b.scan_block_sums, nb);
+  launch_next(k_scan, nb + (removals ? b.nsims : 0), kScanThreads, st, b, n, nb, cell_start, removals ? 1 : 0,
+              summed ? 1 : 0);
 }
 
 void launch_cancel(const DevBatch& b, int sim, cudaStream_t st) { k_cancel<<<1, 32, 0, st>>>(b, sim); }
