@@ -1973,8 +1973,8 @@ int sph_measure_fma_peak(int32_t fp32, double* tflops) {
 
 int sph_measure_fp64_peak(double* tflops) { return sph_measure_fma_peak(0, tflops); }
 
-// The kernels' exact division (div_rn) against the IEEE division on count
-// generated operand pairs of the current device.
+// The kernels' exact divisions (div_rn, div_rn_unsigned0) against the IEEE
+// division on count generated operand pairs of the current device.
 int sph_check_division(uint64_t count, uint64_t seed, uint64_t* mismatches, double* first_bad) {
   if (!mismatches) return SPH_ERR_INVALID_ARGUMENT;
   int dev = 0, sms = 0;

@@ -4976,8 +4976,9 @@ double launch_fp64_probe(double* sink, int blocks, cudaStream_t st) {
   return 2.0 * 8.0 * iters * 256.0 * blocks;
 }
 
-// Self-check of div_rn against the IEEE division a / b on generated
-// operands (SplitMix64 of the seed and the operand index).  Five kinds, by
+// Self-check of div_rn and of div_rn_unsigned0 against the IEEE division a / b
+// (for the latter +0 where a is -0 and b positive) on generated operands
+// (SplitMix64 of the seed and the operand index).  Five kinds, by
 // index mod 5: random signs, significands and exponents in [-64, 63];
 // divisors whose significands are within 255 units of all ones; quotients
 // within a few units of 2^-106 relative of a rounding midpoint of a random
@@ -5031,8 +5032,10 @@ __global__ void __launch_bounds__(256) k_check_division(unsigned long long n, un
         break;
     }
     const double ref = a / b;
-    const double got = div_rn(a, b, __drcp_rn(b));
-    if (__double_as_longlong(ref) != __double_as_longlong(got)) {
+    const double y = __drcp_rn(b);
+    const double ref0 = a == 0.0 && b > 0.0 ? 0.0 : ref;
+    if (__double_as_longlong(ref) != __double_as_longlong(div_rn(a, b, y)) ||
+        __double_as_longlong(ref0) != __double_as_longlong(div_rn_unsigned0(a, b, y))) {
       ++nbad;
       if (atomicCAS(bad + 1, 0ull, 1ull) == 0ull) {   // the first mismatch found keeps its operands
         first[0] = a;
