@@ -811,8 +811,8 @@ void enqueue_early_copy(SphHandle* h, cudaStream_t st, EarlyCopy& ec) {
 // neighbour lists (FP32 screening, issue-bound) both read the freshly sorted
 // state and nothing the other writes, so the boundary pass runs on a second
 // stream beside the lists; captured into the step graph this is a fork and
-// a join.  The FP64 continuity pass starts its sum from the wall term (the
-// reference's order) and waits for both; the FP32c pass sums the pairs
+// a join.  The FP64 continuity pass is one launch, which takes its pair sum
+// from the wall term and waits for both; the FP32c pass sums the pairs
 // beside the boundary pass too and adds the wall term after the join.
 void step_sequence(SphHandle* h, cudaStream_t st, EarlyCopy* early = nullptr) {
   momentum_pass(h, true, st);

@@ -11,9 +11,9 @@
 //    which is increasing particle index inside a cell); inside a cell the
 //    sort orders particles by their caller index, like OrdGrid1's stable
 //    scatter.  The FP64 pair sums therefore run in the reference's order.
-//  * No neighbour lists are materialised: every pair pass recomputes the
-//    distance test and kernel values (the reference stores 60 B per pair
-//    slot, CalcVarLength.f90 / Gest_Trans.f90:138-166).
+//  * A particle's list holds 4-byte slot indices only: every pair pass
+//    recomputes separations and kernel values (the reference stores 60 B per
+//    pair slot, CalcVarLength.f90 / Gest_Trans.f90:138-166).
 //  * Several independent simulations can share one launch: every array is
 //    the concatenation of the simulations' segments and a block only ever
 //    works on one simulation (tile table), reading its SimDev into shared

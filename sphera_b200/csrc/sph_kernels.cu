@@ -1533,15 +1533,16 @@ __device__ __forceinline__ void elastic_reaction(const SimDev& s, const DevBatch
 // step serves its continuity pass and the next step's momentum pass, which
 // see the same positions.
 //
-// Layout: entry k of particle p at ((p / 32) * cap + k) * 32 + p % 32, so a
-// warp reads one 128-byte line per k.  An entry is slot | (run << 28); the
-// run gives the FP32 form the cell-origin difference of the pair.
+// Layout: chunks of four entries (list_base4).  An entry is
+// slot | (run << 28); the run gives the FP32 form the cell-origin difference
+// of the pair.
 //
 // The scan is warp-cooperative: the lanes of a warp that share a (y, x) cell
-// column (nearly always all of them, particles being sorted z-fastest) stage
-// the union of their 3-cell runs through shared memory 32 candidates at a
-// time and test them in lockstep; each lane keeps the candidates of its own
-// k-1..k+1 window, so its accepted sequence is exactly its reference order.
+// column (nearly always all of them, particles being sorted z-fastest) read
+// the runs of their common window, drop what is far from all of them, and
+// test what is left in lockstep, 32 candidates at a time from shared memory;
+// each lane keeps the candidates of its own k-1..k+1 window, in the order of
+// the runs, so its accepted sequence is exactly its reference order.
 // ==========================================================================
 constexpr int kSplitThreads = 128;   // threads of the four-lane FP64 pair passes
 constexpr int kSlotBits = 28;
@@ -1784,8 +1785,8 @@ struct ListStage {
 // Bound by instruction issue and, in small simulations, by a warp's chain of
 // tiles.  Blocks of two warps: small simulations spread over the SMs, and a
 // block does not wait for its slowest of eight warps.  Registers decide the
-// rest: 96 in 3D and 80 in 2D (9 and 12 blocks an SM asked for) keep the loop
-// out of local memory and beat fewer and more (box of 10^6, 8, 9, 12 and 16
+// rest: 96 in 3D and 80 in 2D (9 and 12 blocks an SM asked for; 12 bytes a thread
+// spilled) beat fewer and more (box of 10^6, 8, 9, 12 and 16
 // blocks: 630, 568, 598 and 675 us; 2D, 1.02 10^6 particles, 9, 12 and 16:
 // 137, 122 and 131).  Against one tile for each run part and eight warps a
 // block, on one B200: 735 -> 568 us for that box, 483 -> 379 at 864,000
@@ -3335,8 +3336,8 @@ struct MomentumPairs {
 // Momentum, FP32c form, in two launches.  k_momentum_f32 holds only what
 // the pair loop needs -- the particle's FP32 values, the compensated sums,
 // the list chunk being read and the next one -- so that it runs at 3 blocks
-// of 256 per SM without spilling (gathers are latency-bound: occupancy pays
-// more than loading the next pair's records ahead), and writes the nine
+// of 256 per SM with 12 bytes a thread spilled (gathers are latency-bound:
+// occupancy pays more than loading the next pair's records ahead), and writes the nine
 // compensated sums of each particle to MSUM.
 // k_momentum_f32_finish adds the FP64 wall terms (an independent sum), the
 // laminar flag, gravity and the elastic reaction and, in the fused step,
@@ -3717,7 +3718,7 @@ struct ContinuityPairs {
 // BATCH (not with DIVU): a list chunk's eight neighbour records requested
 // before the chunk's arithmetic, at 3 blocks per SM; the same sums.
 // PAIRED (with BATCH): two entries' terms on paired FP32 instructions
-// (contrib2), the same bits as two calls of `contrib`.
+// (pair2), the same bits as two calls of `pair`.
 template <int DIM, bool DIVU = false, bool BATCH = false, bool PAIRED = false>
 __global__ void __launch_bounds__(kBlock, DIVU ? 2 : (BATCH ? 3 : 5)) k_continuity_f32(DevBatch b) {
   chain_wait();

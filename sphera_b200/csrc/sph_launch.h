@@ -33,7 +33,7 @@ struct DevBatch {
   int scan_nblocks;
   int grid_blocks;         // blocks of the persistent particle kernels (default)
   int sms;                 // streaming multiprocessors of the device
-  int grid[kGridClasses];  // autotuned blocks per kernel class (0 = grid_blocks)
+  int grid[kGridClasses];  // chosen blocks per kernel class (0 = the default: see blocks_for)
   int mom_batch;           // momentum pair loop: 1 = several entries' records loaded together, 2 = the same
                            // with two entries' terms on paired FP32 instructions (FP32c; autotuned)
   int con_batch;           // the same for the continuity pair loop (0, 1, 2)

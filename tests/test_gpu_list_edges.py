@@ -1,8 +1,8 @@
 """The neighbour search where its scan branches: groups of few particles and
 whole warps, blocks of few candidates and of many tiles, lists far longer than
 a lane's waiting entries, lists at NMAXPARTJ, thin columns (a warp over many z
-cells), coordinates far from the origin, and the launch for larger
-simulations.  Whole numbers: counts and lists equal to the oracle's, in its
+cells), coordinates far from the origin, and simulations on both sides of the
+change in what a particle taken singly is held to cost.  Whole numbers: counts and lists equal to the oracle's, in its
 order."""
 import numpy as np
 import pytest
@@ -59,8 +59,9 @@ CASES = {
 }
 
 
-# from 296 tiles of 256 particles on (two to each of 148 SMs) the scan runs in
-# larger blocks: columns about a warp's particles apart, both cell widths, 2D
+# from 296 tiles of 256 particles on (two to each of 148 SMs) a particle taken
+# singly weighs less against its group's common window: columns about a warp's
+# particles apart, both cell widths, 2D
 LARGE = {
     "dam_94221": lambda: cases.dam_break_3d(dx=0.0105, jitter=0.1, seed=5),
     "box_75777": lambda: cases.random_box(n=296 * 256 + 1, seed=5),
