@@ -3453,7 +3453,7 @@ __global__ void __launch_bounds__(kBlock, (C1 || BATCH) ? 2 : 3) k_momentum_f32(
 }
 
 // k_momentum_f32 with four lanes to a particle, for simulations too small to
-// fill the SMs with one (split_pairs): lane j of a particle sums list
+// fill the SMs with one (momentum_split): lane j of a particle sums list
 // chunks j, j + 4, ... and the chunk sums change hands through shared
 // memory; lane j < 3 keeps the compensated sums of one kind (pressure,
 // Monaghan, Morris) and adds the chunks to them in list order, so every sum
@@ -5173,12 +5173,21 @@ static void c1_frontier_2d(const DevBatch& b, bool gradp_only, cudaStream_t st) 
   else k_c1_frontier_2d<false><<<blocks_for(b), kBlock, 0, st>>>(b);
 }
 
-// Four lanes to a particle in a pair pass (without C1): while one lane each
-// would leave an SM with fewer than `warps` warps.
-constexpr int kSplitFp64 = 7, kSplitMomentumF32 = 5, kSplitContinuityF32 = 8;
-static bool split_pairs(const DevBatch& b, int warps) { return !b.c1 && b.ntiles * (kBlock / 32) < b.sms * warps; }
-bool momentum_split(const DevBatch& b) { return split_pairs(b, b.fp32c ? kSplitMomentumF32 : kSplitFp64); }
-bool continuity_split(const DevBatch& b) { return split_pairs(b, b.fp32c ? kSplitContinuityF32 : kSplitFp64); }
+// Four lanes to a particle in a pair pass (without C1), while one lane each
+// would leave an SM with fewer than so many warps.  One lane takes the same time up to
+// about 8 warps an SM (a particle's chain of pairs), four lanes are one wave of
+// blocks at first and then two.  FP32c: the lines are the ends of that wave, 2 and 3
+// blocks an SM (momentum us one lane / four: 3D 18,513 particles 39.6 / 29.9,
+// 23,328 39.9 / 39.9; 2D 15,576 20.9 / 19.5, 21,632 21.5 / 25.4.  Continuity:
+// 2D 15,576 17.4 / 15.3, 27,730 17.4 / 17.4, 32,131 17.4 / 19.4), and in 3D, whose
+// lists of 78 make the chain longer, two waves still pay for the continuity
+// (37,044: 33.2 / 31.7).  FP64 (momentum: 3D 37,044 82.8 / 73.2; 2D 32,131 28.2 /
+// 27.8, 33,800 27.8 / 29.1).
+bool momentum_split(const DevBatch& b) { return !b.c1 && b.ntiles * (kBlock / 32) < b.sms * (b.fp32c ? 4 : 7); }
+bool continuity_split(const DevBatch& b) {
+  const int warps = b.fp32c ? (b.dim == 3 ? 8 : 6) : 7;
+  return !b.c1 && b.ntiles * (kBlock / 32) < b.sms * warps;
+}
 static int split_blocks(const DevBatch& b) { return b.ntiles * (kBlock / (kSplitThreads / 4)); }
 
 void launch_momentum(const DevBatch& b, bool fused, cudaStream_t st) {

@@ -1,6 +1,6 @@
 """The pair passes with one lane to a particle, which simulations of 38,000
-particles and more run (smaller ones without C1 take four lanes, whatever their
-launch shape): each loop shape against the oracle beside walls, all shapes and
+particles and more run (smaller ones without C1 take four lanes, the FP32c form
+up to 19,000 in the momentum pass, whatever their launch shape): each loop shape against the oracle beside walls, all shapes and
 grids against one another bit for bit, and a member's results with four lanes,
 alone, against those with one, in a batch that fills the SMs."""
 import numpy as np
@@ -64,6 +64,31 @@ def test_every_shape_on_the_oracle_and_the_same_bits(dim, precision, oracle_lib)
         if first is None:
             first = got
         assert all(np.array_equal(a, b) for a, b in zip(got, first)), shape
+
+
+# either side of four warps an SM (FP32c momentum) and, in 2D, of six (FP32c
+# continuity) on 148 SMs: 73 and 74 tiles of 256 particles, 110 and 111
+EDGES = {
+    "box_73": lambda: cases.random_box(n=73 * 256, seed=21, precision=abi.SPH_PREC_FP32C),
+    "box_74": lambda: cases.random_box(n=74 * 256, seed=21, precision=abi.SPH_PREC_FP32C),
+    "column_110": lambda: _moving(cases.dam_break_2d(dx=0.00845, jitter=0.1, precision=abi.SPH_PREC_FP32C)),
+    "column_111": lambda: _moving(cases.dam_break_2d(dx=0.0084, jitter=0.1, precision=abi.SPH_PREC_FP32C)),
+}
+
+
+@pytest.mark.parametrize("name", list(EDGES))
+def test_fp32c_rates_where_lanes_change_over(name, oracle_lib):
+    case = EDGES[name]()
+    assert (case.n + 255) // 256 == int(name.split("_")[1])
+    o = oracle_lib.Oracle(case)
+    o.prepare()
+    o.rhs_momentum()
+    o.continuity()
+    want = o.get()
+    sim = Simulation(case)
+    sim.upload(case.state)
+    for got, ref in ((sim.rhs_momentum(), want["acc"]), (sim.continuity(), want["dden"])):
+        assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref)
 
 
 @pytest.mark.parametrize("precision", FORMS)
