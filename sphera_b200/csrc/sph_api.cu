@@ -1734,9 +1734,9 @@ int sph_dump_renormalisation(SphHandle* h, double* b_gradp, double* b_divu) {
 }
 
 // ---------------------------------------------------------------- autotuner
-// Sizes the grid of each kernel class on the live state: every candidate (1
-// to 32 blocks per SM, and one block to a tile) is timed over `reps` launches
-// of a variant that leaves the state unchanged -- the rate-only momentum and
+// Sizes the grid of each kernel class on the live state: the candidates (one
+// block to a tile, and 32 blocks per SM down to 1, until fewer have lost a
+// quarter of the time) are timed over `reps` launches of a variant that leaves the state unchanged -- the rate-only momentum and
 // continuity passes (their laminar-flag write is saved and restored), the
 // neighbour-list and boundary passes (idempotent, timed beside each other) --
 // and the fastest kept.
@@ -1808,11 +1808,13 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
     if (h->precision == SPH_PREC_FP32C) launch_continuity_f32_pairs(b, q);
     cudaStreamWaitEvent(q, h->ev_join, 0);
   };
-  // blocks: multiples of the SMs and, for a pass over tiles, one to a tile
+  // blocks, from the most down: one to a tile for a pass over tiles, and
+  // multiples of the SMs
   auto grids = [&](int cls) {
     std::vector<int> g;
-    for (int m = 1; m <= 32 && (cls == kGridIntegrals || b.sms * m < b.ntiles); m *= 2) g.push_back(b.sms * m);
     if (cls != kGridIntegrals) g.push_back(b.ntiles);
+    for (int m = 32; m >= 1; m /= 2)
+      if (cls == kGridIntegrals || b.sms * m < b.ntiles) g.push_back(b.sms * m);
     return g;
   };
   for (int cls = 0; cls < kGridClasses && e == cudaSuccess; ++cls) {
@@ -1820,33 +1822,36 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
     float best = 1e30f;
     int best_g = b.ntiles;
     const bool split = (cls == kGridMomentum && momentum_split(b)) || (cls == kGridContinuity && continuity_split(b));
-    const int nshapes = (two_shapes && (cls == kGridMomentum || cls == kGridContinuity)) ? pair_shapes : 1;
-    const std::vector<int> g = grids(cls);
-    const int ng = (int)g.size();
-    for (int cand = 0; cand < nshapes * ng && !split; ++cand) {
-      if (nshapes > 1 && cls == kGridMomentum) b.mom_batch = cand / ng;
-      if (nshapes > 1 && cls == kGridContinuity) b.con_batch = cand / ng;
-      b.grid[cls] = g[cand % ng];
-      auto run = [&]() {
-        switch (cls) {
-          case kGridMomentum: momentum_pass(h, false, q); break;
-          case kGridContinuity: continuity_pass(h, false, q); break;
-          default: search(); break;
+    const int nshapes = split ? 0 : (two_shapes && (cls == kGridMomentum || cls == kGridContinuity)) ? pair_shapes : 1;
+    for (int shape = 0; shape < nshapes && e == cudaSuccess; ++shape) {
+      if (nshapes > 1 && cls == kGridMomentum) b.mom_batch = shape;
+      if (nshapes > 1 && cls == kGridContinuity) b.con_batch = shape;
+      float best_of_shape = 1e30f;
+      for (const int g : grids(cls)) {
+        b.grid[cls] = g;
+        auto run = [&]() {
+          switch (cls) {
+            case kGridMomentum: momentum_pass(h, false, q); break;
+            case kGridContinuity: continuity_pass(h, false, q); break;
+            default: search(); break;
+          }
+        };
+        if (best_of_shape == 1e30f) run();   // warm-up: another grid runs the same code on the same data
+        cudaEventRecord(e0, q);
+        for (int r = 0; r < reps; ++r) run();
+        cudaEventRecord(e1, q);
+        e = cudaEventSynchronize(e1);
+        float ms = 0.f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        if (e != cudaSuccess) break;
+        if (ms < best) {
+          best = ms;
+          best_g = g;
+          if (nshapes > 1 && cls == kGridMomentum) best_batch = shape;
+          if (nshapes > 1 && cls == kGridContinuity) best_cbatch = shape;
         }
-      };
-      run();   // warm-up
-      cudaEventRecord(e0, q);
-      for (int r = 0; r < reps; ++r) run();
-      cudaEventRecord(e1, q);
-      e = cudaEventSynchronize(e1);
-      float ms = 0.f;
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-      if (e != cudaSuccess) break;
-      if (ms < best) {
-        best = ms;
-        best_g = b.grid[cls];
-        if (nshapes > 1 && cls == kGridMomentum) best_batch = b.mom_batch;
-        if (nshapes > 1 && cls == kGridContinuity) best_cbatch = b.con_batch;
+        best_of_shape = std::min(best_of_shape, ms);
+        if (ms > 1.25f * best_of_shape) break;   // fewer blocks leave the SMs emptier still
       }
     }
     b.grid[cls] = best_g;
