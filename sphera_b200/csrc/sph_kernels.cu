@@ -1782,8 +1782,10 @@ struct ListStage {
 // (screen_tile).  A dense 3D group takes 16 tiles where a tile for each part of
 // each run took 27.
 //
-// Bound by instruction issue and, in small simulations, by a warp's chain of
-// tiles.  Blocks of two warps: small simulations spread over the SMs, and a
+// Bound by latency: a warp waits for its own shared memory, shuffles and
+// results (6.7 of an instruction's 7.7 warp-cycles at 256,000 particles, with 4.3
+// warps a scheduler; issue slots 57% busy, no pipe above 44%), in small
+// simulations for its chain of tiles.  Blocks of two warps: small simulations spread over the SMs, and a
 // block does not wait for its slowest of eight warps.  Registers decide the
 // rest: 96 in 3D and 80 in 2D (9 and 12 blocks an SM asked for; 12 bytes a thread
 // spilled) beat fewer and more (box of 10^6, 8, 9, 12 and 16
