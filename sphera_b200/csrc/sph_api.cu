@@ -808,7 +808,7 @@ void enqueue_early_copy(SphHandle* h, cudaStream_t st, EarlyCopy& ec) {
 }
 
 // One whole step.  The boundary data (SA-SPH, FP64, latency-bound) and the
-// neighbour lists (FP32 screening, issue-bound) both read the freshly sorted
+// neighbour lists (FP32 screening) both read the freshly sorted
 // state and nothing the other writes, so the boundary pass runs on a second
 // stream beside the lists; captured into the step graph this is a fork and
 // a join.  The FP64 continuity pass is one launch, which takes its pair sum

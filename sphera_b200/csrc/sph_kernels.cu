@@ -3875,8 +3875,10 @@ __global__ void __launch_bounds__(kBlock) k_continuity_f32_finish(DevBatch b) {
     const double rhoi = P.RP[p].x;
     double dden = 0.0;
     const int nb = P.bdt_count[p];
-    double4 vi = make_double4(0.0, 0.0, 0.0, 0.0);   // read by the wall terms alone
-    if (nb > 0) vi = P.V[p];
+    // read by the wall terms alone; with C1 loaded always: a selected load takes
+    // the launch from 127 registers to 154, from two blocks an SM to one
+    double4 vi = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (C1 || nb > 0) vi = P.V[p];
     if (C1 && DIM == 3 && s.c1_be) {
       dden = continuity_boundary_c1(s, b, dyn, nb, nb > 0 ? P.bdt_start[p] : 0, vi, rhoi, p);
       if (s.c1_divu) {
