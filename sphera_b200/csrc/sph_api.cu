@@ -1775,8 +1775,9 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) { cudaGetLastError(); return SPH_ERR_CUDA; }
   // the rate-only momentum pass rewrites the laminar flags: keep them
   SPH_CUDA(cudaMemcpyAsync(b.P.L2, b.P.L, (size_t)h->total_slots, cudaMemcpyDeviceToDevice, q));
-  // with C1 the momentum (first step) and continuity passes complete and
-  // invert the renormalisation matrices in place: keep them too
+  // with C1 the list pass forms the renormalisation matrices and the momentum
+  // (first step) and continuity passes complete and invert them in place:
+  // keep them too
   const size_t nb_bytes = sizeof(double) * 9 * (size_t)h->total_slots;
   double *keep_g = nullptr, *keep_d = nullptr;
   cudaError_t e = cudaSuccess;
@@ -1796,15 +1797,16 @@ int sph_autotune(SphHandle* h, int32_t reps, int32_t* grid_out) {
   const bool two_shapes = !h->any_c1;
   const int pair_shapes = h->precision == SPH_PREC_FP32C ? 3 : 2;
   int best_batch = b.mom_batch, best_cbatch = b.con_batch;
-  // the lists and the wall pass as the step runs them: beside each other,
-  // and the FP32c pair sums of the continuity pass after the lists
+  // the lists and the wall pass as the step runs them: beside each other, the
+  // C1 matrices (kept above) and the FP32c pair sums of the continuity pass
+  // after the lists
   auto search = [&]() {
     launch_boundary_reset(b, q);
     cudaEventRecord(h->ev_fork, q);
     cudaStreamWaitEvent(h->stream2, h->ev_fork, 0);
     launch_boundary(b, h->stream2);
     cudaEventRecord(h->ev_join, h->stream2);
-    launch_neighbour_lists(b, q);
+    lists_pass(h, q);
     if (h->precision == SPH_PREC_FP32C) launch_continuity_f32_pairs(b, q);
     cudaStreamWaitEvent(q, h->ev_join, 0);
   };
