@@ -934,6 +934,7 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
     // particle (Gest_Trans.f90:90), far more than a flow uses
     const size_t quota = hs.prm.bdt_capacity > 0 ? (size_t)hs.prm.bdt_capacity : (size_t)hs.cap * (h->dim == 3 ? 3 : 2);
     if (quota > 0x7fffffff) { delete h; return SPH_ERR_INVALID_ARGUMENT; }
+    hs.dev.bdt_off = (int)bdt_cap;
     hs.dev.bdt_quota = (int)quota;
     bdt_cap += quota;
   }
@@ -988,7 +989,6 @@ int create_batch(int nsims, const SphParams* params, const SphGeometry* geoms, c
   A(h->d_ncount, N);
 #undef A
   if (st != SPH_OK) { sph_destroy(h); return st; }
-  P.bdt_cap = (int)std::min(bdt_cap, (size_t)0x7fffffff);
   P.total_cells = coff;
   P.total_slots = poff;
   // host tables -> device

@@ -44,7 +44,7 @@ struct SimDev {
   int cap;                // particle slots reserved
   int nmaxpartj;          // NMAXPARTJ
   int maxcb;              // MAXCLOSEBOUNDFACES (3D) / MAXCLOSEBOUNDSIDES (2D)
-  int bdt_quota;          // BoundaryDataTab entries this simulation may take from the pool
+  int bdt_off, bdt_quota; // its part of the BoundaryDataTab pool: first entry, entries
   int ioff;               // slab of a decomposed simulation: local x cell i is global cell i + ioff
                           // (extr_lo and dcd stay the whole grid's, so cells are assigned as in it)
   int face_off, nfaces;   // faces (3D)
@@ -169,7 +169,6 @@ struct Particles {
   int* bdt_count;   // per particle
   int* bdt_start;
   BdtEntry* bdt;
-  int bdt_cap;
   // sort work
   int* key;         // global cell key of slot
   int* slot;        // position inside the cell from the atomic histogram

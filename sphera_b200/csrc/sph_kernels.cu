@@ -634,7 +634,7 @@ struct FaceTest {
 // The hemisphere table as the quadrature reads it.  coef(q, l, .) are the
 // factors of point q in the three sums of lane l: (1, 1, r2 r2), (r0, r1,
 // r2), (r0 r0, r0 r1, r0 r2) and (r1 r1, r1 r2, r2 r2).
-struct SharedBit {
+struct BitTable {
   const double (*xy)[2];      // [256] x, y of the points
   const double (*ring)[2];    // [8] z and weight of a ring's points (the same for all of them)
   const double (*cf)[12];     // [256] the factors, lane by lane
@@ -644,21 +644,6 @@ struct SharedBit {
   __device__ __forceinline__ double da(int r) const { return ring[r][1]; }
   __device__ __forceinline__ void coef(int q, int l, double* c) const {
     for (int k = 0; k < 3; ++k) c[k] = cf[q][3 * l + k];
-  }
-};
-
-struct GlobalBit {
-  const double* bit;          // [256][7] of the simulation
-  __device__ __forceinline__ double x(int q) const { return bit[7 * q]; }
-  __device__ __forceinline__ double y(int q) const { return bit[7 * q + 1]; }
-  __device__ __forceinline__ double z(int r) const { return bit[7 * 32 * r + 2]; }
-  __device__ __forceinline__ double da(int r) const { return bit[7 * 32 * r + 3]; }
-  __device__ __forceinline__ void coef(int q, int l, double* c) const { factors(bit + 7 * q, l, c); }
-  __device__ static __forceinline__ void factors(const double* row, int l, double* c) {
-    const double r0 = row[4], r1 = row[5], r2 = row[6];
-    c[0] = l == 0 ? 1.0 : (l == 1 ? r0 : (l == 2 ? r0 * r0 : r1 * r1));
-    c[1] = l == 0 ? 1.0 : (l == 1 ? r1 : (l == 2 ? r0 * r1 : r1 * r2));
-    c[2] = l == 0 ? r2 * r2 : (l == 1 ? r2 : (l == 2 ? r0 * r2 : r2 * r2));
   }
 };
 
@@ -673,9 +658,8 @@ struct GlobalBit {
 // this pass: by one lane (12 sums, 256 tests and the products of the
 // factors, which come from the table here) it took 65 us at 13,500
 // particles and 143 us at 864,000.
-template <class BIT>
-__device__ __forceinline__ void face_integrals(const SimDev& s, const BIT& bit, const FaceDev& f, const double* locx,
-                                               int l, double* sum) {
+__device__ __forceinline__ void face_integrals(const SimDev& s, const BitTable& bit, const FaceDev& f,
+                                               const double* locx, int l, double* sum) {
   FaceTest ft;
   ft.load(f);
   sum[0] = sum[1] = sum[2] = 0.0;
@@ -785,36 +769,32 @@ __device__ __forceinline__ void face_integrals(const SimDev& s, const BIT& bit, 
 
 // Room for n boundary entries of each lane's particle (one simulation to a
 // warp): the first entry, or -1 where n is 0 or there is none.  Each
-// simulation draws on its own quota of the shared pool first, so one that
-// overflows fails alone and the others' entries are unaffected.  One
-// addition per warp and counter: a lane's own met all the others at one
-// address (72 us for the 864,000-particle dam break's face search).
+// simulation draws on its own part of the pool, so one that overflows fails
+// alone and the others' entries are unaffected; what is left of the part when
+// a particle's entries don't fit is marked (face 0), so that every entry
+// below the count is one of this pass.  One addition per warp and counter: a
+// lane's own met all the others at one address (72 us for the
+// 864,000-particle dam break's face search).
 __device__ __forceinline__ int claim_entries(const SimDev& s, const DevBatch& b, SimDyn* dyn, int n) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   if (!__any_sync(FULL, n > 0)) return -1;
-  auto scan = [&](int v) {
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(FULL, v, o);
-      if (lane >= o) v += u;
-    }
-    return v;
-  };
-  int inc = scan(n), base = 0;
+  int inc = n, base = 0;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(FULL, inc, o);
+    if (lane >= o) inc += u;
+  }
   if (lane == 31) base = atomicAdd(&dyn->bdt_sim_used, inc);
   base = __shfl_sync(FULL, base, 31);
+  const int first = base + inc - n;
   if (n > 0 && base + inc > s.bdt_quota) {
     set_status(dyn, SPH_ERR_BDT_OVERFLOW);
+    for (int k = first; k < s.bdt_quota; ++k) b.P.bdt[s.bdt_off + k].clobonum = 0;
     n = 0;
   }
-  inc = scan(n);
-  if (lane == 31) base = atomicAdd(&b.dyn[b.nsims].bdt_used, inc);  // global allocation counter
-  base = __shfl_sync(FULL, base, 31);
-  if (n > 0 && base + inc > b.P.bdt_cap) {
-    set_status(dyn, SPH_ERR_BDT_OVERFLOW);
-    n = 0;
-  }
-  return n > 0 ? base + inc - n : -1;
+  const int taken = __reduce_add_sync(FULL, n);
+  if (lane == 31 && taken > 0) atomicAdd(&b.dyn[b.nsims].bdt_used, taken);   // of all simulations (diagnostics)
+  return n > 0 ? s.bdt_off + first : -1;
 }
 
 // ComputeBoundaryDataTab_3D.f90:67-105 with FindCloseBoundaryFaces3D.f90:79-188:
@@ -890,75 +870,96 @@ __global__ void __launch_bounds__(kBlock) k_boundary3d(DevBatch b) {
       e.loc[1] = locx[1];
       e.loc[2] = locx[2];
       e.clobonum = clob[u];
-      e.pad = tl.sim;            // the integrals pass needs the simulation
     }
+  }
+}
+
+// The integrals of entry e by its four lanes.
+__device__ __forceinline__ void boundary_entry(const SimDev& s, const BitTable& bit, const DevBatch& b, BdtEntry& e,
+                                               int l) {
+  if (e.clobonum == 0) return;
+  const double locx[3] = {e.loc[0], e.loc[1], e.loc[2]};
+  double sum[3];
+  face_integrals(s, bit, b.faces[s.face_off + e.clobonum - 1], locx, l, sum);
+  if (l == 0) {
+    e.bi[0] = 0.0;
+    e.bi[1] = sum[0];
+    e.bi[2] = sum[1];
+    e.bi[6] = sum[2];
+    e.bi[7] = 0.0;
+  } else if (l == 1) {
+    for (int k = 0; k < 3; ++k) e.bi[3 + k] = sum[k];
+  } else if (l == 2) {
+    e.ig[0] = sum[0];
+    e.ig[1] = e.ig[3] = sum[1];
+    e.ig[2] = e.ig[6] = sum[2];
+  } else {
+    e.ig[4] = sum[0];
+    e.ig[5] = e.ig[7] = sum[1];
+    e.ig[8] = sum[2];
   }
 }
 
 // ComputeBoundaryVolumeIntegrals_P0.f90:81-155 for every entry the find
 // pass allocated, four lanes to a (particle, face): the quadrature costs are
 // balanced across the GPU whatever the particles' distribution over tiles.
+// A block works on chunks of 32 entries of one simulation, whose constants and
+// hemisphere table it holds in shared memory; the chunks of 128 simulations at a
+// time are numbered through, one simulation after the other.  (Entries of a
+// pool that the members share as they come mix in a chunk, and those of another
+// member than the table's read theirs from global memory: 300 members of 500
+// particles 806 us, 20 of 13,500 457; with a part of the pool each 372 and 201.)
 __global__ void __launch_bounds__(128) k_boundary3d_integrals(DevBatch b) {
   chain_wait();
-  // the simulation constants and hemisphere table of the chunk's first
-  // entry, staged in shared memory (a batch chunk can mix simulations:
-  // entries of another one read theirs from global memory)
+  constexpr int PER = 32, GROUP = 128;
   __shared__ SimDev ssim;
   __shared__ double sxy[kBitRows][2];
   __shared__ double sring[8][2];
   __shared__ double scf[kBitRows][12];
+  __shared__ int ends[GROUP], part[GROUP / 32];   // chunks up to the end of each simulation of the group
   int loaded = -1;
-  int used = b.dyn[b.nsims].bdt_used;
-  if (used > b.P.bdt_cap) used = b.P.bdt_cap;
-  const int l = threadIdx.x & 3;
-  const int per = blockDim.x / 4;
-  for (int base = blockIdx.x * per; base < used; base += gridDim.x * per) {
-    const int first = b.P.bdt[base].pad;
-    if (first != loaded) {
-      load_sim(ssim, b.sims, first, loaded);
-      const double* src = b.bit + (size_t)first * kBitRows * 7;
-      for (int q = threadIdx.x; q < kBitRows; q += blockDim.x) {
-        const double* row = src + 7 * q;
-        sxy[q][0] = row[0];
-        sxy[q][1] = row[1];
-        if ((q & 31) == 0) {
-          sring[q >> 5][0] = row[2];
-          sring[q >> 5][1] = row[3];
+  const int l = threadIdx.x & 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto entries = [&](int sim) { return min(b.dyn[sim].bdt_sim_used, b.sims[sim].bdt_quota); };
+  int before = 0, next = blockIdx.x;               // chunks of the groups so far; this block's next one
+  for (int s0 = 0; s0 < b.nsims; s0 += GROUP) {
+    int end = s0 + (int)threadIdx.x < b.nsims ? (entries(s0 + threadIdx.x) + PER - 1) / PER : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    __syncthreads();                               // the last group's ends are no longer read
+    if (lane == 31) part[warp] = end;
+    __syncthreads();
+    end += before;
+    for (int w = 0; w < warp; ++w) end += part[w];
+    ends[threadIdx.x] = end;
+    __syncthreads();
+    for (; next < ends[GROUP - 1]; next += gridDim.x) {
+      int k = 0;                                   // the first simulation that ends past the chunk
+      for (int step = GROUP / 2; step > 0; step >>= 1)
+        if (ends[k + step - 1] <= next) k += step;
+      const int sim = s0 + k, chunk = next - (k > 0 ? ends[k - 1] : before);
+      if (sim != loaded) {
+        load_sim(ssim, b.sims, sim, loaded);
+        const double* src = b.bit + (size_t)sim * kBitRows * 7;
+        for (int q = threadIdx.x; q < kBitRows; q += blockDim.x) {
+          const double* row = src + 7 * q;
+          const double r0 = row[4], r1 = row[5], r2 = row[6];
+          sxy[q][0] = row[0];
+          sxy[q][1] = row[1];
+          if ((q & 31) == 0) {
+            sring[q >> 5][0] = row[2];
+            sring[q >> 5][1] = row[3];
+          }
+          const double c[12] = {1.0, 1.0, r2 * r2, r0, r1, r2, r0 * r0, r0 * r1, r0 * r2, r1 * r1, r1 * r2, r2 * r2};
+          for (int j = 0; j < 12; ++j) scf[q][j] = c[j];
         }
-        for (int k = 0; k < 4; ++k) GlobalBit::factors(row, k, &scf[q][3 * k]);
+        __syncthreads();
       }
-      __syncthreads();
+      const int idx = chunk * PER + (threadIdx.x >> 2);
+      if (idx < entries(sim)) boundary_entry(ssim, BitTable{sxy, sring, scf}, b, b.P.bdt[ssim.bdt_off + idx], l);
     }
-    const int idx = base + (threadIdx.x >> 2);
-    if (idx >= used) continue;
-    BdtEntry& e = b.P.bdt[idx];
-    const int sim = e.pad;
-    const double locx[3] = {e.loc[0], e.loc[1], e.loc[2]};
-    double sum[3];
-    if (sim == loaded) {
-      face_integrals(ssim, SharedBit{sxy, sring, scf}, b.faces[ssim.face_off + e.clobonum - 1], locx, l, sum);
-    } else {
-      const SimDev& s = b.sims[sim];
-      face_integrals(s, GlobalBit{b.bit + (size_t)sim * kBitRows * 7}, b.faces[s.face_off + e.clobonum - 1], locx, l,
-                     sum);
-    }
-    if (l == 0) {
-      e.bi[0] = 0.0;
-      e.bi[1] = sum[0];
-      e.bi[2] = sum[1];
-      e.bi[6] = sum[2];
-      e.bi[7] = 0.0;
-    } else if (l == 1) {
-      for (int k = 0; k < 3; ++k) e.bi[3 + k] = sum[k];
-    } else if (l == 2) {
-      e.ig[0] = sum[0];
-      e.ig[1] = e.ig[3] = sum[1];
-      e.ig[2] = e.ig[6] = sum[2];
-    } else {
-      e.ig[4] = sum[0];
-      e.ig[5] = e.ig[7] = sum[1];
-      e.ig[8] = sum[2];
-    }
+    before = ends[GROUP - 1];
   }
 }
 

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from sphera_b200 import Simulation, abi, cases
+from sphera_b200 import Batch, Simulation, abi, cases
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +37,27 @@ def test_both_block_sizes_give_the_same_entries(oracle_lib):
     assert np.array_equal(n, on) and np.array_equal(clob, oc)
     near = n > 0
     assert np.linalg.norm(vals[near] - ov[near]) <= 1.0e-12 * np.linalg.norm(ov[near])
+
+
+@pytest.mark.parametrize("precision", [abi.SPH_PREC_FP64, abi.SPH_PREC_FP32C])
+def test_members_of_a_3d_batch_have_their_own_entries(precision):
+    """The 3D integrals number the chunks of 128 members at a time: members on
+    both sides of that, of unequal sizes, one without particles near a wall's
+    end and one without any, each bit for bit as alone."""
+    cs = [cases.dam_break_3d(dx=0.06 if i % 3 else 0.05, jitter=0.1, seed=i, precision=precision) for i in range(131)]
+    empty = cs[126]
+    none = abi.State.empty(0)
+    batch = Batch(cs)
+    states = [c.state for c in cs]
+    states[126] = none
+    batch.upload(states)
+    batch.step(6)
+    for i in (0, 1, 3, 125, 127, 128, 130):
+        alone = Simulation(cs[i])
+        alone.upload(cs[i].state)
+        alone.step(6)
+        a, b = alone.download(), batch.download(i)
+        for f in ("x", "v", "rho", "p"):
+            assert np.array_equal(getattr(a, f), getattr(b, f)), (i, f)
+        alone.close()
+    assert batch.download(126).n == 0 and empty.n > 0
