@@ -1788,8 +1788,8 @@ struct ListStage {
 // warps a scheduler; issue slots 57% busy, no pipe above 44%), in small
 // simulations for its chain of tiles.  Blocks of two warps: small simulations spread over the SMs, and a
 // block does not wait for its slowest of eight warps.  Registers decide the
-// rest: 96 in 3D and 80 in 2D (9 and 12 blocks an SM asked for; 12 bytes a thread
-// spilled) beat fewer and more (box of 10^6, 8, 9, 12 and 16
+// rest: 96 in 3D and 80 in 2D (9 and 12 blocks an SM asked for) keep the loop
+// out of local memory and beat fewer and more (box of 10^6, 8, 9, 12 and 16
 // blocks: 630, 568, 598 and 675 us; 2D, 1.02 10^6 particles, 9, 12 and 16:
 // 137, 122 and 131).  Against one tile for each run part and eight warps a
 // block, on one B200: 735 -> 568 us for that box, 483 -> 379 at 864,000
@@ -1950,8 +1950,7 @@ __global__ void __launch_bounds__(kListBlock, DIM == 3 ? 9 : 12) k_neighbour_lis
         by1 = __int_as_float(__reduce_max_sync(FULL, mine ? __float_as_int(fmaxf(xf.y, 0.f)) : 0));
       }
       const float far2 = s.rr_hi * 1.001f;
-      bool full = cap <= 0;                          // NMAXPARTJ reached
-      if (full && mine) trunc = cand > 0;
+      int at_cap = 0;                                // the entry at which a lane reached NMAXPARTJ
       __syncwarp();
       // one tile of nt staged candidates, the first of them number c0
       auto tile = [&](int c0, int nt) {
@@ -1995,34 +1994,25 @@ __global__ void __launch_bounds__(kListBlock, DIM == 3 ? 9 : 12) k_neighbour_lis
             hitm = keep ? (hitm | bit) : (hitm & ~bit);
           }
         }
-        if (full) hitm = 0u;                         // every later candidate is refused
+        if (nacc >= cap) hitm = 0u;                  // NMAXPARTJ reached: every later candidate is refused
         const int more = __popc(hitm);
         if (nacc + more >= cap && more > 0) {
           // reaching NMAXPARTJ in this tile (rare): the accepted ones in
-          // visiting order up to the cap; candidates of the window that
-          // follow the last of them are refused
-          unsigned keep = 0u;
-          int u = 0;
-          for (unsigned m = hitm; m && nacc < cap; ++nacc) {
-            u = __clz(m);
-            m &= 0x7fffffffu >> u;
-            keep |= 0x80000000u >> u;
-          }
-          hitm = keep;
-          if (nacc >= cap) {
-            full = true;
-            const int e = g.entry[h + u], last = (int)((unsigned)e >> kSlotBits);
-            const int ml = ck > 1 ? ck - 1 : 1, mh = ck < s.ncd[2] ? ck + 1 : s.ncd[2];
-            int seen = 0;
-            for (int r = 0; r <= last; ++r) {
-              const int jr = (DIM == 3) ? gcj - 1 + r / 3 : gcj, ir = gci - 1 + ((DIM == 3) ? r % 3 : r);
-              if (ir < 1 || ir > s.ncd[0] || jr < 1 || jr > s.ncd[1]) continue;
-              const int base = s.cell_off + ((jr - 1) * s.ncd[0] + (ir - 1)) * s.ncd[2];
-              const int wlo = P.cell_start[base + ml - 1];
-              seen += (r == last ? (e & kSlotMask) + 1 : P.cell_start[base + mh]) - wlo;
+          // visiting order up to the cap, candidate u the last of them
+          int u = 0, left = cap - nacc;
+          unsigned m = hitm;
+#pragma unroll
+          for (int w = 16; w > 0; w >>= 1) {
+            const int c = __popc(m >> (32 - w));
+            if (c < left) {
+              left -= c;
+              m <<= w;
+              u += w;
             }
-            trunc = seen < cand;
           }
+          hitm &= ~(0x7fffffffu >> u);
+          nacc = cap;
+          at_cap = g.entry[h + u];
         } else {
           nacc += more;
         }
@@ -2104,6 +2094,23 @@ __global__ void __launch_bounds__(kListBlock, DIM == 3 ? 9 : 12) k_neighbour_lis
         __syncwarp();
         tile(screened, nt);
       }
+      if (mine && nacc >= cap) {
+        // whether candidates of the window follow the one that reached the
+        // cap: here for all lanes at a time, not for a tile's few lanes each
+        // (200,000 particles cut to 43 of 74 neighbours: 204 us so, 191 here)
+        int seen = 0;
+        if (cap > 0) {
+          const int last = (int)((unsigned)at_cap >> kSlotBits);
+          const int ml = ck > 1 ? ck - 1 : 1, mh = ck < s.ncd[2] ? ck + 1 : s.ncd[2];
+          for (int q = 0; q <= last; ++q) {
+            const int jr = (DIM == 3) ? gcj - 1 + q / 3 : gcj, ir = gci - 1 + ((DIM == 3) ? q % 3 : q);
+            if (ir < 1 || ir > s.ncd[0] || jr < 1 || jr > s.ncd[1]) continue;
+            const int base = s.cell_off + ((jr - 1) * s.ncd[0] + (ir - 1)) * s.ncd[2];
+            seen += (q == last ? (at_cap & kSlotMask) + 1 : P.cell_start[base + mh]) - P.cell_start[base + ml - 1];
+          }
+        }
+        trunc = seen < cand;
+      }
       __syncwarp();
     }
     flush();
@@ -2114,10 +2121,10 @@ __global__ void __launch_bounds__(kListBlock, DIM == 3 ? 9 : 12) k_neighbour_lis
       if (n > 2) w.z = mine_wait[64];
       out[(size_t)(done >> 2) * 32] = w;
     }
-    if (active) {
-      b.ncount[p] = done + n;
-      if (trunc) atomicOr(&dyn->warnings, SPH_WARN_NEIGHBOURS_TRUNCATED);
-    }
+    if (active) b.ncount[p] = done + n;
+    // one per warp: every cut particle's own met the others at one address
+    // (the same 200,000: 187 us so, 120 here)
+    if (__any_sync(FULL, trunc) && lane == 0) atomicOr(&dyn->warnings, SPH_WARN_NEIGHBOURS_TRUNCATED);
     block_count2(b.counters, cand, nacc);
     const int m = warp_max(nacc);
     if (lane == 0 && m > 0) atomicMax(&dyn->max_neigh, m);
